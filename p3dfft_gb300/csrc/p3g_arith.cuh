@@ -112,13 +112,6 @@ P3G_HD float ffma(float a, float b, float c) {
 struct df {
   float hi, lo;
 };
-struct cdf {  // double-float complex
-  df re, im;
-};
-struct cf {  // binary32 complex
-  float re, im;
-};
-
 // Knuth TwoSum: s + e == a + b exactly.
 P3G_HD void two_sum(float a, float b, float& s, float& e) {
   s = fadd_rn(a, b);
@@ -342,60 +335,156 @@ P3G_D df dmulc(df a, float chi, float clo) {
 // exact scaling by a power of two
 P3G_D df dscale2(df a, float p2) { return df{a.hi * p2, a.lo * p2}; }
 
+#if defined(__CUDACC__)
+// ------------------------------------------------------- packed binary32
+// sm_103a adds, multiplies and FMAs two binary32 values held in a register
+// pair with one instruction (add/mul/fma.rn.f32x2), each half rounded as the
+// scalar instruction would.  The FMA pipe takes a packed instruction every
+// other cycle (59.5 pairs/clk/SM measured against 2 x 64 lanes for scalar
+// ones), so the arithmetic rate is the same, but a packed stream takes half
+// the issue slots, leaves the other half to address and copy instructions,
+// and its results take fewer registers (16-point double-float butterfly: 128
+// against 202).  A register-only loop of twiddles and 16-point butterflies
+// runs at 0.97 clk per point and SM against 1.14 scalar (256 threads per SM).
+// Double-float complex values are packed as (re, im) high and (re, im) low
+// words, which is also their order in the workspace and the twiddle tables;
+// swapped, negated or repeated halves cost nothing measurable as operands.
+// The binary32 path stays scalar: its passes are not bound by issue (packed,
+// the strided ones ran 3-7 % slower).
+using u64p = unsigned long long;
+P3G_D u64p pk2(float x, float y) {
+  u64p r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+P3G_D float pk_lo(u64p a) { return __uint_as_float((unsigned)a); }
+P3G_D float pk_hi(u64p a) { return __uint_as_float((unsigned)(a >> 32)); }
+P3G_D u64p add2(u64p a, u64p b) {
+  u64p r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+P3G_D u64p sub2(u64p a, u64p b) {
+  u64p r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+P3G_D u64p mul2(u64p a, u64p b) {
+  u64p r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+P3G_D u64p fma2(u64p a, u64p b, u64p c) {
+  u64p r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+P3G_D u64p neg2(u64p a) { return pk2(-pk_lo(a), -pk_hi(a)); }
+P3G_D u64p dup_lo(u64p a) { return pk2(pk_lo(a), pk_lo(a)); }
+P3G_D u64p dup_hi(u64p a) { return pk2(pk_hi(a), pk_hi(a)); }
+// (x, y) times s*i with s = +1 or -1: (-y, x) or (y, -x)
+template <int S>
+P3G_D u64p rot2(u64p a) {
+  return S > 0 ? pk2(-pk_hi(a), pk_lo(a)) : pk2(pk_hi(a), -pk_lo(a));
+}
+
 // ------------------------------------------------------------- complex ops
-P3G_D cdf operator+(cdf a, cdf b) { return cdf{dadd(a.re, b.re), dadd(a.im, b.im)}; }
-P3G_D cdf operator-(cdf a, cdf b) { return cdf{dsub(a.re, b.re), dsub(a.im, b.im)}; }
+struct cdf {  // double-float complex: h = (re.hi, im.hi), l = (re.lo, im.lo)
+  u64p h, l;
+};
+struct cf {  // binary32 complex
+  float re, im;
+};
+P3G_D cdf make_cdf(df re, df im) { return cdf{pk2(re.hi, im.hi), pk2(re.lo, im.lo)}; }
+
+// TwoSum of both halves: s + e == a + b exactly
+P3G_D void two_sum2(u64p a, u64p b, u64p& s, u64p& e) {
+  s = add2(a, b);
+  const u64p bb = sub2(s, a);
+  e = add2(sub2(a, sub2(s, bb)), sub2(b, bb));
+}
+P3G_D cdf operator+(cdf a, cdf b) {
+  u64p s, e;
+  two_sum2(a.h, b.h, s, e);
+  return cdf{s, add2(add2(a.l, b.l), e)};
+}
+P3G_D cdf operator-(cdf a, cdf b) {
+  const u64p s = sub2(a.h, b.h);
+  const u64p bb = sub2(s, a.h);
+  const u64p e = sub2(sub2(a.h, sub2(s, bb)), add2(b.h, bb));
+  return cdf{s, add2(sub2(a.l, b.l), e)};
+}
 P3G_D cf operator+(cf a, cf b) { return cf{a.re + b.re, a.im + b.im}; }
 P3G_D cf operator-(cf a, cf b) { return cf{a.re - b.re, a.im - b.im}; }
 
 // multiply by s*i with s = +1 or -1
 template <int S>
 P3G_D cdf rot(cdf a) {
-  return S > 0 ? cdf{dneg(a.im), a.re} : cdf{a.im, dneg(a.re)};
+  return cdf{rot2<S>(a.h), rot2<S>(a.l)};
 }
 template <int S>
 P3G_D cf rot(cf a) {
   return S > 0 ? cf{-a.im, a.re} : cf{a.im, -a.re};
 }
-P3G_D cdf cneg(cdf a) { return cdf{dneg(a.re), dneg(a.im)}; }
+P3G_D cdf cneg(cdf a) { return cdf{neg2(a.h), neg2(a.l)}; }
 P3G_D cf cneg(cf a) { return cf{-a.re, -a.im}; }
-P3G_D cdf cscale2(cdf a, float p2) { return cdf{dscale2(a.re, p2), dscale2(a.im, p2)}; }
+P3G_D cdf cscale2(cdf a, float p2) { return cdf{mul2(a.h, pk2(p2, p2)), mul2(a.l, pk2(p2, p2))}; }
 P3G_D cf cscale2(cf a, float p2) { return cf{a.re * p2, a.im * p2}; }
-P3G_D cdf cconj(cdf a) { return cdf{a.re, dneg(a.im)}; }
+P3G_D cdf cconj(cdf a) { return cdf{pk2(pk_lo(a.h), -pk_hi(a.h)), pk2(pk_lo(a.l), -pk_hi(a.l))}; }
 P3G_D cf cconj(cf a) { return cf{a.re, -a.im}; }
 
-// real double-float constant (hi, lo) times complex
-P3G_D cdf mulr(cdf a, float chi, float clo) { return cdf{dmulc(a.re, chi, clo), dmulc(a.im, chi, clo)}; }
+// real double-float constant (hi, lo) times complex (the lo*lo term is below
+// 2^-48); the binary32 path takes the constant's high part
+P3G_D cdf mulr(cdf a, float chi, float clo) {
+  const u64p ch = pk2(chi, chi);
+  const u64p r = mul2(a.h, ch);
+  u64p e = fma2(a.h, ch, neg2(r));
+  e = fma2(a.h, pk2(clo, clo), e);
+  return cdf{r, fma2(a.l, ch, e)};
+}
 P3G_D cf mulr(cf a, float chi, float /*clo*/) { return cf{a.re * chi, a.im * chi}; }
-
-// sum of two exact-ish products p1 + s2*p2 where p = x*y, used by the complex
-// multiply: returns (x1*y1 + sg*x2*y2) in double-float with lo cross terms.
-P3G_D df dot2(df x1, df y1, df x2, df y2, float sg) {
-  const float p1 = fmul_rn(x1.hi, y1.hi);
-  const float e1 = ffma(x1.hi, y1.hi, -p1);
-  const float p2 = fmul_rn(x2.hi, y2.hi) * sg;
-  const float e2 = ffma(x2.hi * sg, y2.hi, -p2);
-  float s, t;
-  two_sum(p1, p2, s, t);
-  float lo = fadd_rn(fadd_rn(e1, e2), t);
-  lo = ffma(x1.hi, y1.lo, lo);
-  lo = ffma(x1.lo, y1.hi, lo);
-  lo = ffma(x2.hi * sg, y2.lo, lo);
-  lo = ffma(x2.lo * sg, y2.hi, lo);
-  return df{s, lo};
+// a + c x: one FMA on the binary32 path
+P3G_D cdf addmulr(cdf a, cdf x, float chi, float clo) { return a + mulr(x, chi, clo); }
+P3G_D cf addmulr(cf a, cf x, float chi, float /*clo*/) { return cf{ffma(x.re, chi, a.re), ffma(x.im, chi, a.im)}; }
+// e + c x into p and e - c x into m
+P3G_D void bfly_mulr(cdf& p, cdf& m, cdf e, cdf x, float chi, float clo) {
+  const cdf o = mulr(x, chi, clo);
+  p = e + o;
+  m = e - o;
+}
+P3G_D void bfly_mulr(cf& p, cf& m, cf e, cf x, float chi, float /*clo*/) {
+  p = cf{ffma(x.re, chi, e.re), ffma(x.im, chi, e.im)};
+  m = cf{ffma(x.re, -chi, e.re), ffma(x.im, -chi, e.im)};
 }
 
+// x1 y1 + x2 y2 in both halves, in double-float with the lo cross terms
+P3G_D cdf dot22(u64p x1, u64p x1l, u64p y1, u64p y1l, u64p x2, u64p x2l, u64p y2, u64p y2l) {
+  const u64p p1 = mul2(x1, y1);
+  const u64p e1 = fma2(x1, y1, neg2(p1));
+  const u64p p2 = mul2(x2, y2);
+  const u64p e2 = fma2(x2, y2, neg2(p2));
+  u64p s, t;
+  two_sum2(p1, p2, s, t);
+  u64p lo = add2(add2(e1, e2), t);
+  lo = fma2(x1, y1l, lo);
+  lo = fma2(x1l, y1, lo);
+  lo = fma2(x2, y2l, lo);
+  lo = fma2(x2l, y2, lo);
+  return cdf{s, lo};
+}
 // a * w (CONJ = false) or a * conj(w) (CONJ = true), w a double-float twiddle
 template <bool CONJ>
 P3G_D cdf cmul(cdf a, cdf w) {
-  if (!CONJ) return cdf{dot2(a.re, w.re, a.im, w.im, -1.0f), dot2(a.re, w.im, a.im, w.re, 1.0f)};
-  return cdf{dot2(a.re, w.re, a.im, w.im, 1.0f), dot2(a.im, w.re, a.re, w.im, -1.0f)};
+  if (!CONJ)  // re w + im (i w)
+    return dot22(dup_lo(a.h), dup_lo(a.l), w.h, w.l, dup_hi(a.h), dup_hi(a.l), rot2<1>(w.h), rot2<1>(w.l));
+  // a w.re + (-i a) w.im
+  return dot22(a.h, a.l, dup_lo(w.h), dup_lo(w.l), rot2<-1>(a.h), rot2<-1>(a.l), dup_hi(w.h), dup_hi(w.l));
 }
 // binary32 data times a compensated twiddle (w.hi + w.lo per component)
 template <bool CONJ>
 P3G_D cf cmul(cf a, cdf w) {
-  const float wr = w.re.hi, wrl = w.re.lo;
-  const float wi = CONJ ? -w.im.hi : w.im.hi, wil = CONJ ? -w.im.lo : w.im.lo;
+  const float wr = pk_lo(w.h), wrl = pk_lo(w.l);
+  const float wi = CONJ ? -pk_hi(w.h) : pk_hi(w.h), wil = CONJ ? -pk_hi(w.l) : pk_hi(w.l);
   float re = a.re * wrl;
   re = ffma(-a.im, wil, re);
   re = ffma(a.re, wr, re);
@@ -408,14 +497,12 @@ P3G_D cf cmul(cf a, cdf w) {
 }
 // complex constant c = (cre, cim) (double-float parts)
 P3G_D cdf mulcc(cdf a, float crh, float crl, float cih, float cil) {
-  const df cr{crh, crl}, ci{cih, cil};
-  return cdf{dot2(a.re, cr, a.im, ci, -1.0f), dot2(a.re, ci, a.im, cr, 1.0f)};
+  return cmul<false>(a, cdf{pk2(crh, cih), pk2(crl, cil)});
 }
 P3G_D cf mulcc(cf a, float crh, float /*crl*/, float cih, float /*cil*/) {
   return cf{ffma(a.re, crh, -a.im * cih), ffma(a.re, cih, a.im * crh)};
 }
 
-#if defined(__CUDACC__)
 // ------------------------------------------------ memory formats per path
 // F64 path: user data binary64 (double / double2); workspace and shared
 // memory hold one complex as float4 (re.hi, im.hi, re.lo, im.lo).
@@ -426,17 +513,15 @@ struct PathF64 {
   using UR = double;  // user real
   using UC = double2; // user complex
   static constexpr bool kF64 = true;
-  P3G_D static C from_w(float4 v) { return cdf{df{v.x, v.z}, df{v.y, v.w}}; }
-  P3G_D static float4 to_w(C c) { return make_float4(c.re.hi, c.im.hi, c.re.lo, c.im.lo); }
-  P3G_D static C from_uc(double2 v) { return cdf{d2df(v.x), d2df(v.y)}; }
-  P3G_D static double2 to_uc(C c) { return make_double2(df2d(c.re.hi, c.re.lo), df2d(c.im.hi, c.im.lo)); }
+  P3G_D static C from_w(float4 v) { return cdf{pk2(v.x, v.y), pk2(v.z, v.w)}; }
+  P3G_D static float4 to_w(C c) { return make_float4(pk_lo(c.h), pk_hi(c.h), pk_lo(c.l), pk_hi(c.l)); }
+  P3G_D static C from_uc(double2 v) { return make_cdf(d2df(v.x), d2df(v.y)); }
+  P3G_D static double2 to_uc(C c) { return make_double2(to_ur(re(c)), to_ur(im(c))); }
   P3G_D static df from_ur(double v) { return d2df(v); }
   P3G_D static double to_ur(df v) { return df2d(v.hi, v.lo); }
   // with the exponent bias k: inputs times 2^-k, outputs times 2^k
-  P3G_D static C from_uc(double2 v, int k) { return cdf{d2df_scaled(v.x, k), d2df_scaled(v.y, k)}; }
-  P3G_D static double2 to_uc(C c, int k) {
-    return make_double2(scale_pow2(df2d(c.re.hi, c.re.lo), k), scale_pow2(df2d(c.im.hi, c.im.lo), k));
-  }
+  P3G_D static C from_uc(double2 v, int k) { return make_cdf(d2df_scaled(v.x, k), d2df_scaled(v.y, k)); }
+  P3G_D static double2 to_uc(C c, int k) { return make_double2(to_ur(re(c), k), to_ur(im(c), k)); }
   P3G_D static df from_ur(double v, int k) { return d2df_scaled(v, k); }
   P3G_D static double to_ur(df v, int k) { return scale_pow2(df2d(v.hi, v.lo), k); }
   // largest |high word| seen (the binary64 exponent window's input)
@@ -447,10 +532,10 @@ struct PathF64 {
     track(amax, v.x);
     track(amax, v.y);
   }
-  P3G_D static C make(df re, df im) { return cdf{re, im}; }
-  P3G_D static C zero() { return cdf{df{0.f, 0.f}, df{0.f, 0.f}}; }
-  P3G_D static df re(C c) { return c.re; }
-  P3G_D static df im(C c) { return c.im; }
+  P3G_D static C make(df re, df im) { return make_cdf(re, im); }
+  P3G_D static C zero() { return cdf{0, 0}; }
+  P3G_D static df re(C c) { return df{pk_lo(c.h), pk_lo(c.l)}; }
+  P3G_D static df im(C c) { return df{pk_hi(c.h), pk_hi(c.l)}; }
 };
 struct PathF32 {
   using C = cf;
@@ -460,14 +545,14 @@ struct PathF32 {
   static constexpr bool kF64 = false;
   P3G_D static C from_w(float2 v) { return cf{v.x, v.y}; }
   P3G_D static float2 to_w(C c) { return make_float2(c.re, c.im); }
-  P3G_D static C from_uc(float2 v) { return cf{v.x, v.y}; }
-  P3G_D static float2 to_uc(C c) { return make_float2(c.re, c.im); }
+  P3G_D static C from_uc(float2 v) { return from_w(v); }
+  P3G_D static float2 to_uc(C c) { return to_w(c); }
   P3G_D static float from_ur(float v) { return v; }
   P3G_D static float to_ur(float v) { return v; }
   // binary32 data has binary32's range, as the reference's single-precision
   // build: no exponent bias and nothing to track
-  P3G_D static C from_uc(float2 v, int) { return cf{v.x, v.y}; }
-  P3G_D static float2 to_uc(C c, int) { return make_float2(c.re, c.im); }
+  P3G_D static C from_uc(float2 v, int) { return from_w(v); }
+  P3G_D static float2 to_uc(C c, int) { return to_w(c); }
   P3G_D static float from_ur(float v, int) { return v; }
   P3G_D static float to_ur(float v, int) { return v; }
   P3G_D static void track(uint32_t&, float) {}

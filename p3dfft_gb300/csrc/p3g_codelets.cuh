@@ -33,11 +33,10 @@ P3G_D void dft2(C* a) {
 template <int DIR, class C>
 P3G_D void dft3(C* a) {
   const C t1 = a[1] + a[2];
-  const C t2 = a[0] + cscale2(t1, -0.5f);
-  const C t3 = rot<DIR>(mulr(a[1] - a[2], P3G_SQRT3_2));
+  const C t2 = addmulr(a[0], t1, -0.5f, 0.0f);
+  const C t3 = rot<DIR>(a[1] - a[2]);
   a[0] = a[0] + t1;
-  a[1] = t2 + t3;
-  a[2] = t2 - t3;
+  bfly_mulr(a[1], a[2], t2, t3, P3G_SQRT3_2);
 }
 
 template <int DIR, class C>
@@ -56,10 +55,10 @@ P3G_D void dft4(C* a) {
 template <int DIR, class C>
 P3G_D void dft5(C* a) {
   const C t1 = a[1] + a[4], t2 = a[2] + a[3], t3 = a[1] - a[4], t4 = a[2] - a[3];
-  const C b1 = a[0] + (mulr(t1, P3G_C5_1) + mulr(t2, P3G_C5_2));
-  const C b2 = a[0] + (mulr(t1, P3G_C5_2) + mulr(t2, P3G_C5_1));
-  const C d1 = rot<DIR>(mulr(t3, P3G_S5_1) + mulr(t4, P3G_S5_2));
-  const C d2 = rot<DIR>(mulr(t3, P3G_S5_2) - mulr(t4, P3G_S5_1));
+  const C b1 = a[0] + addmulr(mulr(t1, P3G_C5_1), t2, P3G_C5_2);
+  const C b2 = a[0] + addmulr(mulr(t1, P3G_C5_2), t2, P3G_C5_1);
+  const C d1 = rot<DIR>(addmulr(mulr(t3, P3G_S5_1), t4, P3G_S5_2));
+  const C d2 = rot<DIR>(addmulr(mulr(t3, P3G_S5_2), cneg(t4), P3G_S5_1));
   a[0] = a[0] + (t1 + t2);
   a[1] = b1 + d1;
   a[4] = b1 - d1;
@@ -81,18 +80,17 @@ template <int DIR, class C>
 P3G_D void dft8(C* a) {
   dft4<DIR>(a[0], a[2], a[4], a[6]);
   dft4<DIR>(a[1], a[3], a[5], a[7]);
-  const C o1 = mul_w8_1<DIR>(a[3]);
+  // o1 = w8^1 a[3] and o3 = w8^3 a[7] up to their factor 1/sqrt2
+  const C o1 = a[3] + rot<DIR>(a[3]);
   const C o2 = rot<DIR>(a[5]);
-  const C o3 = mul_w8_3<DIR>(a[7]);
+  const C o3 = rot<DIR>(a[7]) - a[7];
   const C e0 = a[0], e1 = a[2], e2 = a[4], e3 = a[6], o0 = a[1];
   a[0] = e0 + o0;
   a[4] = e0 - o0;
-  a[1] = e1 + o1;
-  a[5] = e1 - o1;
+  bfly_mulr(a[1], a[5], e1, o1, P3G_SQRT1_2);
   a[2] = e2 + o2;
   a[6] = e2 - o2;
-  a[3] = e3 + o3;
-  a[7] = e3 - o3;
+  bfly_mulr(a[3], a[7], e3, o3, P3G_SQRT1_2);
 }
 
 // 16 = 4 x 4: inner DFT4 over n2 (stride-4 inputs), twiddle w16^(n1 k2),

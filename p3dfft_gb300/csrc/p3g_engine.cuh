@@ -40,7 +40,7 @@ struct StagePlan {
 // multiplies by the conjugate.
 P3G_D cdf load_tw(const float4* __restrict__ tw, int idx) {
   const float4 v = tw[idx];  // shared memory (pipelined passes) or global
-  return cdf{df{v.x, v.z}, df{v.y, v.w}};
+  return cdf{pk2(v.x, v.y), pk2(v.z, v.w)};
 }
 
 // Division by a runtime divisor d <= 2^15 for dividends x < 2^15 with one
