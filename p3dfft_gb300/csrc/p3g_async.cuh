@@ -58,6 +58,11 @@ P3G_D void mbar_arrive_expect_tx(uint64_t* b, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_u32(b)), "r"(bytes)
                : "memory");
 }
+// Arrives on the barrier once every cp.async this thread issued before has
+// completed (counts as one of the barrier's expected arrivals).
+P3G_D void cp_async_mbar_arrive(uint64_t* b) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];\n" ::"r"(smem_u32(b)) : "memory");
+}
 P3G_D bool mbar_try_wait(uint64_t* b, uint32_t parity) {
   uint32_t ok;
   asm volatile(

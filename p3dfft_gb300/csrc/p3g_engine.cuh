@@ -10,12 +10,14 @@
 // by w_{Ns R}^{q (j mod Ns)}, runs a register DFT of size R and writes points
 // (j / Ns) Ns R + (j mod Ns) + q Ns.  All reads of a stage finish before any
 // write (one barrier), so a stage works in place: every thread keeps all of its
-// butterflies of the stage in registers (at most ceil(E/R), E = elements per
-// thread, which the launch guarantees by using ceil(M N / E) threads).
+// butterflies of the stage in registers (at most stage_butterflies, for which
+// the launch has enough threads).
 //
 // Radices 2, 3, 4, 5, 8, 16, 32 are register codelets.  Any other prime p runs a
 // generic direct-DFT stage through a second shared-memory buffer (O(N p) work).
 #pragma once
+
+#include <type_traits>
 
 #include "p3g_codelets.cuh"
 
@@ -24,11 +26,24 @@ namespace p3g {
 constexpr int kMaxStages = 20;
 constexpr int kElemsPerThread = 16;  // E
 
+// The register codelets in the order their stages run: powers of two first,
+// so that the sub-transform length before any of them is a power of two.
+constexpr int kFamilies[] = {32, 16, 8, 4, 2, 3, 5};
+constexpr int kNumFamilies = sizeof(kFamilies) / sizeof(kFamilies[0]);
+P3G_HD int family_count(unsigned long long fam, int i) { return (int)(fam >> (4 * i)) & 15; }
+
+// Most butterflies of radix r that a thread of E elements runs per stage: as
+// many as cover E elements or, where the launch can have the threads for it
+// (the grouped kernels), as many as E elements hold.
+P3G_HD constexpr int stage_butterflies(int E, int r, bool hold) {
+  return hold ? (E / r > 1 ? E / r : 1) : (E + r - 1) / r;
+}
+
 struct StagePlan {
   int n;                   // transform length (1 allowed: no stages)
   int nstages;
   int has_generic;         // a stage with a radix outside {2,3,4,5,8,16}
-  int cnt[7];              // number of stages of radix 32, 16, 8, 4, 2, 3, 5 (stored in this order, then generic)
+  unsigned long long fam;  // stages of each radix family, 4 bits each in the order of kFamilies, then generic
   int radix[kMaxStages];
   int ns[kMaxStages];      // sub-transform length before the stage
   int tw_off[kMaxStages];  // float4 offset of this stage's twiddles [k < ns][q-1 < radix-1]
@@ -99,7 +114,51 @@ P3G_D void sts(uint32_t a, float2 v) {
 // equally spaced in the padded layout.
 P3G_D int pad_index(int j, int ps) { return ps ? j + (j >> ps) : j; }
 
-template <class P>
+// Hardware barrier with a compile-time id.  Each radix uses its own id: with a
+// plain __syncthreads() the compiler merges the identical barriers of all
+// switch cases in cta_fft, which keeps every case's registers live at once.
+template <int ID>
+P3G_D void cta_barrier() {
+  asm volatile("bar.sync %0;" ::"n"(ID) : "memory");
+}
+
+// The threads that work on one tile: the whole CTA, or one group of a CTA
+// whose groups work on tiles of their own (t = index in the group, n = its
+// threads, id = its named barrier).
+struct CtaThreads {
+  static constexpr bool kHold = false;  // stage_butterflies
+  P3G_D int tid() const { return (int)threadIdx.x; }
+  P3G_D int count() const { return (int)blockDim.x; }
+  P3G_D void sync() const { __syncthreads(); }
+  template <int ID>
+  P3G_D void stage_sync() const {
+    cta_barrier<ID>();
+  }
+};
+struct GroupThreads {
+  static constexpr bool kHold = true;
+  int t = 0, n = 0, id = 0;
+  P3G_D int tid() const { return t; }
+  P3G_D int count() const { return n; }
+  P3G_D void sync() const { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
+  template <int ID>
+  P3G_D void stage_sync() const {
+    sync();
+  }
+  // barrier, true if p holds for any thread of the group (not the aligned
+  // form: the threads come from wait loops of their own lengths)
+  P3G_D bool sync_or(bool p) const {
+    uint32_t r;
+    asm volatile(
+        "{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n barrier.red.or.pred q, %2, %3, p;\n selp.u32 %0, 1, 0, q;\n}\n"
+        : "=r"(r)
+        : "r"((uint32_t)p), "r"(id), "r"(n)
+        : "memory");
+    return r != 0;
+  }
+};
+
+template <class P, class TH = CtaThreads>
 struct Tile {
   typename P::W* sm;       // M lines x N points
   typename P::W* scratch;  // same size, generic stages only
@@ -109,6 +168,7 @@ struct Tile {
   // and the thread's running largest |high word| (null: not tracked)
   int ebias = 0;
   uint32_t* amax = nullptr;
+  TH th{};
   P3G_D int addr(int line, int j) const { return line * LS + (LS == 1 ? j * JS : pad_index(j, ps)); }
   P3G_D uint32_t saddr(int line, int j) const {
     return (uint32_t)__cvta_generic_to_shared(sm) + (uint32_t)((line * LS + j * JS) * (int)sizeof(typename P::W));
@@ -136,23 +196,14 @@ struct Tile {
   }
 };
 
-// Hardware barrier with a compile-time id.  Each radix uses its own id: with a
-// plain __syncthreads() the compiler merges the identical barriers of all
-// switch cases in cta_fft, which keeps every case's registers live at once.
-template <int ID>
-P3G_D void cta_barrier() {
-  asm volatile("bar.sync %0;" ::"n"(ID) : "memory");
-}
-
 // Tile layouts a kernel can fix at compile time: the strided passes use
 // point-major tiles (LS = 1, JS = M), the X passes line-major ones (LS =
 // padded N, JS = 1); kAnyLayout reads the layout from the tile.
 enum { kAnyLayout = -1, kLineMajor = 0, kPointMajor = 1 };
 
 // One stage of radix R.  FULL: every thread owns exactly MAXB butterflies
-// (M N / R == MAXB x blockDim.x, the usual case), so no butterfly needs a
-// guard or a placeholder value.  With a known layout the butterfly -> point
-// mapping needs no runtime layout test: point-major, butterfly b reads
+// (M N / R == MAXB x threads), so no butterfly needs a guard or a placeholder
+// value.  With a known layout the butterfly -> point mapping needs no runtime layout test: point-major, butterfly b reads
 // element b (line b mod M, position b / M); line-major, b / (N / R) is the
 // line.  In the power-of-two families ns is a power of two (they run first),
 // so the twiddle index is a mask.
@@ -169,15 +220,15 @@ enum { kAnyLayout = -1, kLineMajor = 0, kPointMajor = 1 };
 //            p = 0 and p = N/2 modes ignored (as c2r does).
 enum { kRawNone = 0, kRawR2C = 1, kRawC2R = 2 };
 
-template <class P, int DIR, int R, int E, int LAY, bool FULL, int RAW = kRawNone>
-__device__ __forceinline__ void stage_reg(const Tile<P>& t, int N, int ns, const float4* __restrict__ tw) {
+template <class P, int DIR, int R, int E, int LAY, bool FULL, int RAW = kRawNone, class TH = CtaThreads>
+__device__ __forceinline__ void stage_reg(const Tile<P, TH>& t, int N, int ns, const float4* __restrict__ tw) {
   using C = typename P::C;
   using W = typename P::W;
-  constexpr int MAXB = (E + R - 1) / R;
+  constexpr int MAXB = stage_butterflies(E, R, TH::kHold);
   constexpr bool kPow2 = (R & (R - 1)) == 0;
   constexpr uint32_t kW = (uint32_t)sizeof(W);
   const int per_line = N / R;
-  const int T = blockDim.x;
+  const int T = t.th.count();
   const bool pm = LAY == kPointMajor || (LAY == kAnyLayout && t.LS == 1);
   const FastDiv fd_line((uint32_t)(pm ? 1 : per_line)), fd_ns((uint32_t)(kPow2 ? 1 : ns));
   const int nb = t.M * per_line;
@@ -188,14 +239,17 @@ __device__ __forceinline__ void stage_reg(const Tile<P>& t, int N, int ns, const
                               : (uint32_t)(t.JS * (int)kW) * (uint32_t)pad_index(per_line, ps);
   const uint32_t ostride =
       pm ? ((uint32_t)ns << t.log2m) * kW : (uint32_t)(t.JS * (int)kW) * (uint32_t)pad_index(ns, ps);
-  // Non-full stages: explicitly initialised, because the arrays are written
-  // and read under correlated guards (b < nb) the compiler cannot prove, and
-  // inside a persistent tile loop an uninitialised element would otherwise be
-  // kept live around the loop, with every codelet's registers.
+  // Non-full stages.  Grouped kernels: a thread past the last butterfly
+  // computes that one again and stores nothing (no branches, every element
+  // defined).  CTA-wide kernels skip it, with the arrays explicitly
+  // initialised: they are written and read under correlated guards the
+  // compiler cannot prove, and inside a persistent tile loop an uninitialised
+  // element would otherwise be kept live around the loop.  (The batch kernel
+  // spills 16 bytes with the guards and 220 without; the strided one the
+  // reverse.)
   C v[MAXB][R];
   uint32_t oaddr[MAXB];
-  bool live[MAXB];
-  if constexpr (!FULL) {
+  if constexpr (!FULL && !TH::kHold) {
 #pragma unroll
     for (int i = 0; i < MAXB; ++i) {
       oaddr[i] = 0;
@@ -205,9 +259,9 @@ __device__ __forceinline__ void stage_reg(const Tile<P>& t, int N, int ns, const
   }
 #pragma unroll
   for (int i = 0; i < MAXB; ++i) {
-    const int b = threadIdx.x + i * T;
-    live[i] = FULL || b < nb;
-    if (live[i]) {
+    const int bi = t.th.tid() + i * T;
+    const int b = FULL || !TH::kHold ? bi : min(bi, nb - 1);
+    if (FULL || TH::kHold || bi < nb) {
       int line, j;
       uint32_t ia;
       if (pm) {
@@ -271,15 +325,15 @@ __device__ __forceinline__ void stage_reg(const Tile<P>& t, int N, int ns, const
       oaddr[i] = sbase + (pm ? (uint32_t)(line + (jo << t.log2m)) * kW : (uint32_t)(t.addr(line, jo) * (int)kW));
     }
   }
-  cta_barrier<(R == 16 ? 1 : (R == 32 ? 6 : R))>();
+  t.th.template stage_sync<(R == 16 ? 1 : (R == 32 ? 6 : R))>();
 #pragma unroll
   for (int i = 0; i < MAXB; ++i) {
-    if (live[i]) {
+    if (FULL || t.th.tid() + i * T < nb) {
 #pragma unroll
       for (int q = 0; q < R; ++q) sts(oaddr[i] + q * ostride, P::to_w(v[i][q]));
     }
   }
-  cta_barrier<(R == 16 ? 1 : (R == 32 ? 6 : R))>();
+  t.th.template stage_sync<(R == 16 ? 1 : (R == 32 ? 6 : R))>();
 }
 
 // Generic prime radix p: twiddle the inputs into scratch, then each output is
@@ -324,17 +378,17 @@ __device__ __noinline__ void stage_generic(const Tile<P>& t, int N, int p, int n
 // length ns(s) = product of the radices before it; both follow from the
 // family counts, so they are carried in registers instead of being loaded
 // per stage (stage 0 owns one placeholder twiddle, see build_stages).
-template <class P, int DIR, int R, int E, int LAY, int RAW>
-__device__ __forceinline__ void run_family(const Tile<P>& t, const float4* __restrict__ tw, int N, int cnt, int& ns,
-                                           int& off, bool& raw) {
-  constexpr int MAXB = (E + R - 1) / R;
-  const bool full = t.M * (N / R) == MAXB * (int)blockDim.x;
+template <class P, int DIR, int R, int E, int LAY, bool FULL, int RAW, class TH>
+__device__ __forceinline__ void run_family(const Tile<P, TH>& t, const float4* __restrict__ tw, int N, int cnt, int& ns,
+                                           int& off) {
+  // the CTA-wide kernels run plans of every kind and take the unguarded form
+  // stage by stage; the grouped kernels are compiled for one of them
+  const bool full = FULL || (!TH::kHold && t.M * (N / R) == stage_butterflies(E, R, TH::kHold) * t.th.count());
 #pragma unroll 1
   for (int c = 0; c < cnt; ++c) {
-    if (RAW != kRawNone && raw) {  // the plan's first stage reads the raw line pairs
+    if (RAW != kRawNone && ns == 1) {  // the plan's first stage reads the raw line pairs
       if (full) stage_reg<P, DIR, R, E, LAY, true, RAW>(t, N, ns, tw + off);
       else stage_reg<P, DIR, R, E, LAY, false, RAW>(t, N, ns, tw + off);
-      raw = false;
     } else if (full) {
       stage_reg<P, DIR, R, E, LAY, true>(t, N, ns, tw + off);
     } else {
@@ -346,45 +400,47 @@ __device__ __forceinline__ void run_family(const Tile<P>& t, const float4* __res
 }
 
 // Runs all stages of the plan on the tile (sm must be filled and
-// synchronised).  MAXR is the largest power-of-two radix compiled in: 16 on
-// the F32 path and 8 on F64, 32 and 16 in the wide pipelined kernels (the
-// large codelets need many registers, so only kernels that may use them
-// carry them; the plans they run never exceed MAXR).  The plan orders its stages by radix family (16, 8, 4, 2, 3,
-// 5, then generic primes) and each family runs in its own loop: a single loop
-// with a switch over the radix makes the register allocator keep the live
-// ranges of every codelet at once and spill.  Radix 16 is compiled only for
-// the F32 path (the F64 codelet needs ~200 registers; radix 8 has the same
-// double-float operation count per point for the sizes used here).
+// synchronised).  MAXR is the largest radix compiled in (the large codelets
+// need many registers, so only kernels that may use them carry them; the
+// plans they run never exceed MAXR).  Each family runs in its own loop: a
+// single loop with a switch over the radix makes the register allocator keep
+// the live ranges of every codelet at once and spill.  FULL: a plan of
+// power-of-two radices whose stages all fill every thread; only those
+// families are compiled, without guards.
 // tw points at the twiddle table entry tw_base (the full table with
 // tw_base = 0, or a pass's slice copied to shared memory).  E = elements each
-// thread holds per stage; the launch uses ceil(M N / E) threads.  LAY: the
+// thread holds per stage.  LAY: the
 // tile layout when the caller knows it (kPointMajor, kLineMajor).  RAW: the
 // tile still holds the raw line pairs of an X r2c or c2r tile (kRawR2C,
 // kRawC2R; plans without generic stages only), read by the first stage.
 template <class P, int DIR, int E = kElemsPerThread, int LAY = kAnyLayout, int RAW = kRawNone,
-          int MAXR = P::kF64 ? 8 : 16>
-__device__ __forceinline__ void cta_fft(const Tile<P>& t, const StagePlan* __restrict__ sp,
+          int MAXR = P::kF64 ? 8 : 16, bool FULL = false, class TH = CtaThreads>
+__device__ __forceinline__ void cta_fft(const Tile<P, TH>& t, const StagePlan* __restrict__ sp,
                                         const float4* __restrict__ tw, int tw_base = 0) {
   const int N = __ldg(&sp->n);
-  int c[7];
-#pragma unroll
-  for (int i = 0; i < 7; ++i) c[i] = __ldg(&sp->cnt[i]);
-  const int nst = __ldg(&sp->nstages);
+  const unsigned long long fam = __ldg(&sp->fam);
   int ns = 1;
   int off = __ldg(&sp->tw_off[0]) - tw_base;
-  bool raw = RAW != kRawNone;
-  if constexpr (MAXR >= 32) run_family<P, DIR, 32, E, LAY, RAW>(t, tw, N, c[0], ns, off, raw);
-  if constexpr (MAXR >= 16) run_family<P, DIR, 16, E, LAY, RAW>(t, tw, N, c[1], ns, off, raw);
-  run_family<P, DIR, 8, E, LAY, RAW>(t, tw, N, c[2], ns, off, raw);
-  run_family<P, DIR, 4, E, LAY, RAW>(t, tw, N, c[3], ns, off, raw);
-  run_family<P, DIR, 2, E, LAY, RAW>(t, tw, N, c[4], ns, off, raw);
-  run_family<P, DIR, 3, E, LAY, RAW>(t, tw, N, c[5], ns, off, raw);
-  run_family<P, DIR, 5, E, LAY, RAW>(t, tw, N, c[6], ns, off, raw);
-  const int sg = c[0] + c[1] + c[2] + c[3] + c[4] + c[5] + c[6];
+  if constexpr (MAXR >= 32) run_family<P, DIR, 32, E, LAY, FULL, RAW>(t, tw, N, family_count(fam, 0), ns, off);
+  if constexpr (MAXR >= 16) run_family<P, DIR, 16, E, LAY, FULL, RAW>(t, tw, N, family_count(fam, 1), ns, off);
+  run_family<P, DIR, 8, E, LAY, FULL, RAW>(t, tw, N, family_count(fam, 2), ns, off);
+  run_family<P, DIR, 4, E, LAY, FULL, RAW>(t, tw, N, family_count(fam, 3), ns, off);
+  run_family<P, DIR, 2, E, LAY, FULL, RAW>(t, tw, N, family_count(fam, 4), ns, off);
+  if constexpr (!FULL) {
+    run_family<P, DIR, 3, E, LAY, false, RAW>(t, tw, N, family_count(fam, 5), ns, off);
+    run_family<P, DIR, 5, E, LAY, false, RAW>(t, tw, N, family_count(fam, 6), ns, off);
+    if constexpr (std::is_same<TH, CtaThreads>::value) {
+      if (__ldg(&sp->has_generic)) {
+        int sg = 0;
+        for (int i = 0; i < kNumFamilies; ++i) sg += family_count(fam, i);
+        const int nst = __ldg(&sp->nstages);
 #pragma unroll 1
-  for (int s = sg; s < nst; ++s)
-    stage_generic<P, DIR>(t, N, __ldg(&sp->radix[s]), __ldg(&sp->ns[s]), tw + (__ldg(&sp->tw_off[s]) - tw_base),
-                          tw + (__ldg(&sp->root_off[s]) - tw_base));
+        for (int s = sg; s < nst; ++s)
+          stage_generic<P, DIR>(t, N, __ldg(&sp->radix[s]), __ldg(&sp->ns[s]), tw + (__ldg(&sp->tw_off[s]) - tw_base),
+                                tw + (__ldg(&sp->root_off[s]) - tw_base));
+      }
+    }
+  }
 }
 
 }  // namespace p3g

@@ -414,31 +414,7 @@ cudaError_t launch_cheby(const ChebyParams& p, int nfields, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-// Pipelined launchers: E (elements per thread) selects the instantiation.
-template <class P, int E>
-cudaError_t launch_strided_pipe_e(const CUtensorMap* map, const CUtensorMap* omap, const SPipeParams& p,
-                                  const StagePlan* sp, const float4* tw, bool forward_sign, int threads, size_t smem,
-                                  int grid, cudaStream_t st) {
-  cudaError_t ea = opt_in_smem((const void*)k_strided_pipe<P, -1, E>, 227 * 1024);
-  if (ea == cudaSuccess) ea = opt_in_smem((const void*)k_strided_pipe<P, 1, E>, 227 * 1024);
-  if (ea != cudaSuccess) return ea;
-  if (forward_sign) k_strided_pipe<P, -1, E><<<grid, threads, smem, st>>>(*map, *omap, p, sp, tw);
-  else k_strided_pipe<P, 1, E><<<grid, threads, smem, st>>>(*map, *omap, p, sp, tw);
-  return cudaGetLastError();
-}
-template <class P>
-cudaError_t launch_strided_pipe(const CUtensorMap* map, const CUtensorMap* omap, const SPipeParams& p,
-                                const StagePlan* sp, const float4* tw, bool forward_sign, int E, int threads,
-                                size_t smem, int grid, cudaStream_t st) {
-  if constexpr (P::kF64) {
-    if (E == 8) return launch_strided_pipe_e<P, 8>(map, omap, p, sp, tw, forward_sign, threads, smem, grid, st);
-    if (E == 16) return launch_strided_pipe_e<P, 16>(map, omap, p, sp, tw, forward_sign, threads, smem, grid, st);
-  } else {
-    if (E == 16) return launch_strided_pipe_e<P, 16>(map, omap, p, sp, tw, forward_sign, threads, smem, grid, st);
-    if (E == 32) return launch_strided_pipe_e<P, 32>(map, omap, p, sp, tw, forward_sign, threads, smem, grid, st);
-  }
-  return cudaErrorInvalidValue;
-}
+// X pass launchers: E (elements per thread) selects the instantiation.
 template <class P, int E>
 cudaError_t launch_xr2c_pipe_e(const XPipeParams& p, const StagePlan* sp, const float4* tw, int threads, size_t smem,
                                int grid, cudaStream_t st) {
@@ -480,13 +456,12 @@ cudaError_t launch_xc2r_pipe(const XPipeParams& p, const StagePlan* sp, const fl
   return cudaErrorInvalidValue;
 }
 
-// Resident CTAs per SM of a pipelined kernel (kind 0 strided, 1 r2c, 2 c2r)
+// Resident CTAs per SM of an X pass kernel (kind 1 r2c, 2 c2r)
 // with E elements per thread for the given block size and dynamic shared
 // memory; 1 if the query fails.
 template <class P, int E>
 int pipe_blocks_per_sm_e(int kind, int threads, size_t smem) {
-  const void* f = kind == 0 ? (const void*)k_strided_pipe<P, -1, E>
-                            : (kind == 1 ? (const void*)k_xr2c_pipe<P, E> : (const void*)k_xc2r_pipe<P, E>);
+  const void* f = kind == 1 ? (const void*)k_xr2c_pipe<P, E> : (const void*)k_xc2r_pipe<P, E>;
   int n = 0;
   if (opt_in_smem(f, 227 * 1024) != cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, f, threads, smem) != cudaSuccess || n < 1) {
@@ -515,9 +490,6 @@ int pipe_blocks_per_sm(int kind, int E, int threads, size_t smem) {
   template cudaError_t launch_cheby<P>(const ChebyParams&, int, cudaStream_t);                                     \
   template cudaError_t launch_x_long<P>(int, const XLongParams&, int, cudaStream_t);                               \
   template int pipe_blocks_per_sm<P>(int, int, int, size_t);                                                            \
-  template cudaError_t launch_strided_pipe<P>(const CUtensorMap*, const CUtensorMap*, const SPipeParams&,         \
-                                              const StagePlan*, const float4*, bool, int, int, size_t, int,       \
-                                              cudaStream_t);                                                      \
   template cudaError_t launch_xr2c_pipe<P>(const XPipeParams&, const StagePlan*, const float4*, int, int, size_t,  \
                                            int, cudaStream_t);                                                     \
   template cudaError_t launch_xc2r_pipe<P>(const XPipeParams&, const StagePlan*, const float4*, int, int, size_t,  \

@@ -26,7 +26,8 @@ struct PipeCommon {
   int tiles_per_field;
   int tw_base, tw_count;    // this pass's slice of the twiddle table (float4)
   int buf_elems;            // elements (W) per buffer
-  int nbuf;                 // tile buffers (2 or 3): loads run nbuf - 1 tiles ahead (nbuf - 2 with TMA stores)
+  int nbuf;                 // tile buffers (X kernels: 2 or 3, loads run nbuf - 1 tiles ahead)
+  int groups, gthreads;     // strided kernels: thread groups per CTA and threads of each
   int* err;                 // device error flag
 };
 
@@ -39,9 +40,7 @@ struct SPipeParams {
   int tx_extra;             // test hook: bytes the barrier expects beyond the boxes (0)
   int chunk;                // cp.async bytes per element copy (16 or 8)
   // 1: the transformed tile leaves by TMA stores (one thread, asynchronous)
-  // in onbox boxes of obrows rows; the kernel then keeps nbuf = 3 buffers
-  // and loads one tile ahead, so a buffer is reloaded two iterations after
-  // its store was issued
+  // in onbox boxes of obrows rows
   int tma_store;
   int obrows, onbox;
 };
@@ -60,23 +59,23 @@ P3G_D unsigned char* align1k(unsigned char* p) {
   return reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(p) + 1023) & ~uintptr_t(1023));
 }
 
-// Tiles hold at most 4096 (F64) or 8192 (F32) elements; a thread holds E
-// of them per stage: on the F64 path 16 for axes with radix-16 stages (one
-// 16-point butterfly per thread and stage: 1024 = 16 x 16 x 4) and 8
-// otherwise (512 threads, 16 warps per SM to hide the latency of the
-// dependent double-float chains); on the F32 path 32 for axes with radix-32
-// stages (one 32-point butterfly per thread and stage takes a 1024-point line
-// through two stages) and 16 otherwise.
+// Strided passes: one CTA per SM, of up to 512 threads (128 registers each).
+// A thread holds E elements per stage: 16 on F64 (one 16-point butterfly),
+// 32 on F32 (one 32-point butterfly).  FULL kernels run the power-of-two
+// lengths whose stages fill every thread (cta_fft): without the guarded
+// stages of the other radices they fit their registers without spilling,
+// which the others do not quite.
+template <class P>
+struct StridedElems {
+  static constexpr int value = P::kF64 ? 16 : 32;
+};
+constexpr int kMaxGroups = 8;        // named barriers 1..8
+constexpr int kMaxTileBuffers = 12;  // ring of tile buffers
+
+// kWide marks the X kernels compiled with the large radices.
 template <class P, int E>
 struct PipeLimits {
-  // one radix-32 (F32) or radix-16 (F64) butterfly per thread and stage
   static constexpr bool kWide = P::kF64 ? E == 16 : E == 32;
-  static constexpr int kMaxThreads = (P::kF64 ? 4096 : 8192) / E;
-  // 128 registers per thread (with a larger budget the scheduler hoists
-  // shared-memory loads across codelets and spills), except for the wide
-  // kernels: one 256-thread CTA per SM (its two 64 KB tiles fill shared
-  // memory) with up to 255 registers for the 32- or 16-point butterflies
-  static constexpr int kMinBlocks = kWide ? 1 : 65536 / 128 / kMaxThreads;
 };
 
 // X passes: 256-thread CTAs, three per SM (85 registers; for the F32
@@ -106,7 +105,8 @@ template <class P>
 struct StridedSmem {
   typename P::W* buf0;
   float4* tw;
-  uint64_t* mbar;
+  uint64_t* mbar;  // one per buffer: its load has landed
+  int* issued;     // loads issued into each buffer so far, then the CTA's failure flag
 };
 template <class P>
 P3G_D StridedSmem<P> strided_smem(const PipeCommon& pc) {
@@ -115,6 +115,7 @@ P3G_D StridedSmem<P> strided_smem(const PipeCommon& pc) {
   r.buf0 = reinterpret_cast<typename P::W*>(align1k(p3g_pipe_smem));
   r.tw = reinterpret_cast<float4*>(r.buf0 + pc.nbuf * pc.buf_elems);
   r.mbar = reinterpret_cast<uint64_t*>(r.tw + pc.tw_count);
+  r.issued = reinterpret_cast<int*>(r.mbar + pc.nbuf);
   return r;
 }
 
@@ -129,8 +130,8 @@ P3G_D void strided_decode(const SPipeParams& q, int tile, int& xt, int& o1, int&
 // o2) into dst, without a commit; the DCT-I/DST-I extension rows are extra
 // copies of the same elements (the DST-I negation happens in the fix-up
 // step).
-template <class P, bool WALK = false>
-P3G_D void strided_copy(const SParams& s, typename P::W* dst, int xt, int o1, int o2) {
+template <class P, bool WALK = false, class TH = CtaThreads>
+P3G_D void strided_copy(const SParams& s, typename P::W* dst, int xt, int o1, int o2, const TH& th = TH()) {
   using W = typename P::W;
   const int M = s.M, L = s.L;
   const int ph = strided_phase(s, o1, o2);
@@ -169,7 +170,7 @@ P3G_D void strided_copy(const SParams& s, typename P::W* dst, int xt, int o1, in
       }
     }
   };
-  const int T = blockDim.x;
+  const int T = th.count(), tid = th.tid();
   if constexpr (esz == 8) {
     // 8-byte elements with adjacent columns: two columns per 16-byte copy when
     // the tile's first column and the row stride keep the pair 16-byte aligned
@@ -185,8 +186,8 @@ P3G_D void strided_copy(const SParams& s, typename P::W* dst, int xt, int o1, in
         // rows with addresses advanced by constant steps (faster inside the
         // batch kernel; slower for the long lines of the pass kernels, whose
         // loads are measured ~10 % slower with it)
-        const int m = 2 * (threadIdx.x & (MP - 1));
-        const int j0 = threadIdx.x >> lmp, js = T >> lmp;
+        const int m = 2 * (tid & (MP - 1));
+        const int j0 = tid >> lmp, js = T >> lmp;
         const char* g = in + (ib + m + (long long)j0 * s.in_axis) * esz;
         const long long gstep = (long long)js * s.in_axis * esz;
         W* d = dst + j0 * M + m;
@@ -194,7 +195,7 @@ P3G_D void strided_copy(const SParams& s, typename P::W* dst, int xt, int o1, in
         for (int j = j0; j < L; j += js, g += gstep, d += js * M) cp_async16(d, g, 16u);
         return;
       }
-      for (int e = threadIdx.x; e < MP * L; e += T) {
+      for (int e = tid; e < MP * L; e += T) {
         const int m = 2 * (e & (MP - 1));
         const int j = e >> lmp;
         const int src = j >= s.lmap_a1 ? j - s.lmap_d : (j < s.lmap_a0 ? j : -1);
@@ -220,30 +221,59 @@ P3G_D void strided_copy(const SParams& s, typename P::W* dst, int xt, int o1, in
   }
   if (s.in_xs != 1) {  // rows adjacent in memory (STRIDE1 user layout): rows fastest
     const FastDiv div_l(L);
-    for (int e = threadIdx.x; e < M * L; e += T) {
+    for (int e = tid; e < M * L; e += T) {
       const int m = (int)div_l.div(e);
       one(m, e - m * L);
     }
   } else if ((T & (M - 1)) == 0) {  // each thread keeps one column m: rows strided by T/M
-    const int m = threadIdx.x & (M - 1);
-    for (int j = threadIdx.x >> s.log2m; j < L; j += T >> s.log2m) one(m, j);
+    const int m = tid & (M - 1);
+    for (int j = tid >> s.log2m; j < L; j += T >> s.log2m) one(m, j);
   } else {
-    for (int e = threadIdx.x; e < M * L; e += T) one(e & (M - 1), e >> s.log2m);
+    for (int e = tid; e < M * L; e += T) one(e & (M - 1), e >> s.log2m);
   }
 }
 
-// Copies of one tile into buffer b.  TMA: thread 0 arms the barrier and
-// issues the boxes.  cp.async: every thread, one commit group per call.
+// A buffer's loads are counted when they are issued.  The wait for use `use`
+// of a buffer first waits (bounded) until that load has been issued: groups
+// drift, and a group that asked for a parity two phases ahead of the barrier
+// would take the phase before last for its own.  Load `use` is issued only
+// after tile use - 1 of the buffer was consumed, so from then on the parity
+// is unambiguous.
+P3G_D void ring_mark_issued(int* issued) {
+  __threadfence_block();
+  *reinterpret_cast<volatile int*>(issued) = *issued + 1;
+}
+P3G_D bool ring_wait(uint64_t* bar, const int* issued, int use, int* err) {
+  const volatile int* n = issued;
+  if (*n <= use) {
+    const uint64_t t0 = global_ns();
+    uint32_t i = 0;
+    while (*n <= use) {
+      if (++i >= kMbarSpinLimit || ((i & 15) == 15 && global_ns() - t0 > kMbarWaitNs)) {
+        if (err) atomicExch(err, kErrMbarTimeout);
+        return false;
+      }
+      if (i > 16) __nanosleep(32);
+    }
+  }
+  __threadfence_block();
+  return mbar_wait_bounded(bar, use & 1, err);
+}
+
+// Copies of one tile into buffer b by one group.  TMA: its first thread arms
+// the buffer's barrier and issues the boxes.  cp.async: every thread of the
+// group copies its share and arrives on the barrier when it has landed.
 template <class P>
-P3G_D void strided_issue(const SPipeParams& q, const CUtensorMap* tin, int tile, int b) {
+P3G_D void strided_issue(const SPipeParams& q, const CUtensorMap* tin, int tile, int b, const GroupThreads& th) {
   using W = typename P::W;
   const StridedSmem<P> sm = strided_smem<P>(q.c);
   W* dst = sm.buf0 + b * q.c.buf_elems;
   int xt, o1, o2;
   strided_decode(q, tile, xt, o1, o2);
   if (q.use_tma) {
-    if (threadIdx.x == 0) {
+    if (th.t == 0) {
       constexpr int kWords = sizeof(W) / 4;
+      ring_mark_issued(&sm.issued[b]);
       fence_proxy_async_smem();
       mbar_arrive_expect_tx(&sm.mbar[b], (uint32_t)(q.nbox * q.box_bytes + q.tx_extra));
       for (int i = 0; i < q.nbox; ++i)
@@ -251,22 +281,23 @@ P3G_D void strided_issue(const SPipeParams& q, const CUtensorMap* tin, int tile,
     }
     return;
   }
-  strided_copy<P>(q.s, dst, xt, o1, o2);
-  cp_async_commit();
+  if (th.t == 0) ring_mark_issued(&sm.issued[b]);
+  strided_copy<P>(q.s, dst, xt, o1, o2, th);
+  cp_async_mbar_arrive(&sm.mbar[b]);
 }
 
 // Fix-up of a loaded strided tile, element-wise in place: user format ->
 // working format, DST-I negation, DCT-I mirror after a TMA load (tma).
 // Ends with a barrier when it changed anything.
-template <class P>
-P3G_D void strided_fix(const SParams& s, bool tma, typename P::W* sm, int k, uint32_t& amax) {
+template <class P, class TH = CtaThreads>
+P3G_D void strided_fix(const SParams& s, bool tma, typename P::W* sm, int k, uint32_t& amax, const TH& th = TH()) {
   using W = typename P::W;
   using C = typename P::C;
   const bool raw_user = s.in_user != 0 && P::kF64;  // binary32 user data is the working format
   if (raw_user || s.pre == 2 || (tma && s.pre == 1)) {
     const int M = s.M, L = s.L;
     const int rows = tma ? L : s.N;
-    for (int e = threadIdx.x; e < M * rows; e += blockDim.x) {
+    for (int e = th.tid(); e < M * rows; e += th.count()) {
       const int m = e & (M - 1);
       const int j = e >> s.log2m;
       C v;
@@ -282,14 +313,15 @@ P3G_D void strided_fix(const SParams& s, bool tma, typename P::W* sm, int k, uin
       sm[j * M + m] = w;
       if (tma && s.pre == 1 && j >= 1 && j <= L - 2) sm[(2 * (L - 1) - j) * M + m] = w;
     }
-    __syncthreads();
+    th.sync();
   }
 }
 
 // Store of a transformed strided tile with the pruning map and the output
 // format (DST-I output rows k+1 times i).
-template <class P>
-P3G_D void strided_store(const SParams& s, const typename P::W* sm, int xt, int o1, int o2, int kb) {
+template <class P, class TH = CtaThreads>
+P3G_D void strided_store(const SParams& s, const typename P::W* sm, int xt, int o1, int o2, int kb,
+                         const TH& th = TH()) {
   using C = typename P::C;
   const int M = s.M;
   const int ph = strided_phase(s, o1, o2);  // the tile's columns as loaded by strided_copy
@@ -304,11 +336,11 @@ P3G_D void strided_store(const SParams& s, const typename P::W* sm, int xt, int 
     else v = P::from_w(sm[k * M + m]);
     store_elem<P>(s.out, s.out_user, obase + strided_col_out(s, c) + (long long)jo * s.out_axis, v, kb);
   };
-  const int T = blockDim.x;
+  const int T = th.count(), tid = th.tid();
   if (s.tw4) {
     // four-step twiddle w_N^(o1 jo) on every stored element (rows one to one)
     const unsigned long long n4 = (unsigned long long)s.tw4_n;
-    for (int e = threadIdx.x; e < M * s.Lout; e += T) {
+    for (int e = tid; e < M * s.Lout; e += T) {
       const int m = e & (M - 1), jo = e >> s.log2m;
       if (x0 + m >= xend) continue;
       const int c = x0 + m < s.X ? x0 + m : x0 + m - s.X;
@@ -323,10 +355,10 @@ P3G_D void strided_store(const SParams& s, const typename P::W* sm, int xt, int 
     // rows stored one to one (no pruning gap, no DST shift): each thread keeps
     // one column and walks its rows with a shared-memory address and an
     // output pointer advanced by constant steps
-    const int m = threadIdx.x & (M - 1);
+    const int m = tid & (M - 1);
     if (x0 + m >= xend) return;
     const int c = x0 + m < s.X ? x0 + m : x0 + m - s.X;
-    const int j0 = threadIdx.x >> s.log2m, js = T >> s.log2m;
+    const int j0 = tid >> s.log2m, js = T >> s.log2m;
     using W = typename P::W;
     uint32_t a = (uint32_t)__cvta_generic_to_shared(sm) + (uint32_t)((j0 * M + m) * (int)sizeof(W));
     const uint32_t astep = (uint32_t)(T * (int)sizeof(W));
@@ -345,16 +377,16 @@ P3G_D void strided_store(const SParams& s, const typename P::W* sm, int xt, int 
   }
   if (s.out_xs != 1) {  // rows adjacent in memory (STRIDE1 user layout): rows fastest
     const FastDiv div_lo(s.Lout);
-    for (int e = threadIdx.x; e < M * s.Lout; e += T) {
+    for (int e = tid; e < M * s.Lout; e += T) {
       const int m = (int)div_lo.div(e);
       if (x0 + m < xend) one(m, e - m * s.Lout);
     }
   } else if ((T & (M - 1)) == 0) {
-    const int m = threadIdx.x & (M - 1);
+    const int m = tid & (M - 1);
     if (x0 + m < xend)
-      for (int jo = threadIdx.x >> s.log2m; jo < s.Lout; jo += T >> s.log2m) one(m, jo);
+      for (int jo = tid >> s.log2m; jo < s.Lout; jo += T >> s.log2m) one(m, jo);
   } else {
-    for (int e = threadIdx.x; e < M * s.Lout; e += T) {
+    for (int e = tid; e < M * s.Lout; e += T) {
       const int m = e & (M - 1);
       if (x0 + m < xend) one(m, e >> s.log2m);
     }
@@ -368,106 +400,124 @@ P3G_D void cp_async_wait_ahead(int nbuf) {
   else cp_async_wait<1>();
 }
 
-template <class P, int DIR, int E>
-__global__ void __launch_bounds__(PipeLimits<P, E>::kMaxThreads, PipeLimits<P, E>::kMinBlocks)
+// The CTA's threads form `groups` groups that each transform whole tiles with
+// barriers of their own; the tiles go round the groups, and round a ring of
+// nbuf > groups buffers.  While the groups work, the loads of the next tiles
+// are in flight in the other buffers: a group that has finished a tile hands
+// its buffer back by loading the tile nbuf places further on into it, for
+// whichever group's turn that will be.  With one group of all threads every
+// warp is in the same phase of a tile, and the FMA pipes idle through its
+// shared-memory exchanges and barriers; two or more groups drift apart and
+// fill each other's gaps.
+template <class P, int DIR, int MODE>
+__global__ void __launch_bounds__(strided_max_threads(MODE), 1)
     k_strided_pipe(const __grid_constant__ CUtensorMap tin, const __grid_constant__ CUtensorMap tout,
                    const __grid_constant__ SPipeParams pp, const StagePlan* __restrict__ sp,
                    const float4* __restrict__ tw_g) {
-  const int nb = pp.c.nbuf;
-  const int la = nb - 1 - pp.tma_store;  // tiles loaded ahead of the current one
+  const int nb = pp.c.nbuf, G = pp.c.groups;
+  const int step = (int)gridDim.x;
   {
     const StridedSmem<P> sm = strided_smem<P>(pp.c);
     for (int i = threadIdx.x; i < pp.c.tw_count; i += blockDim.x) sm.tw[i] = __ldg(tw_g + pp.c.tw_base + i);
-    if (threadIdx.x == 0 && pp.use_tma) {
-      for (int i = 0; i < nb; ++i) mbar_init(&sm.mbar[i], 1);
+    if (threadIdx.x == 0) {
+      for (int i = 0; i < nb; ++i) {
+        mbar_init(&sm.mbar[i], pp.use_tma ? 1 : pp.c.gthreads);
+        sm.issued[i] = 0;
+      }
+      sm.issued[nb] = 0;
       mbar_fence_init();
     }
   }
   __syncthreads();
   const int k = range_k(pp.s.range);
   uint32_t amax = 0;
-  int it = 0;
-  int tile = blockIdx.x;
-  // tiles of the first la iterations in flight before the loop
-  for (int j = 0; j < la; ++j) {
-    const int t = tile + j * (int)gridDim.x;
-    if (t < pp.c.ntiles) strided_issue<P>(pp, &tin, t, j);
-    else if (!pp.use_tma) cp_async_commit();
-  }
-  int b = 0, ph = 0;  // buffer of iteration it and the parity of its use
+  const int g = (int)threadIdx.x / pp.c.gthreads;
+  const GroupThreads th{(int)threadIdx.x - g * pp.c.gthreads, pp.c.gthreads, 1 + g};
+  // one group alone (nb >= 3) loads one tile ahead, into the buffer whose store
+  // was issued two tiles ago: its first thread never waits for a store that
+  // has just begun
+  const bool lag = G == 1 && nb >= 3 && pp.tma_store;
+  const int first = lag ? 1 : nb;
+  // the first tile of every buffer
+  for (int j = 0, tile = blockIdx.x; j < first && tile < pp.c.ntiles; ++j, tile += step)
+    if (pp.use_tma ? g == 0 : j % G == g) strided_issue<P>(pp, &tin, tile, j, th);
+  int b = g, use = 0;  // this tile's buffer and how often it was used before
+  int rtile = -1, rbuf = 0;  // a load to issue once the TMA store has read the buffer
 #pragma unroll 1
-  for (; tile < pp.c.ntiles; tile += gridDim.x, ++it) {
-    bool ok = true;
-    {
-      const SPipeParams& q = pp;
-      // into the buffer of iteration it + la - nb (with TMA stores: the
-      // store issued two iterations ago, which must have read its tile)
-      const int ahead = tile + la * (int)gridDim.x;
-      const int bl = b + la >= nb ? b + la - nb : b + la;
-      if (ahead < q.c.ntiles) {
-        if (q.tma_store && threadIdx.x == 0) bulk_wait_read<1>();
-        strided_issue<P>(q, &tin, ahead, bl);
-      } else if (!q.use_tma) {
-        cp_async_commit();  // one group per iteration
-      }
-      if (q.use_tma) ok = mbar_wait_bounded(&strided_smem<P>(q.c).mbar[b], ph, q.c.err);
-      else cp_async_wait_ahead(nb);
+  for (int tile = blockIdx.x + g * step; tile < pp.c.ntiles; tile += G * step) {
+    if (lag && tile + step < pp.c.ntiles && th.t == 0) {
+      bulk_wait_read<1>();
+      strided_issue<P>(pp, &tin, tile + step, b + 1 == nb ? 0 : b + 1, th);
     }
-    if (__syncthreads_or(!ok)) break;
-    strided_fix<P>(pp.s, pp.use_tma != 0, strided_smem<P>(pp.c).buf0 + b * pp.c.buf_elems, k, amax);
+    const bool ok = ring_wait(&strided_smem<P>(pp.c).mbar[b], &strided_smem<P>(pp.c).issued[b], use, pp.c.err);
+    if (th.sync_or(!ok)) {
+      if (th.t == 0) strided_smem<P>(pp.c).issued[nb] = 1;
+      break;
+    }
+    if (rtile >= 0 && th.t == 0) {
+      bulk_wait_read<0>();
+      strided_issue<P>(pp, &tin, rtile, rbuf, th);
+    }
+    strided_fix<P>(pp.s, pp.use_tma != 0, strided_smem<P>(pp.c).buf0 + b * pp.c.buf_elems, k, amax, th);
     {
-      const SPipeParams& q = pp;
-      const StridedSmem<P> sm = strided_smem<P>(q.c);
-      Tile<P> t{sm.buf0 + b * q.c.buf_elems, nullptr, q.s.M, q.s.log2m, 1, q.s.M};
-      cta_fft<P, DIR, E, kPointMajor, kRawNone, PipeMaxR<P, E>::value>(t, sp, sm.tw, q.c.tw_base);
+      const StridedSmem<P> sm = strided_smem<P>(pp.c);
+      Tile<P, GroupThreads> t{sm.buf0 + b * pp.c.buf_elems, nullptr, pp.s.M, pp.s.log2m, 1, pp.s.M, 0, 0, nullptr, th};
+      constexpr int E = MODE == kStridedSmall ? StridedElems<P>::value / 2 : StridedElems<P>::value;
+      constexpr bool kFull = MODE == kStridedFull || MODE == kStridedFullWide;
+      cta_fft<P, DIR, E, kPointMajor, kRawNone, E, kFull>(t, sp, sm.tw, pp.c.tw_base);
     }
     {
       int xt, o1, o2;
       strided_decode(pp, tile, xt, o1, o2);
-      const typename P::W* tb = strided_smem<P>(pp.c).buf0 + b * pp.c.buf_elems;
+      typename P::W* tb = strided_smem<P>(pp.c).buf0 + b * pp.c.buf_elems;
+      rtile = !lag && tile + nb * step < pp.c.ntiles ? tile + nb * step : -1;
+      rbuf = b;
       if (pp.tma_store) {
         if constexpr (P::kF64) {
           if (pp.s.out_user) {  // binary64 user format, converted in place (16 bytes each)
-            typename P::W* tm = strided_smem<P>(pp.c).buf0 + b * pp.c.buf_elems;
             const int ne = pp.s.Lout * pp.s.M;
-            for (int e = threadIdx.x; e < ne; e += blockDim.x)
-              reinterpret_cast<typename P::UC*>(tm)[e] = P::to_uc(P::from_w(tm[e]), k);
+            for (int e = th.t; e < ne; e += th.n)
+              reinterpret_cast<typename P::UC*>(tb)[e] = P::to_uc(P::from_w(tb[e]), k);
           }
         }
         fence_proxy_async_smem();  // this thread's tile writes, before the async-proxy reads
-        __syncthreads();
-        if (threadIdx.x == 0) {
+        th.sync();
+        if (th.t == 0) {
           constexpr int kWords = sizeof(typename P::W) / 4;
           for (int i = 0; i < pp.onbox; ++i)
             tma_store_4d(&tout, tb + i * pp.obrows * pp.s.M, xt * pp.s.M * kWords, i * pp.obrows, o1, o2);
           bulk_commit_group();
         }
+        if (nb == G && rtile >= 0) {  // no spare buffer: the next load is this group's own
+          if (th.t == 0) bulk_wait_read<0>();
+          th.sync();
+          strided_issue<P>(pp, &tin, rtile, rbuf, th);
+          rtile = -1;
+        }
       } else {
-        strided_store<P>(pp.s, tb, xt, o1, o2, k);
+        strided_store<P>(pp.s, tb, xt, o1, o2, k, th);
+        th.sync();
+        if (rtile >= 0) strided_issue<P>(pp, &tin, rtile, rbuf, th);
+        rtile = -1;
       }
     }
-    __syncthreads();
-    if (++b == nb) {
-      b = 0;
-      ph ^= 1;
+    b += G;
+    if (b >= nb) {
+      b -= nb;
+      ++use;
     }
   }
-  // early exit after a timed-out wait: wait (bounded) for the copies of the
-  // tiles issued and not yet consumed
-  if (pp.use_tma) {
-    if (threadIdx.x == 0) {
-      const StridedSmem<P> sm = strided_smem<P>(pp.c);
-      for (int j = 0; j <= la; ++j)
-        if (tile + j * (int)gridDim.x < pp.c.ntiles) {
-          const int i = it + j;
-          mbar_wait_bounded(&sm.mbar[i % nb], (i / nb) & 1, nullptr);
-        }
-    }
-  } else {
-    cp_async_wait<0>();
-  }
+  if (!pp.use_tma) cp_async_wait<0>();
   // the tile stores must have completed before the CTA's shared memory goes
-  if (pp.tma_store && threadIdx.x == 0) bulk_wait_all();
+  if (pp.tma_store && th.t == 0) bulk_wait_all();
+  __syncthreads();
+  // a wait timed out: loads may be in flight that no group waits for
+  if (threadIdx.x == 0 && pp.use_tma) {
+    const StridedSmem<P> sm = strided_smem<P>(pp.c);
+    if (sm.issued[nb])
+      for (int i = 0; i < nb; ++i)
+        if (sm.issued[i]) mbar_wait_bounded(&sm.mbar[i], (sm.issued[i] - 1) & 1, nullptr);
+  }
   range_flush(pp.s.range, amax);
 }
 

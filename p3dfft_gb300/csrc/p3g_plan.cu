@@ -15,6 +15,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <map>
 #include <mutex>
 #include <set>
 #include <string>
@@ -133,24 +134,71 @@ static bool factor(int n, int max_pow2, std::vector<int>& radices) {
   return (int)radices.size() <= kMaxStages;
 }
 
+// The plan's twiddle table.  Every twiddle of an axis is a root of unity of
+// its stage's sub-transform length, taken from one table of that length's
+// roots (half of them evaluated, with angles reflected into [0, pi/4]; the
+// rest are conjugates), and axes of the same length share their stage plan and
+// its slice of the table.
 struct HostTw {
   std::vector<float4> v;
-  int mark = 0;  // start of the axis being built
-  int push_root(long long num, long long den) {  // exp(-2 pi i num/den), split into hi/lo
+  int mark = 0, count = 0;  // slice of the axis built last
+  std::map<long long, std::vector<float4>> roots;  // by length: exp(-2 pi i t / n)
+  struct Built {
+    StagePlan sp;
+    int lo, cnt;
+  };
+  std::map<std::pair<int, int>, Built> built;  // by (length, largest power-of-two radix)
+
+  // exp(-2 pi i t / n) for 0 <= t < n, split into hi/lo
+  static float4 root(long long t, long long n) {
     const long double two_pi = 6.283185307179586476925286766559L;
-    long long t = num % den;
-    const long double ang = -two_pi * (long double)t / (long double)den;
-    const long double c = cosl(ang), s = sinl(ang);
+    // reflect the angle 2 pi t / n into [0, pi/4]
+    long long num = 8 * t;
+    bool neg_s = false, neg_c = false, swap = false;
+    if (num > 4 * n) {
+      num = 8 * n - num;
+      neg_s = true;
+    }
+    if (num > 2 * n) {
+      num = 4 * n - num;
+      neg_c = true;
+    }
+    if (num > n) {
+      num = 2 * n - num;
+      swap = true;
+    }
+    const long double ang = two_pi * (long double)num / (long double)(8 * n);
+    long double c = cosl(ang), s = sinl(ang);
+    if (swap) std::swap(c, s);
+    if (neg_c) c = -c;
+    if (!neg_s) s = -s;  // forward sign
     const float ch = (float)c, sh = (float)s;
-    const float cl = (float)(c - (long double)ch), sl = (float)(s - (long double)sh);
-    v.push_back(make_float4(ch, sh, cl, sl));
+    return make_float4(ch, sh, (float)(c - (long double)ch), (float)(s - (long double)sh));
+  }
+  const std::vector<float4>& table(long long n) {
+    std::vector<float4>& r = roots[n];
+    if (!r.empty()) return r;
+    r.resize(n);
+    for (long long t = 0; 2 * t <= n; ++t) {
+      r[t] = root(t, n);
+      if (t > 0) r[n - t] = make_float4(r[t].x, -r[t].y, r[t].z, -r[t].w);
+    }
+    return r;
+  }
+  int push_root(long long num, long long den) {  // exp(-2 pi i num/den)
+    v.push_back(table(den)[num % den]);
     return (int)v.size() - 1;
   }
 };
 
-
-
 static bool build_stages(int n, int max_pow2, HostTw& tw, StagePlan& sp) {
+  const auto known = tw.built.find({n, max_pow2});
+  if (known != tw.built.end()) {
+    sp = known->second.sp;
+    tw.mark = known->second.lo;
+    tw.count = known->second.cnt;
+    return true;
+  }
   std::memset(&sp, 0, sizeof(sp));
   tw.mark = (int)tw.v.size();
   sp.n = n;
@@ -162,16 +210,10 @@ static bool build_stages(int n, int max_pow2, HostTw& tw, StagePlan& sp) {
     const int r = rad[s];
     sp.radix[s] = r;
     sp.ns[s] = ns;
-    switch (r) {
-      case 32: sp.cnt[0]++; break;
-      case 16: sp.cnt[1]++; break;
-      case 8: sp.cnt[2]++; break;
-      case 4: sp.cnt[3]++; break;
-      case 2: sp.cnt[4]++; break;
-      case 3: sp.cnt[5]++; break;
-      case 5: sp.cnt[6]++; break;
-      default: sp.has_generic = 1; break;
-    }
+    int fam = 0;
+    while (fam < kNumFamilies && kFamilies[fam] != r) ++fam;
+    if (fam < kNumFamilies) sp.fam += 1ull << (4 * fam);
+    else sp.has_generic = 1;
     sp.tw_off[s] = (int)tw.v.size();
     if (ns > 1) {
       for (int k = 0; k < ns; ++k)
@@ -180,10 +222,12 @@ static bool build_stages(int n, int max_pow2, HostTw& tw, StagePlan& sp) {
       tw.push_root(0, 1);  // keep offsets valid
     }
     sp.root_off[s] = (int)tw.v.size();
-    if (r != 2 && r != 3 && r != 4 && r != 5 && r != 8 && r != 16 && r != 32)
+    if (fam == kNumFamilies)
       for (int m = 0; m < r; ++m) tw.push_root(m, r);
     ns *= r;
   }
+  tw.count = (int)tw.v.size() - tw.mark;
+  tw.built[{n, max_pow2}] = HostTw::Built{sp, tw.mark, tw.count};
   return true;
 }
 
@@ -191,6 +235,20 @@ static int ilog2(int v) {
   int l = 0;
   while ((1 << l) < v) ++l;
   return l;
+}
+
+static int round_threads(long long t) { return (int)std::max(32LL, (t + 31) / 32 * 32); }
+
+// Threads (a multiple of 32) that a tile of M lines needs for every register
+// stage of its plan in a grouped kernel of E elements per thread.
+static int stage_threads(const StagePlan& sp, long long M, int E) {
+  const long long points = M * sp.n;
+  long long t = (points + E - 1) / E;
+  for (int s = 0; s < sp.nstages; ++s) {
+    const int r = sp.radix[s], b = stage_butterflies(E, r, true);
+    t = std::max(t, (points / r + b - 1) / b);
+  }
+  return round_threads(t);
 }
 
 // Tile sizing: M lines of n points so that one tile holds about `budget`
@@ -204,11 +262,7 @@ static bool size_tile(AxisPlan& ap, int n, int lines_avail, bool f64, int max_m 
   const size_t esize = f64 ? 16 : 8;
   int M = 1;
   while (M * 2 * n <= budget && M * 2 <= (1 << ilog2(lines_avail > 0 ? lines_avail : 1)) && M * 2 <= max_m) M *= 2;
-  auto threads_for = [&](int m) {
-    int t = (m * n + kElemsPerThread - 1) / kElemsPerThread;
-    t = (t + 31) / 32 * 32;
-    return t < 32 ? 32 : t;
-  };
+  auto threads_for = [&](int m) { return round_threads(((long long)m * n + kElemsPerThread - 1) / kElemsPerThread); };
   while (M > 1 && threads_for(M) > max_threads) M /= 2;
   if (threads_for(M) > max_threads) return false;
   ap.n = n;
@@ -219,48 +273,131 @@ static bool size_tile(AxisPlan& ap, int n, int lines_avail, bool f64, int max_m 
   return ap.smem <= 227 * 1024;
 }
 
-// Launch shape of a pipelined kernel with E elements per thread: the most
+// Launch shape of an X pass kernel with E elements per thread: the most
 // threads per CTA and the registers per thread its launch bounds allow.
 template <class P, int E>
-static void pipe_shape(bool xk, int& max_threads, int& regs) {
-  max_threads = xk ? XPipeLimits<P, E>::kMaxThreads : PipeLimits<P, E>::kMaxThreads;
-  const int blocks = xk ? XPipeLimits<P, E>::kMinBlocks : PipeLimits<P, E>::kMinBlocks;
-  regs = std::min(255, 65536 / (max_threads * blocks));
+static void pipe_shape(int& max_threads, int& regs) {
+  max_threads = XPipeLimits<P, E>::kMaxThreads;
+  regs = std::min(255, 65536 / (max_threads * XPipeLimits<P, E>::kMinBlocks));
 }
 
-// Pipelined kernels: two tile buffers (1 KB aligned), the axis's twiddles
-// and two mbarriers in shared memory.  kind: 0 strided, 1 r2c, 2 c2r.  The
-// elements per thread follow the axis's stage plans: 16 on F64 and 32 on F32
-// when the axis has a wide plan, else 8 and 16.
+// Strided pipelined kernel (k_strided_pipe): one CTA per SM of g groups of tg
+// threads, each group on tiles of M columns, and a ring of nbuf buffers (1 KB
+// aligned), the axis's twiddles and the buffers' mbarriers in shared memory.
+// X columns and O1 row sets are the pass's extents; tstore: the tiles leave by
+// thread stores (binary32 user rows); far_rows: a line's points lie 3 MB or
+// more apart in the pass's input or output.
+//
+// The stage plan (wide, or narrow with half the points per thread), the tile
+// width M and the groups are those with the least estimate of
+//   (tiles per SM) x (points per tile, idle lanes included) x (clocks per
+//   point) / (row efficiency x overlap) + latency of one tile,
+// row efficiency being that of the tile's row segments in memory: 32-byte
+// segments ran the 1024-point binary32 Y pass at 4.0 ms against 1.95 ms with
+// 64 bytes.  Fewer than 12 busy warps or a single group leave the FMA pipes
+// idle through the tiles' exchanges (1024-point binary64 Y: 6.9 ms with one
+// group of 256 threads, 5.3 ms with two).  The latency term matters when the
+// grid has fewer tiles than the GPU has groups: half the points per thread
+// halve the length of a thread's serial chain.
+static void size_strided(AxisPlan& ap, bool f64, int X, int O1, int max_m, int sm_count, bool tstore,
+                         bool far_rows) {
+  ap.pipe_ok = false;
+  if (ap.sp.nstages < 1 || ap.sp.has_generic || ap.n < 2) return;
+  const size_t esize = f64 ? 16 : 8;
+  const int Emax = f64 ? StridedElems<PathF64>::value : StridedElems<PathF32>::value;
+  const int n = ap.n;
+  const size_t room = 227 * 1024;
+  const int wide_index = ap.spw_index;
+  int use_wide = wide_index;
+  double best = 1e300;
+  for (int narrow = wide_index >= 0 ? 0 : 1; narrow < 2; ++narrow) {
+    const StagePlan& sp = narrow ? ap.sp : ap.spw;
+    bool pow2 = true;
+    int rmax = 0;
+    for (int i = 0; i < sp.nstages; ++i) {
+      pow2 = pow2 && (sp.radix[i] & (sp.radix[i] - 1)) == 0;
+      rmax = std::max(rmax, sp.radix[i]);
+    }
+    const size_t fixed = 1024 + (size_t)(narrow ? ap.tw_cnt : ap.tw_cnt_w) * 16 + 256;
+    for (int E = Emax; E >= Emax / 2 && E >= rmax; E /= 2) {
+      for (int M = 1; M <= max_m && M <= (1 << ilog2(X)); M *= 2) {
+        const int tg = stage_threads(sp, M, E);
+        const bool full = pow2 && (long long)M * n == (long long)tg * E && E == Emax;
+        // binary32 FULL passes that store by threads run one group with twice
+        // the registers: at 128 the spilled words and the stores share what is
+        // left of the L1 (1024-point Z forward 5.4 ms against 2.5 ms).  So do
+        // those with far rows, where every row of a tile is in a memory page
+        // of its own and groups that drift apart spread over more pages at a
+        // time (Y of 1024^3, 4.2 MB apart: 1.95 ms with two groups, 1.81 ms
+        // with one; of 768 x 1024 x 540, 1.7 MB apart: 0.59 against 0.73 ms)
+        const StridedMode mode =
+            E < Emax ? kStridedSmall : (!full ? kStridedGeneral : (!f64 && (tstore || far_rows) ? kStridedFullWide : kStridedFull));
+        const int max_threads = strided_max_threads(mode);
+        const size_t buf = ((size_t)M * n * esize + 1023) / 1024 * 1024;
+        if (tg > strided_max_threads(kStridedGeneral) || fixed + 2 * buf > room) break;
+        if (tg > max_threads) continue;
+        const int fit = (int)std::min<size_t>((room - fixed) / buf, kMaxTileBuffers);
+        const double tiles = (double)((X + M - 1) / M) * O1;
+        const double per_sm = std::ceil(tiles / sm_count);
+        // groups: as many as the threads, one spare buffer and the tiles allow
+        const int g = (int)std::max(
+            1.0, std::min({(double)(max_threads / tg), (double)kMaxGroups, (double)(fit - 1), per_sm}));
+        // half the points per thread: only where every tile has a group of its own
+        if (E < Emax && per_sm > g) continue;
+        const size_t row = M * esize;
+        const double rows = row >= 128 ? 1.0 : (row >= 64 ? 0.97 : (row >= 32 ? 0.45 : 0.25));
+        const double warps = (mode == kStridedFullWide ? 1.5 : 1.0) * g * tg / 32;
+        const double overlap = std::min(1.0, warps / 12) * (g >= 2 || mode == kStridedFullWide ? 1.0 : 0.8);
+        const double clocks = (f64 ? 1.0 : 0.35) * sp.nstages;
+        const double t = per_sm * tg * E * clocks / (rows * overlap) + 100.0 * E * sp.nstages / (f64 ? 1 : 2);
+        if (t < best * 0.999) {
+          best = t;
+          use_wide = narrow ? -1 : wide_index;
+          ap.pipe_ok = true;
+          ap.pipe_m = M;
+          ap.pipe_log2m = ilog2(M);
+          ap.pipe_mode = mode;
+          ap.pipe_g = g;
+          ap.pipe_threads = g * tg;
+          // more loads in flight than one beyond the groups pay off only where
+          // the tiles leave by TMA (binary32 512^3 Y: 0.19 ms with two, 0.26
+          // with one; 540-point binary32 Z: 1.60 with two, 1.55 with one)
+          ap.pipe_nbuf = std::min(fit, g + (tstore ? 1 : 2));
+          ap.buf_elems = (int)(buf / esize);
+          ap.pipe_smem = fixed + ap.pipe_nbuf * buf;
+        }
+      }
+    }
+  }
+  if (ap.pipe_ok) ap.spw_index = use_wide;
+}
+
+// X pass kernels: two or three tile buffers (1 KB aligned) and their
+// mbarriers in shared memory.  kind: 1 r2c, 2 c2r.  The elements per thread
+// follow the axis's stage plans: 8 on F64; 32 on F32 with the wide plan, else 16.
 static void size_pipe(AxisPlan& ap, int kind, bool f64, int thread_cap = 0) {
   ap.pipe_ok = false;
   if (ap.sp.nstages < 1 || ap.sp.has_generic || ap.n < 2) return;
   const size_t esize = f64 ? 16 : 8;
-  const bool xk = kind != 0;  // X kernels have their own launch shape (XPipeLimits)
   const int E = f64 ? (ap.spw_index >= 0 ? 16 : 8) : (ap.spw_index >= 0 ? 32 : 16);
   ap.pipe_e = E;
   int max_threads = 0, regs_max = 0;
   if (f64) {
-    if (E == 16) pipe_shape<PathF64, 16>(xk, max_threads, regs_max);
-    else pipe_shape<PathF64, 8>(xk, max_threads, regs_max);
-  } else if (E == 32) pipe_shape<PathF32, 32>(xk, max_threads, regs_max);
-  else pipe_shape<PathF32, 16>(xk, max_threads, regs_max);
+    if (E == 16) pipe_shape<PathF64, 16>(max_threads, regs_max);
+    else pipe_shape<PathF64, 8>(max_threads, regs_max);
+  } else if (E == 32) pipe_shape<PathF32, 32>(max_threads, regs_max);
+  else pipe_shape<PathF32, 16>(max_threads, regs_max);
   if (thread_cap > 0 && thread_cap < max_threads) max_threads = thread_cap;
-  const bool tw_shared = !xk;  // the X kernels read the global table
   const int n = ap.n;
   const int nh = n / 2 + 1;
-  auto threads_for = [&](int M) {
-    int t = (M * n + E - 1) / E;
-    t = (t + 31) / 32 * 32;
-    return t < 32 ? 32 : t;
-  };
+  auto threads_for = [&](int M) { return round_threads((M * n + E - 1) / E); };
   auto smem_for = [&](int M, size_t& buf_bytes, int nbuf = 2) {
-    // buffer stride rounded to 1 KB so every buffer (TMA destinations) stays aligned
+    // buffer stride rounded to 1 KB so every buffer stays aligned
     const int raw = 2 * xc2r_raw_stride(nh, (int)esize);  // c2r raw line pair
     const int ls = ap.pipe_ls();
-    const size_t need = (size_t)(kind == 0 ? M * n : M * (ls > raw ? ls : raw)) * esize;
+    const size_t need = (size_t)(M * (ls > raw ? ls : raw)) * esize;
     buf_bytes = (need + 1023) / 1024 * 1024;
-    return 1024 + nbuf * buf_bytes + (tw_shared ? (size_t)ap.pipe_tw_cnt() * 16 : 0) + 8 * nbuf + 16;
+    return 1024 + nbuf * buf_bytes + 8 * nbuf + 16;
   };
   // resident warps per SM for tile width M: registers per thread from the
   // kernel's launch bounds, 2048 threads and ~228 KB of shared memory per SM
@@ -268,16 +405,13 @@ static void size_pipe(AxisPlan& ap, int kind, bool f64, int thread_cap = 0) {
     const int t = threads_for(M);
     size_t bb;
     const size_t sm = smem_for(M, bb, nbuf);
-    const int regs = regs_max;
-    int b = 65536 / (regs * t);
+    int b = 65536 / (regs_max * t);
     b = std::min(b, 2048 / t);
     b = std::min(b, (int)((228 * 1024) / sm));
     return b * t / 32;
   };
   // widest tile whose CTA fits the kernel; a narrower one (down to half of
-  // that, at least 2 lines) only when it keeps 1.5x more warps resident,
-  // e.g. 540-point lines whose 4-line tile needs 288 threads (one CTA of
-  // 9 warps per SM) against 160 threads for 2 lines (three CTAs)
+  // that, at least 2 lines) only when it keeps 1.5x more warps resident
   int M = ap.M;
   while (M > 1 && threads_for(M) > max_threads) M /= 2;
   if (threads_for(M) > max_threads) return;
@@ -286,20 +420,14 @@ static void size_pipe(AxisPlan& ap, int kind, bool f64, int thread_cap = 0) {
   ap.pipe_threads = threads_for(M);
   ap.pipe_m = M;
   ap.pipe_log2m = ilog2(M);
-  // a third tile buffer (loads two tiles ahead) for the X kernels where it
-  // fits without costing resident warps; the strided kernels load one tile
-  // ahead (two loads in flight per CTA ran their scattered rows 3-15 %
-  // slower) and take a third buffer only to drain TMA stores (pipe_smem3)
+  // a third tile buffer (loads two tiles ahead) where it fits without costing
+  // resident warps
   size_t buf_bytes = 0;
   ap.pipe_nbuf = 2;
-  if (xk && smem_for(M, buf_bytes, 3) <= 227 * 1024 && warps_for(M, 3) >= warps_for(M, 2)) ap.pipe_nbuf = 3;
+  if (smem_for(M, buf_bytes, 3) <= 227 * 1024 && warps_for(M, 3) >= warps_for(M, 2)) ap.pipe_nbuf = 3;
   ap.pipe_smem = smem_for(M, buf_bytes, ap.pipe_nbuf);
   ap.buf_elems = (int)(buf_bytes / esize);
   ap.pipe_ok = ap.pipe_smem <= 227 * 1024;
-  // the strided kernels' TMA-store form: a third buffer drains the stores
-  ap.pipe_smem3 = 0;
-  if (!xk && smem_for(M, buf_bytes, 3) <= 227 * 1024 && warps_for(M, 3) >= warps_for(M, 2))
-    ap.pipe_smem3 = smem_for(M, buf_bytes, 3);
 }
 
 
@@ -511,6 +639,8 @@ int run_strided(p3g_plan p, SParams& s, const AxisPlan& ap, bool fwd_sign, int n
     pp.c.tw_count = ap.pipe_tw_cnt();
     pp.c.buf_elems = ap.buf_elems;
     pp.c.nbuf = ap.pipe_nbuf;
+    pp.c.groups = ap.pipe_g;
+    pp.c.gthreads = ap.pipe_threads / ap.pipe_g;
     pp.c.err = p->d_err;
     pp.chunk = esize;
     CUtensorMap map, omap;
@@ -530,13 +660,12 @@ int run_strided(p3g_plan p, SParams& s, const AxisPlan& ap, bool fwd_sign, int n
       }
     }
     // TMA tile stores: output rows stored one to one (no pruning gap, no DST
-    // shift, no four-step twiddle) in device memory, when the axis has room
-    // for a third buffer.  Binary64 user output is converted in shared memory
-    // first; binary32 user rows of an odd length (not 16-byte aligned) fail
-    // the tensor map's stride check and keep the thread stores
-    size_t smem = ap.pipe_smem;
+    // shift, no four-step twiddle) in device memory.  Binary64 user output is
+    // converted in shared memory first; binary32 user rows of an odd length
+    // (not 16-byte aligned) fail the tensor map's stride check and keep the
+    // thread stores
     const bool identity_store = q.smap_s0 >= q.Lout || q.smap_d == 0;
-    if (pp.use_tma && ap.pipe_smem3 && q.out_xs == 1 && q.post == 0 && identity_store && !q.tw4 &&
+    if (pp.use_tma && q.out_xs == 1 && q.post == 0 && identity_store && !q.tw4 &&
         q.xrow == 0 && aligned_to(q.out, 16) && device_memory(q.out)) {
       const int obrows = pick_box_rows(q.Lout, ap.n, q.M, esize);
       if (obrows > 0 && encode_strided_map(&omap, q.out, esize, q.X, q.Lout, q.O1, nv, q.out_axis, q.out_o1,
@@ -544,14 +673,13 @@ int run_strided(p3g_plan p, SParams& s, const AxisPlan& ap, bool fwd_sign, int n
         pp.tma_store = 1;
         pp.obrows = obrows;
         pp.onbox = (q.Lout + obrows - 1) / obrows;
-        pp.c.nbuf = 3;
-        smem = ap.pipe_smem3;
       }
     }
-    const int slots = (max_sms > 0 && max_sms < p->sm_count ? max_sms : p->sm_count) * ap.pipe_bps;
+    const int slots = max_sms > 0 && max_sms < p->sm_count ? max_sms : p->sm_count;
     const int grid = pp.c.ntiles < slots ? pp.c.ntiles : slots;
-    cudaError_t e = launch_strided_pipe<P>(&map, &omap, pp, p->d_sp + ap.pipe_sp(), p->d_tw, fwd_sign, ap.pipe_e,
-                                           ap.pipe_threads, smem, grid, st);
+    const auto launch = fwd_sign ? launch_strided_pipe<P, -1> : launch_strided_pipe<P, 1>;
+    cudaError_t e = launch(&map, &omap, pp, p->d_sp + ap.pipe_sp(), p->d_tw, ap.pipe_mode, ap.pipe_threads,
+                           ap.pipe_smem, grid, st);
     if (e != cudaSuccess) return fail(P3G_E_CUDA, std::string("strided pass launch: ") + cudaGetErrorString(e));
     p->launches++;
     return P3G_OK;
@@ -1403,6 +1531,15 @@ int p3g_plan_create_tuned(p3g_plan* out, int nx, int ny, int nz, int nxc, int ny
   const long long align = f64 ? 8 : 16;  // 128-byte workspace rows
   p->pitch = (p->nxhpc + align - 1) / align * align;
 
+  {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&p->sm_count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+      cudaGetLastError();
+      p->sm_count = 132;
+    }
+  }
+
   HostTw tw;
   std::vector<StagePlan> sps;
   int strided_max_m = f64 ? 64 : 128;  // 256 words per TMA box row
@@ -1423,14 +1560,14 @@ int p3g_plan_create_tuned(p3g_plan* out, int nx, int ny, int nz, int nxc, int ny
   // on the Y pass only (1024 points: 8.2 -> 7.8 ms at 1024^3; the X passes'
   // 128-thread CTAs and the Z passes' user-format stores ran slower with it)
   auto wide_ok = [&](const AxisPlan& ap, int n) {
+    if (f64) return &ap != &p->ax_x && (max_radix == 0 || max_radix >= 16);
     if ((n & (n - 1)) != 0) return false;
-    if (f64) return &ap == &p->ax_y && (max_radix == 0 || max_radix >= 16) && n >= 256;
     return max_radix == 0 || max_radix >= 32;
   };
   auto add_axis = [&](AxisPlan& ap, int n, int lines) -> bool {
     if (!build_stages(n, std::min(axis_pow2(n), f64 ? 8 : 16), tw, ap.sp)) return false;
     ap.tw_lo = tw.mark;
-    ap.tw_cnt = (int)tw.v.size() - tw.mark;
+    ap.tw_cnt = tw.count;
     if (!size_tile(ap, n, lines, f64, &ap == &p->ax_x ? x_max_m : strided_max_m)) return false;
     ap.sp_index = (int)sps.size();
     sps.push_back(ap.sp);
@@ -1438,10 +1575,10 @@ int p3g_plan_create_tuned(p3g_plan* out, int nx, int ny, int nz, int nxc, int ny
     // against 16 x 16 x 4 on F32), kept when it has a wide stage
     if (wide_ok(ap, n)) {
       StagePlan w;
-      if (build_stages(n, f64 ? 16 : 32, tw, w) && w.cnt[f64 ? 1 : 0] > 0) {
+      if (build_stages(n, f64 ? 16 : 32, tw, w) && family_count(w.fam, f64 ? 1 : 0) > 0) {
         ap.spw = w;
         ap.tw_lo_w = tw.mark;
-        ap.tw_cnt_w = (int)tw.v.size() - tw.mark;
+        ap.tw_cnt_w = tw.count;
         ap.spw_index = (int)sps.size();
         sps.push_back(w);
       }
@@ -1523,14 +1660,6 @@ int p3g_plan_create_tuned(p3g_plan* out, int nx, int ny, int nz, int nxc, int ny
     if (!size_tile(p->ax_z[3], nz, p->nxhpc, f64, strided_max_m)) p->z_ok[3] = false;
   }
   if (!p->z_ok[0] && !p->z_ok[1] && !p->z_ok[3]) return bad("z length " + std::to_string(nz) + " is too long");
-  // the wide kernels take fewer points per tile line set (fewer threads per
-  // CTA); an axis whose wide tile does not fit runs the narrow kernels
-  auto narrow_if_unfit = [&](AxisPlan& ap, int kind) {
-    if (!ap.pipe_ok && ap.spw_index >= 0) {
-      ap.spw_index = -1;
-      size_pipe(ap, kind, f64);
-    }
-  };
   auto size_x = [&] {  // r2c and c2r share the tile; c2r needs the larger buffer
     size_pipe(p->ax_x, 1, f64);
     AxisPlan c2r = p->ax_x;
@@ -1558,56 +1687,38 @@ int p3g_plan_create_tuned(p3g_plan* out, int nx, int ny, int nz, int nxc, int ny
     size_pipe(p->ax_xc, 2, f64, nx >= 512 && (nx & (nx - 1)) == 0 ? 128 : 0);
     if (!p->ax_xc.pipe_ok) size_pipe(p->ax_xc, 2, f64);
   }
-  size_pipe(p->ax_y, 0, f64);
-  narrow_if_unfit(p->ax_y, 0);
+  const int yx = p->nxhpc;
+  const bool far_y = (long long)nz * p->pitch * p->esize() >= 3 << 20;  // the Y/Z workspace's row stride along y
+  auto size_s = [&](AxisPlan& ap, int X, long long O1, bool tstore, bool far_rows) {
+    size_strided(ap, f64, X, (int)std::min<long long>(O1, 1 << 30), strided_max_m, p->sm_count, tstore,
+                 far_rows);
+    if (!ap.pipe_ok && ap.spw_index >= 0) {
+      ap.spw_index = -1;
+      size_strided(ap, f64, X, (int)std::min<long long>(O1, 1 << 30), strided_max_m, p->sm_count, tstore,
+                 far_rows);
+    }
+  };
+  size_s(p->ax_y, yx, nz, false, far_y);
   for (int i = 0; i < 2; ++i) {
-    if (p->four_y) {
-      size_pipe(p->ly[i], 0, f64);
-      narrow_if_unfit(p->ly[i], 0);
-    }
-    if (p->four_z) {
-      size_pipe(p->lz[i], 0, f64);
-      narrow_if_unfit(p->lz[i], 0);
-    }
+    if (p->four_y) size_s(p->ly[i], yx, (long long)nz * p->ly[1 - i].n, false, far_y);
+    if (p->four_z) size_s(p->lz[i], yx, (long long)nyc * p->lz[1 - i].n, !f64, false);
   }
   for (int i = 0; i < 4; ++i)
-    if (p->z_ok[i]) {
-      size_pipe(p->ax_z[i], 0, f64);
-      narrow_if_unfit(p->ax_z[i], 0);
-    }
+    if (p->z_ok[i]) size_s(p->ax_z[i], yx, nyc, !f64, false);
   {
-    auto bps = [&](AxisPlan& ap, int kind) {
+    auto bps = [&](AxisPlan& ap) {
       if (!ap.pipe_ok) return;
-      auto occ = [&](size_t sm) {
-        return f64 ? pipe_blocks_per_sm<PathF64>(kind, ap.pipe_e, ap.pipe_threads, sm)
-                   : pipe_blocks_per_sm<PathF32>(kind, ap.pipe_e, ap.pipe_threads, sm);
-      };
-      ap.pipe_bps = occ(ap.pipe_smem);
-      if (ap.pipe_smem3 && occ(ap.pipe_smem3) < ap.pipe_bps) ap.pipe_smem3 = 0;
+      ap.pipe_bps = f64 ? pipe_blocks_per_sm<PathF64>(2, ap.pipe_e, ap.pipe_threads, ap.pipe_smem)
+                        : pipe_blocks_per_sm<PathF32>(2, ap.pipe_e, ap.pipe_threads, ap.pipe_smem);
     };
-    bps(p->ax_x, 2);
-    bps(p->ax_xc, 2);
-    bps(p->ax_y, 0);
-    for (int i = 0; i < 2; ++i) {
-      if (p->four_y) bps(p->ly[i], 0);
-      if (p->four_z) bps(p->lz[i], 0);
-    }
-    for (int i = 0; i < 4; ++i) bps(p->ax_z[i], 0);
+    bps(p->ax_x);
+    bps(p->ax_xc);
   }
   {
     const char* e = std::getenv("P3G_NO_PIPE");
     p->use_pipe = !(e && *e && *e != '0');
     e = std::getenv("P3G_NO_TMA");
     p->use_tma = !(e && *e && *e != '0');
-  }
-  if (cudaDeviceGetAttribute(&p->sm_count, cudaDevAttrMultiProcessorCount, 0) != cudaSuccess) {
-    cudaGetLastError();
-    p->sm_count = 132;
-  }
-  {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&p->sm_count, cudaDevAttrMultiProcessorCount, dev);
   }
 
   {

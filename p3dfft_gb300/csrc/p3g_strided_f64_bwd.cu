@@ -1,0 +1,6 @@
+// Strided Y/Z pass kernels, F64 path, backward sign.
+#include "p3g_strided_impl.cuh"
+
+namespace p3g {
+P3G_STRIDED_INSTANTIATE(PathF64, 1)
+}  // namespace p3g
