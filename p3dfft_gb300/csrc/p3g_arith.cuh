@@ -171,11 +171,14 @@ P3G_HD uint32_t shl3_funnel(uint32_t lo, uint32_t hi) {
 #endif
 }
 
-P3G_HD df d2df(double x) {
+P3G_HD bool d2df_is_edge(uint32_t hw) {  // e < 949 or e > 1150
+  return (hw & 0x7FFFFFFFu) - (949u << 20) >= (202u << 20);
+}
+// The short route alone (x must not be an edge value).
+P3G_HD df d2df_mid(double x) {
   const uint64_t b = d2u(x);
   const uint32_t hw = (uint32_t)(b >> 32), lw = (uint32_t)b;
   const uint32_t a = hw & 0x7FFFFFFFu;
-  if (a - (949u << 20) >= (202u << 20)) return d2df_edge(x);  // e < 949 or e > 1150
   const uint32_t hb = shl3_funnel(lw, a - (896u << 20)) | (hw & 0x80000000u);
   // 2^(e-1075) = 2^(e_hi - 179) with the sign of x; e_hi >= 53, so the
   // subtraction stays inside the exponent field
@@ -184,6 +187,10 @@ P3G_HD df d2df(double x) {
   r.hi = u2f(hb);
   r.lo = ffma(u32_to_f32_rn(lw & 0x1FFFFFFFu), u2f(scale), 0.0f);
   return r;
+}
+P3G_HD df d2df(double x) {
+  if (d2df_is_edge((uint32_t)(d2u(x) >> 32))) return d2df_edge(x);
+  return d2df_mid(x);
 }
 
 // Nearest integer of a binary32 value below 2^30.
@@ -523,6 +530,16 @@ struct PathF64 {
   P3G_D static C from_uc(double2 v, int k) { return make_cdf(d2df_scaled(v.x, k), d2df_scaled(v.y, k)); }
   P3G_D static double2 to_uc(C c, int k) { return make_double2(to_ur(re(c), k), to_ur(im(c), k)); }
   P3G_D static df from_ur(double v, int k) { return d2df_scaled(v, k); }
+  // z = x1 + i x2 for values of the short route; `edge` collects whether the
+  // caller has to convert again with make_slow
+  P3G_D static C make_mid(double x1, double x2, bool& edge) {
+    edge = edge || d2df_is_edge((uint32_t)__double2hiint(x1)) || d2df_is_edge((uint32_t)__double2hiint(x2));
+    return make_cdf(d2df_mid(x1), d2df_mid(x2));
+  }
+  static __device__ __noinline__ float4 make_slow(double x1, double x2, int k) {
+    const df a = d2df_scaled(x1, k), b = d2df_scaled(x2, k);
+    return make_float4(a.hi, b.hi, a.lo, b.lo);
+  }
   P3G_D static double to_ur(df v, int k) { return scale_pow2(df2d(v.hi, v.lo), k); }
   // largest |high word| seen (the binary64 exponent window's input)
   P3G_D static void track(uint32_t& amax, double v) {
@@ -554,6 +571,8 @@ struct PathF32 {
   P3G_D static C from_uc(float2 v, int) { return from_w(v); }
   P3G_D static float2 to_uc(C c, int) { return to_w(c); }
   P3G_D static float from_ur(float v, int) { return v; }
+  P3G_D static C make_mid(float x1, float x2, bool&) { return make(x1, x2); }
+  P3G_D static float2 make_slow(float x1, float x2, int) { return make_float2(x1, x2); }
   P3G_D static float to_ur(float v, int) { return v; }
   P3G_D static void track(uint32_t&, float) {}
   P3G_D static void track(uint32_t&, float2) {}

@@ -106,12 +106,12 @@ P3G_D void sts(uint32_t a, float2 v) {
   asm volatile("st.shared.v2.f32 [%0], {%1, %2};\n" ::"r"(a), "f"(v.x), "f"(v.y) : "memory");
 }
 
-// Line-major tiles may be padded by one element every 2^ps elements
-// (ps = log2 of the plan's first radix, 0 = no padding) so that the first
-// stage's stride-R writes hit distinct banks.  For the plans that use it
-// (all radices powers of two, every stage's N/R and every later stage's
-// sub-length multiples of 2^ps) each stage's R inputs and R outputs stay
-// equally spaced in the padded layout.
+// Line-major tiles may be padded by one element every 2^ps elements (0 = no
+// padding) so that the first stage's stride-R writes hit different banks.
+// 2^ps divides the plan's first radix and every stage's N/R (and with the
+// first radix every later stage's sub-length), so each stage's R inputs and
+// the R outputs of every stage but the first stay equally spaced in the padded
+// layout; output q of the first stage lies q + (q >> ps) further on.
 P3G_D int pad_index(int j, int ps) { return ps ? j + (j >> ps) : j; }
 
 // Hardware barrier with a compile-time id.  Each radix uses its own id: with a
@@ -169,6 +169,7 @@ struct Tile {
   int ebias = 0;
   uint32_t* amax = nullptr;
   TH th{};
+  unsigned* amax_out = nullptr;  // grouped X tiles: where the first stage leaves each warp's largest
   P3G_D int addr(int line, int j) const { return line * LS + (LS == 1 ? j * JS : pad_index(j, ps)); }
   P3G_D uint32_t saddr(int line, int j) const {
     return (uint32_t)__cvta_generic_to_shared(sm) + (uint32_t)((line * LS + j * JS) * (int)sizeof(typename P::W));
@@ -280,35 +281,68 @@ __device__ __forceinline__ void stage_reg(const Tile<P, TH>& t, int N, int ns, c
         constexpr uint32_t kU = (uint32_t)sizeof(UR);
         const uint32_t ra = sbase + (uint32_t)((2 * line * N + j) * (int)kU);
         const uint32_t rstep = (uint32_t)per_line * kU, lstep = (uint32_t)N * kU;
+        // one branch per butterfly for the values (or bias) that need the long
+        // conversion, out of line: with one per value the inlined long route
+        // made the stage's code several times larger
+        bool edge = false;
+        uint32_t am = 0;
 #pragma unroll
         for (int q = 0; q < R; ++q) {
           const UR x1 = lds1(ra + q * rstep, (UR*)nullptr), x2 = lds1(ra + lstep + q * rstep, (UR*)nullptr);
-          if (t.amax) {
-            P::track(*t.amax, x1);
-            P::track(*t.amax, x2);
-          }
-          v[i][q] = P::make(P::from_ur(x1, t.ebias), P::from_ur(x2, t.ebias));
+          P::track(am, x1);
+          P::track(am, x2);
+          v[i][q] = P::make_mid(x1, x2, edge);
+        }
+        if (t.amax) *t.amax = max(*t.amax, am);
+        if (P::kF64 && (edge || t.ebias != 0)) {
+#pragma unroll
+          for (int q = 0; q < R; ++q)
+            v[i][q] = P::from_w(P::make_slow(lds1(ra + q * rstep, (UR*)nullptr),
+                                             lds1(ra + lstep + q * rstep, (UR*)nullptr), t.ebias));
         }
       } else if constexpr (RAW == kRawC2R) {
         const int nh = N / 2 + 1;
         const int rs = sizeof(W) == 8 ? (nh + 1) & ~1 : nh;  // raw line stride (xc2r_raw_stride)
         const uint32_t ra = sbase + (uint32_t)(line * 2 * rs * (int)kW);
+        if constexpr (R % 2 == 0) {
+          // points j + q N/R lie below N/2 for q < R/2 and mirror above it, at
+          // addresses equally spaced in q; only j = 0 meets p = 0 (q = 0) and
+          // p = N/2 (q = R/2)
+          const uint32_t step = (uint32_t)(per_line * (int)kW), ro = (uint32_t)(rs * (int)kW);
+          const uint32_t up = ra + (uint32_t)(j * (int)kW), down = ra + (uint32_t)((N - j) * (int)kW);
 #pragma unroll
-        for (int q = 0; q < R; ++q) {
-          const int pt = j + q * per_line;
-          const bool mir = 2 * pt > N;
-          const int pm = mir ? N - pt : pt;
-          C x1 = P::from_w(lds(ra + (uint32_t)(pm * (int)kW), (W*)nullptr));
-          C x2 = P::from_w(lds(ra + (uint32_t)((rs + pm) * (int)kW), (W*)nullptr));
-          if (pm == 0 || 2 * pm == N) {
-            x1 = P::make(P::re(x1), P::re(P::zero()));
-            x2 = P::make(P::re(x2), P::re(P::zero()));
+          for (int q = 0; q < R; ++q) {
+            const uint32_t pa = q < R / 2 ? up + q * step : down - q * step;
+            C x1 = P::from_w(lds(pa, (W*)nullptr));
+            C x2 = P::from_w(lds(pa + ro, (W*)nullptr));
+            if ((q == 0 || q == R / 2) && j == 0) {
+              x1 = P::make(P::re(x1), P::re(P::zero()));
+              x2 = P::make(P::re(x2), P::re(P::zero()));
+            }
+            if (q >= R / 2) {
+              x1 = cconj(x1);
+              x2 = cconj(x2);
+            }
+            v[i][q] = x1 + rot<1>(x2);
           }
-          if (mir) {
-            x1 = cconj(x1);
-            x2 = cconj(x2);
+        } else {
+#pragma unroll
+          for (int q = 0; q < R; ++q) {
+            const int pt = j + q * per_line;
+            const bool mir = 2 * pt > N;
+            const int pm = mir ? N - pt : pt;
+            C x1 = P::from_w(lds(ra + (uint32_t)(pm * (int)kW), (W*)nullptr));
+            C x2 = P::from_w(lds(ra + (uint32_t)((rs + pm) * (int)kW), (W*)nullptr));
+            if (pm == 0 || 2 * pm == N) {
+              x1 = P::make(P::re(x1), P::re(P::zero()));
+              x2 = P::make(P::re(x2), P::re(P::zero()));
+            }
+            if (mir) {
+              x1 = cconj(x1);
+              x2 = cconj(x2);
+            }
+            v[i][q] = x1 + rot<1>(x2);
           }
-          v[i][q] = x1 + rot<1>(x2);
         }
       } else {
 #pragma unroll
@@ -325,12 +359,21 @@ __device__ __forceinline__ void stage_reg(const Tile<P, TH>& t, int N, int ns, c
       oaddr[i] = sbase + (pm ? (uint32_t)(line + (jo << t.log2m)) * kW : (uint32_t)(t.addr(line, jo) * (int)kW));
     }
   }
+  if constexpr (RAW == kRawR2C && TH::kHold && P::kF64) {
+    const uint32_t w = __reduce_max_sync(0xFFFFFFFFu, *t.amax);
+    if ((t.th.tid() & 31) == 0) atomicMax(t.amax_out, w);
+  }
   t.th.template stage_sync<(R == 16 ? 1 : (R == 32 ? 6 : R))>();
 #pragma unroll
   for (int i = 0; i < MAXB; ++i) {
     if (FULL || t.th.tid() + i * T < nb) {
+      if (LAY != kPointMajor && ns == 1 && ps > 0 && (1 << ps) < R) {
 #pragma unroll
-      for (int q = 0; q < R; ++q) sts(oaddr[i] + q * ostride, P::to_w(v[i][q]));
+        for (int q = 0; q < R; ++q) sts(oaddr[i] + (uint32_t)((q + (q >> ps)) * t.JS) * kW, P::to_w(v[i][q]));
+      } else {
+#pragma unroll
+        for (int q = 0; q < R; ++q) sts(oaddr[i] + q * ostride, P::to_w(v[i][q]));
+      }
     }
   }
   t.th.template stage_sync<(R == 16 ? 1 : (R == 32 ? 6 : R))>();
@@ -407,20 +450,14 @@ __device__ __forceinline__ void run_family(const Tile<P, TH>& t, const float4* _
 // the live ranges of every codelet at once and spill.  FULL: a plan of
 // power-of-two radices whose stages all fill every thread; only those
 // families are compiled, without guards.
-// tw points at the twiddle table entry tw_base (the full table with
-// tw_base = 0, or a pass's slice copied to shared memory).  E = elements each
-// thread holds per stage.  LAY: the
-// tile layout when the caller knows it (kPointMajor, kLineMajor).  RAW: the
+// The first stage's twiddles start at tw[off].  E = elements each thread holds
+// per stage.  LAY: the tile layout when the caller knows it (kPointMajor, kLineMajor).  RAW: the
 // tile still holds the raw line pairs of an X r2c or c2r tile (kRawR2C,
 // kRawC2R; plans without generic stages only), read by the first stage.
-template <class P, int DIR, int E = kElemsPerThread, int LAY = kAnyLayout, int RAW = kRawNone,
-          int MAXR = P::kF64 ? 8 : 16, bool FULL = false, class TH = CtaThreads>
-__device__ __forceinline__ void cta_fft(const Tile<P, TH>& t, const StagePlan* __restrict__ sp,
-                                        const float4* __restrict__ tw, int tw_base = 0) {
-  const int N = __ldg(&sp->n);
-  const unsigned long long fam = __ldg(&sp->fam);
+template <class P, int DIR, int E, int LAY, int RAW, int MAXR, bool FULL, class TH>
+__device__ __forceinline__ void run_families(const Tile<P, TH>& t, const float4* __restrict__ tw, int N,
+                                             unsigned long long fam, int off) {
   int ns = 1;
-  int off = __ldg(&sp->tw_off[0]) - tw_base;
   if constexpr (MAXR >= 32) run_family<P, DIR, 32, E, LAY, FULL, RAW>(t, tw, N, family_count(fam, 0), ns, off);
   if constexpr (MAXR >= 16) run_family<P, DIR, 16, E, LAY, FULL, RAW>(t, tw, N, family_count(fam, 1), ns, off);
   run_family<P, DIR, 8, E, LAY, FULL, RAW>(t, tw, N, family_count(fam, 2), ns, off);
@@ -429,17 +466,25 @@ __device__ __forceinline__ void cta_fft(const Tile<P, TH>& t, const StagePlan* _
   if constexpr (!FULL) {
     run_family<P, DIR, 3, E, LAY, false, RAW>(t, tw, N, family_count(fam, 5), ns, off);
     run_family<P, DIR, 5, E, LAY, false, RAW>(t, tw, N, family_count(fam, 6), ns, off);
-    if constexpr (std::is_same<TH, CtaThreads>::value) {
-      if (__ldg(&sp->has_generic)) {
-        int sg = 0;
-        for (int i = 0; i < kNumFamilies; ++i) sg += family_count(fam, i);
-        const int nst = __ldg(&sp->nstages);
+  }
+}
+
+// The CTA-wide form reads the plan from global memory and runs generic primes.
+template <class P, int DIR, int E = kElemsPerThread, int LAY = kAnyLayout, int RAW = kRawNone,
+          int MAXR = P::kF64 ? 8 : 16>
+__device__ __forceinline__ void cta_fft(const Tile<P>& t, const StagePlan* __restrict__ sp,
+                                        const float4* __restrict__ tw) {
+  const int N = __ldg(&sp->n);
+  const unsigned long long fam = __ldg(&sp->fam);
+  run_families<P, DIR, E, LAY, RAW, MAXR, false>(t, tw, N, fam, __ldg(&sp->tw_off[0]));
+  if (__ldg(&sp->has_generic)) {
+    int sg = 0;
+    for (int i = 0; i < kNumFamilies; ++i) sg += family_count(fam, i);
+    const int nst = __ldg(&sp->nstages);
 #pragma unroll 1
-        for (int s = sg; s < nst; ++s)
-          stage_generic<P, DIR>(t, N, __ldg(&sp->radix[s]), __ldg(&sp->ns[s]), tw + (__ldg(&sp->tw_off[s]) - tw_base),
-                                tw + (__ldg(&sp->root_off[s]) - tw_base));
-      }
-    }
+    for (int s = sg; s < nst; ++s)
+      stage_generic<P, DIR>(t, N, __ldg(&sp->radix[s]), __ldg(&sp->ns[s]), tw + __ldg(&sp->tw_off[s]),
+                            tw + __ldg(&sp->root_off[s]));
   }
 }
 

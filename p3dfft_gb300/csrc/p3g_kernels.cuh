@@ -190,23 +190,18 @@ cudaError_t launch_x_long(int kind, const XLongParams& q, int sm_count, cudaStre
 // pipelined kernels (p3g_pipe.cuh)
 struct SPipeParams;
 struct XPipeParams;
-// Instantiations of the strided pipelined kernel: kStridedFull runs
-// power-of-two lengths whose stages fill every thread, kStridedFullWide the
-// same with half the threads and twice the registers, kStridedGeneral any
-// plan, kStridedSmall any narrow plan with half the points per thread.
-enum StridedMode { kStridedGeneral = 0, kStridedFull = 1, kStridedFullWide = 2, kStridedSmall = 3 };
-constexpr int strided_max_threads(int mode) { return mode == kStridedFullWide ? 256 : 512; }
+// Instantiations of the pipelined kernels: kTileFull runs power-of-two lengths
+// whose stages fill every thread, kTileFullWide the same with fewer threads
+// and more registers (binary32 only), kTileGeneral any plan, kTileSmall any
+// narrow plan with half the points per thread.
+enum TileMode { kTileGeneral = 0, kTileFull = 1, kTileFullWide = 2, kTileSmall = 3 };
+constexpr int tile_max_threads(int mode, bool x_pass = false) { return mode == kTileFullWide ? (x_pass ? 384 : 256) : 512; }
 template <class P, int DIR>
 cudaError_t launch_strided_pipe(const CUtensorMap* map, const CUtensorMap* omap, const SPipeParams& p,
-                                const StagePlan* sp, const float4* tw, StridedMode mode, int threads, size_t smem, int grid,
+                                const float4* tw, TileMode mode, int threads, size_t smem, int grid,
                                 cudaStream_t st);
-template <class P>
-cudaError_t launch_xr2c_pipe(const XPipeParams& p, const StagePlan* sp, const float4* tw, int E, int threads,
-                             size_t smem, int grid, cudaStream_t st);
-template <class P>
-int pipe_blocks_per_sm(int kind, int E, int threads, size_t smem);
-template <class P>
-cudaError_t launch_xc2r_pipe(const XPipeParams& p, const StagePlan* sp, const float4* tw, int E, int threads,
-                             size_t smem, int grid, cudaStream_t st);
+template <class P, bool R2C>
+cudaError_t launch_x_pipe(const XPipeParams& p, const float4* tw, TileMode mode, int threads,
+                          size_t smem, int grid, cudaStream_t st);
 
 }  // namespace p3g

@@ -414,72 +414,6 @@ cudaError_t launch_cheby(const ChebyParams& p, int nfields, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-// X pass launchers: E (elements per thread) selects the instantiation.
-template <class P, int E>
-cudaError_t launch_xr2c_pipe_e(const XPipeParams& p, const StagePlan* sp, const float4* tw, int threads, size_t smem,
-                               int grid, cudaStream_t st) {
-  cudaError_t ea = opt_in_smem((const void*)k_xr2c_pipe<P, E>, 227 * 1024);
-  if (ea != cudaSuccess) return ea;
-  k_xr2c_pipe<P, E><<<grid, threads, smem, st>>>(p, sp, tw);
-  return cudaGetLastError();
-}
-template <class P>
-cudaError_t launch_xr2c_pipe(const XPipeParams& p, const StagePlan* sp, const float4* tw, int E, int threads,
-                             size_t smem, int grid, cudaStream_t st) {
-  if constexpr (P::kF64) {
-    if (E == 8) return launch_xr2c_pipe_e<P, 8>(p, sp, tw, threads, smem, grid, st);
-    if (E == 16) return launch_xr2c_pipe_e<P, 16>(p, sp, tw, threads, smem, grid, st);
-  } else {
-    if (E == 16) return launch_xr2c_pipe_e<P, 16>(p, sp, tw, threads, smem, grid, st);
-    if (E == 32) return launch_xr2c_pipe_e<P, 32>(p, sp, tw, threads, smem, grid, st);
-  }
-  return cudaErrorInvalidValue;
-}
-template <class P, int E>
-cudaError_t launch_xc2r_pipe_e(const XPipeParams& p, const StagePlan* sp, const float4* tw, int threads, size_t smem,
-                               int grid, cudaStream_t st) {
-  cudaError_t ea = opt_in_smem((const void*)k_xc2r_pipe<P, E>, 227 * 1024);
-  if (ea != cudaSuccess) return ea;
-  k_xc2r_pipe<P, E><<<grid, threads, smem, st>>>(p, sp, tw);
-  return cudaGetLastError();
-}
-template <class P>
-cudaError_t launch_xc2r_pipe(const XPipeParams& p, const StagePlan* sp, const float4* tw, int E, int threads,
-                             size_t smem, int grid, cudaStream_t st) {
-  if constexpr (P::kF64) {
-    if (E == 8) return launch_xc2r_pipe_e<P, 8>(p, sp, tw, threads, smem, grid, st);
-    if (E == 16) return launch_xc2r_pipe_e<P, 16>(p, sp, tw, threads, smem, grid, st);
-  } else {
-    if (E == 16) return launch_xc2r_pipe_e<P, 16>(p, sp, tw, threads, smem, grid, st);
-    if (E == 32) return launch_xc2r_pipe_e<P, 32>(p, sp, tw, threads, smem, grid, st);
-  }
-  return cudaErrorInvalidValue;
-}
-
-// Resident CTAs per SM of an X pass kernel (kind 1 r2c, 2 c2r)
-// with E elements per thread for the given block size and dynamic shared
-// memory; 1 if the query fails.
-template <class P, int E>
-int pipe_blocks_per_sm_e(int kind, int threads, size_t smem) {
-  const void* f = kind == 1 ? (const void*)k_xr2c_pipe<P, E> : (const void*)k_xc2r_pipe<P, E>;
-  int n = 0;
-  if (opt_in_smem(f, 227 * 1024) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, f, threads, smem) != cudaSuccess || n < 1) {
-    cudaGetLastError();
-    return 1;
-  }
-  return n;
-}
-template <class P>
-int pipe_blocks_per_sm(int kind, int E, int threads, size_t smem) {
-  if constexpr (P::kF64) {
-    return E == 16 ? pipe_blocks_per_sm_e<P, 16>(kind, threads, smem) : pipe_blocks_per_sm_e<P, 8>(kind, threads, smem);
-  } else {
-    return E == 32 ? pipe_blocks_per_sm_e<P, 32>(kind, threads, smem)
-                   : pipe_blocks_per_sm_e<P, 16>(kind, threads, smem);
-  }
-}
-
 #define P3G_INSTANTIATE(P)                                                                                          \
   template cudaError_t launch_x_r2c<P>(const XParams&, const StagePlan*, const float4*, int, size_t, int,          \
                                        cudaStream_t);                                                              \
@@ -488,11 +422,6 @@ int pipe_blocks_per_sm(int kind, int E, int threads, size_t smem) {
   template cudaError_t launch_strided<P>(const SParams&, const StagePlan*, const float4*, bool, int, size_t, int,  \
                                          cudaStream_t);                                                            \
   template cudaError_t launch_cheby<P>(const ChebyParams&, int, cudaStream_t);                                     \
-  template cudaError_t launch_x_long<P>(int, const XLongParams&, int, cudaStream_t);                               \
-  template int pipe_blocks_per_sm<P>(int, int, int, size_t);                                                            \
-  template cudaError_t launch_xr2c_pipe<P>(const XPipeParams&, const StagePlan*, const float4*, int, int, size_t,  \
-                                           int, cudaStream_t);                                                     \
-  template cudaError_t launch_xc2r_pipe<P>(const XPipeParams&, const StagePlan*, const float4*, int, int, size_t,  \
-                                           int, cudaStream_t);
+  template cudaError_t launch_x_long<P>(int, const XLongParams&, int, cudaStream_t);
 
 }  // namespace p3g

@@ -25,9 +25,10 @@ struct PipeCommon {
   int ntiles;               // tiles over all fields
   int tiles_per_field;
   int tw_base, tw_count;    // this pass's slice of the twiddle table (float4)
+  unsigned long long fam;   // the plan's stages (StagePlan::fam), read from the kernel's parameters
   int buf_elems;            // elements (W) per buffer
-  int nbuf;                 // tile buffers (X kernels: 2 or 3, loads run nbuf - 1 tiles ahead)
-  int groups, gthreads;     // strided kernels: thread groups per CTA and threads of each
+  int nbuf;                 // tile buffers
+  int groups, gthreads;     // thread groups per CTA and threads of each
   int* err;                 // device error flag
 };
 
@@ -49,9 +50,9 @@ struct XPipeParams {
   XParams x;
   PipeCommon c;
   int chunk;                // r2c: cp.async bytes per copy (4, 8 or 16)
-  // 1: thread 0 loads tiles with 1-D bulk copies on an mbarrier (r2c: the
-  // tile's 2M contiguous real lines in one copy, full tiles only; c2r: one
-  // copy per line of every mode), else every thread issues cp.async
+  // 1: a group's first thread loads its tile with 1-D bulk copies on the
+  // buffer's mbarrier (r2c: the tile's contiguous real lines in one copy;
+  // c2r: one copy per line), else every thread issues cp.async
   int bulk;
 };
 
@@ -66,56 +67,30 @@ P3G_D unsigned char* align1k(unsigned char* p) {
 // stages of the other radices they fit their registers without spilling,
 // which the others do not quite.
 template <class P>
-struct StridedElems {
+struct TileElems {
   static constexpr int value = P::kF64 ? 16 : 32;
 };
 constexpr int kMaxGroups = 8;        // named barriers 1..8
 constexpr int kMaxTileBuffers = 12;  // ring of tile buffers
 
-// kWide marks the X kernels compiled with the large radices.
-template <class P, int E>
-struct PipeLimits {
-  static constexpr bool kWide = P::kF64 ? E == 16 : E == 32;
-};
-
-// X passes: 256-thread CTAs, three per SM (85 registers; for the F32
-// radix-32 stages 64-thread CTAs, six per SM, with up to 170 registers: 1024
-// points X r2c 2.57 -> 2.49 ms at 1024^3 against three 128-thread CTAs; the
-// F64 radix-16 kernel keeps 128-thread CTAs), with the twiddles
-// read from the global table through L1 instead of a shared-memory copy,
-// which leaves room for three double-buffered tiles per SM.  The X passes
-// gain from the extra resident CTAs; the strided passes, whose tiles must
-// stay wide for their long-stride DRAM rows, keep PipeLimits.
-template <class P, int E>
-struct XPipeLimits {
-  static constexpr int kMaxThreads = PipeLimits<P, E>::kWide ? (P::kF64 ? 128 : 64) : 256;
-  static constexpr int kMinBlocks = PipeLimits<P, E>::kWide && !P::kF64 ? 6 : 3;
-};
-
-// Largest radix compiled into a pipelined kernel (cta_fft's MAXR).
-template <class P, int E>
-struct PipeMaxR {
-  static constexpr int value = P::kF64 ? (E == 16 ? 16 : 8) : (E == 32 ? 32 : 16);
-};
-
-
-
 // ------------------------------------------------------------ strided Y/Z
 template <class P>
-struct StridedSmem {
+struct RingSmem {
   typename P::W* buf0;
   float4* tw;
   uint64_t* mbar;  // one per buffer: its load has landed
-  int* issued;     // loads issued into each buffer so far, then the CTA's failure flag
+  int* issued;     // loads issued into each buffer so far
+  int* cta;        // [0] failure flag; X passes: [1] exponent bias, [2] largest |high word| seen
 };
 template <class P>
-P3G_D StridedSmem<P> strided_smem(const PipeCommon& pc) {
+P3G_D RingSmem<P> ring_smem(const PipeCommon& pc) {
   extern __shared__ unsigned char p3g_pipe_smem[];
-  StridedSmem<P> r;
+  RingSmem<P> r;
   r.buf0 = reinterpret_cast<typename P::W*>(align1k(p3g_pipe_smem));
   r.tw = reinterpret_cast<float4*>(r.buf0 + pc.nbuf * pc.buf_elems);
   r.mbar = reinterpret_cast<uint64_t*>(r.tw + pc.tw_count);
   r.issued = reinterpret_cast<int*>(r.mbar + pc.nbuf);
+  r.cta = r.issued + pc.nbuf;
   return r;
 }
 
@@ -266,7 +241,7 @@ P3G_D bool ring_wait(uint64_t* bar, const int* issued, int use, int* err) {
 template <class P>
 P3G_D void strided_issue(const SPipeParams& q, const CUtensorMap* tin, int tile, int b, const GroupThreads& th) {
   using W = typename P::W;
-  const StridedSmem<P> sm = strided_smem<P>(q.c);
+  const RingSmem<P> sm = ring_smem<P>(q.c);
   W* dst = sm.buf0 + b * q.c.buf_elems;
   int xt, o1, o2;
   strided_decode(q, tile, xt, o1, o2);
@@ -393,13 +368,6 @@ P3G_D void strided_store(const SParams& s, const typename P::W* sm, int xt, int 
   }
 }
 
-// Waits for the copies of tile slot it (buffer it % nbuf): cp.async groups
-// (nbuf - 1 may stay in flight) or the TMA mbarrier; false after a time-out.
-P3G_D void cp_async_wait_ahead(int nbuf) {
-  if (nbuf >= 3) cp_async_wait<2>();
-  else cp_async_wait<1>();
-}
-
 // The CTA's threads form `groups` groups that each transform whole tiles with
 // barriers of their own; the tiles go round the groups, and round a ring of
 // nbuf > groups buffers.  While the groups work, the loads of the next tiles
@@ -410,21 +378,20 @@ P3G_D void cp_async_wait_ahead(int nbuf) {
 // shared-memory exchanges and barriers; two or more groups drift apart and
 // fill each other's gaps.
 template <class P, int DIR, int MODE>
-__global__ void __launch_bounds__(strided_max_threads(MODE), 1)
+__global__ void __launch_bounds__(tile_max_threads(MODE), 1)
     k_strided_pipe(const __grid_constant__ CUtensorMap tin, const __grid_constant__ CUtensorMap tout,
-                   const __grid_constant__ SPipeParams pp, const StagePlan* __restrict__ sp,
-                   const float4* __restrict__ tw_g) {
+                   const __grid_constant__ SPipeParams pp, const float4* __restrict__ tw_g) {
   const int nb = pp.c.nbuf, G = pp.c.groups;
   const int step = (int)gridDim.x;
   {
-    const StridedSmem<P> sm = strided_smem<P>(pp.c);
+    const RingSmem<P> sm = ring_smem<P>(pp.c);
     for (int i = threadIdx.x; i < pp.c.tw_count; i += blockDim.x) sm.tw[i] = __ldg(tw_g + pp.c.tw_base + i);
     if (threadIdx.x == 0) {
       for (int i = 0; i < nb; ++i) {
         mbar_init(&sm.mbar[i], pp.use_tma ? 1 : pp.c.gthreads);
         sm.issued[i] = 0;
       }
-      sm.issued[nb] = 0;
+      sm.cta[0] = 0;
       mbar_fence_init();
     }
   }
@@ -449,27 +416,27 @@ __global__ void __launch_bounds__(strided_max_threads(MODE), 1)
       bulk_wait_read<1>();
       strided_issue<P>(pp, &tin, tile + step, b + 1 == nb ? 0 : b + 1, th);
     }
-    const bool ok = ring_wait(&strided_smem<P>(pp.c).mbar[b], &strided_smem<P>(pp.c).issued[b], use, pp.c.err);
+    const bool ok = ring_wait(&ring_smem<P>(pp.c).mbar[b], &ring_smem<P>(pp.c).issued[b], use, pp.c.err);
     if (th.sync_or(!ok)) {
-      if (th.t == 0) strided_smem<P>(pp.c).issued[nb] = 1;
+      if (th.t == 0) ring_smem<P>(pp.c).cta[0] = 1;
       break;
     }
     if (rtile >= 0 && th.t == 0) {
       bulk_wait_read<0>();
       strided_issue<P>(pp, &tin, rtile, rbuf, th);
     }
-    strided_fix<P>(pp.s, pp.use_tma != 0, strided_smem<P>(pp.c).buf0 + b * pp.c.buf_elems, k, amax, th);
+    strided_fix<P>(pp.s, pp.use_tma != 0, ring_smem<P>(pp.c).buf0 + b * pp.c.buf_elems, k, amax, th);
     {
-      const StridedSmem<P> sm = strided_smem<P>(pp.c);
+      const RingSmem<P> sm = ring_smem<P>(pp.c);
       Tile<P, GroupThreads> t{sm.buf0 + b * pp.c.buf_elems, nullptr, pp.s.M, pp.s.log2m, 1, pp.s.M, 0, 0, nullptr, th};
-      constexpr int E = MODE == kStridedSmall ? StridedElems<P>::value / 2 : StridedElems<P>::value;
-      constexpr bool kFull = MODE == kStridedFull || MODE == kStridedFullWide;
-      cta_fft<P, DIR, E, kPointMajor, kRawNone, E, kFull>(t, sp, sm.tw, pp.c.tw_base);
+      constexpr int E = MODE == kTileSmall ? TileElems<P>::value / 2 : TileElems<P>::value;
+      constexpr bool kFull = MODE == kTileFull || MODE == kTileFullWide;
+      run_families<P, DIR, E, kPointMajor, kRawNone, E, kFull>(t, sm.tw, pp.s.N, pp.c.fam, 0);
     }
     {
       int xt, o1, o2;
       strided_decode(pp, tile, xt, o1, o2);
-      typename P::W* tb = strided_smem<P>(pp.c).buf0 + b * pp.c.buf_elems;
+      typename P::W* tb = ring_smem<P>(pp.c).buf0 + b * pp.c.buf_elems;
       rtile = !lag && tile + nb * step < pp.c.ntiles ? tile + nb * step : -1;
       rbuf = b;
       if (pp.tma_store) {
@@ -513,8 +480,8 @@ __global__ void __launch_bounds__(strided_max_threads(MODE), 1)
   __syncthreads();
   // a wait timed out: loads may be in flight that no group waits for
   if (threadIdx.x == 0 && pp.use_tma) {
-    const StridedSmem<P> sm = strided_smem<P>(pp.c);
-    if (sm.issued[nb])
+    const RingSmem<P> sm = ring_smem<P>(pp.c);
+    if (sm.cta[0])
       for (int i = 0; i < nb; ++i)
         if (sm.issued[i]) mbar_wait_bounded(&sm.mbar[i], (sm.issued[i] - 1) & 1, nullptr);
   }
@@ -522,17 +489,6 @@ __global__ void __launch_bounds__(strided_max_threads(MODE), 1)
 }
 
 // ---------------------------------------------------------------- X passes
-template <class P>
-P3G_D typename P::W* xpipe_buf(const PipeCommon& pc, int b) {
-  extern __shared__ unsigned char p3g_pipe_smem[];
-  return reinterpret_cast<typename P::W*>(align1k(p3g_pipe_smem)) + b * pc.buf_elems;
-}
-// the bulk copies' mbarriers, one per buffer, after the buffers
-template <class P>
-P3G_D uint64_t* xpipe_mbar(const PipeCommon& pc) {
-  return reinterpret_cast<uint64_t*>(xpipe_buf<P>(pc, pc.nbuf));
-}
-
 // cp.async of CH bytes (16, 8 or 4)
 template <int CH>
 P3G_D void cp_async_n(void* d, const void* g, uint32_t nb) {
@@ -543,38 +499,38 @@ P3G_D void cp_async_n(void* d, const void* g, uint32_t nb) {
 
 // Line by line: each thread copies every blockDim.x-th chunk of each line, with
 // the line's addresses formed once (lines at least blockDim.x chunks long).
-template <class P, int CH>
-P3G_D void xr2c_copy_lines(const XParams& x, const char* in, char* dst, int p0) {
+template <class P, int CH, class TH>
+P3G_D void xr2c_copy_lines(const XParams& x, const char* in, char* dst, int p0, const TH& th) {
   using UR = typename P::UR;
   const int lbytes = x.nx * (int)sizeof(UR);
-  const int step = (int)blockDim.x * CH;
+  const int step = th.count() * CH;
   for (int lt = 0; lt < 2 * x.M; ++lt) {
     const int line = 2 * p0 + lt;
     const bool ok = line < x.nlines;
     const char* g = in + (ok ? (long long)line * x.in_line * (long long)sizeof(UR) : 0LL);
     char* d = dst + lt * lbytes;
     const uint32_t nb = ok ? (uint32_t)CH : 0u;
-    for (int c = (int)threadIdx.x * CH; c < lbytes; c += step) cp_async_n<CH>(d + c, g + c, nb);
+    for (int c = th.tid() * CH; c < lbytes; c += step) cp_async_n<CH>(d + c, g + c, nb);
   }
 }
 
 // r2c: real lines 2p, 2p+1 of the tile (first pair p0 of field `field`)
 // copied raw ([line][x]) into dst, `chunk` bytes per copy, without a commit.
-template <class P>
-P3G_D void xr2c_copy(const XParams& x, int chunk, typename P::W* dst_w, int p0, int field) {
+template <class P, class TH = CtaThreads>
+P3G_D void xr2c_copy(const XParams& x, int chunk, typename P::W* dst_w, int p0, int field, const TH& th = TH()) {
   using UR = typename P::UR;
   const int M = x.M, N = x.nx;
   const char* in = reinterpret_cast<const char*>(static_cast<const UR*>(x.in) + field * x.in_field);
   char* dst = reinterpret_cast<char*>(dst_w);
   const int cpl = N * (int)sizeof(UR) / chunk;  // copies per line
-  if (cpl >= (int)blockDim.x) {
-    if (chunk == 16) xr2c_copy_lines<P, 16>(x, in, dst, p0);
-    else if (chunk == 8) xr2c_copy_lines<P, 8>(x, in, dst, p0);
-    else xr2c_copy_lines<P, 4>(x, in, dst, p0);
+  if (cpl >= th.count()) {
+    if (chunk == 16) xr2c_copy_lines<P, 16>(x, in, dst, p0, th);
+    else if (chunk == 8) xr2c_copy_lines<P, 8>(x, in, dst, p0, th);
+    else xr2c_copy_lines<P, 4>(x, in, dst, p0, th);
     return;
   }
   const FastDiv fcpl((uint32_t)cpl);
-  for (int e = threadIdx.x; e < 2 * M * cpl; e += blockDim.x) {
+  for (int e = th.tid(); e < 2 * M * cpl; e += th.count()) {
     const int lt = (int)fcpl.div((uint32_t)e);
     const int c = e - lt * cpl;
     const int line = 2 * p0 + lt;
@@ -588,49 +544,42 @@ P3G_D void xr2c_copy(const XParams& x, int chunk, typename P::W* dst_w, int p0, 
   }
 }
 
-// r2c tiles that arrive by one bulk copy: bulk loads on and the tile's 2M
-// lines all inside the field (a partial tile is zero-filled by cp.async)
-P3G_D bool xr2c_tile_bulk(const XPipeParams& q, int tile) {
-  if (!q.bulk) return false;
-  const int field = tile / q.c.tiles_per_field;
-  const int p0 = (tile - field * q.c.tiles_per_field) * q.x.M;
-  return 2 * (p0 + q.x.M) <= q.x.nlines;
-}
-
-// Copies of one r2c tile into buffer b: one bulk copy by thread 0 (with an
-// empty commit group so that every tile counts one group) or cp.async.
+// Copies of one r2c tile into buffer b by one group (strided_issue's rules).
 template <class P>
-P3G_D void xr2c_issue(const XPipeParams& q, int tile, int b) {
+P3G_D void xr2c_issue(const XPipeParams& q, int tile, int b, const GroupThreads& th) {
   using UR = typename P::UR;
+  const RingSmem<P> sm = ring_smem<P>(q.c);
+  typename P::W* dst = sm.buf0 + b * q.c.buf_elems;
   const int field = tile / q.c.tiles_per_field;
   const int p0 = (tile - field * q.c.tiles_per_field) * q.x.M;
-  if (xr2c_tile_bulk(q, tile)) {
-    if (threadIdx.x == 0) {
-      uint64_t* bar = xpipe_mbar<P>(q.c) + b;
-      const uint32_t bytes = (uint32_t)(2 * q.x.M * q.x.nx) * (uint32_t)sizeof(UR);
-      const UR* src = static_cast<const UR*>(q.x.in) + field * q.x.in_field + (long long)2 * p0 * q.x.nx;
+  if (q.bulk) {
+    if (th.t == 0) {
+      const int nl = min(2 * q.x.M, q.x.nlines - 2 * p0);
+      const uint32_t bytes = (uint32_t)(nl * q.x.nx) * (uint32_t)sizeof(UR);
+      ring_mark_issued(&sm.issued[b]);
       fence_proxy_async_smem();
-      mbar_arrive_expect_tx(bar, bytes);
-      bulk_load(xpipe_buf<P>(q.c, b), src, bytes, bar);
+      mbar_arrive_expect_tx(&sm.mbar[b], bytes);
+      bulk_load(dst, static_cast<const UR*>(q.x.in) + field * q.x.in_field + (long long)2 * p0 * q.x.nx, bytes,
+                &sm.mbar[b]);
     }
-  } else {
-    xr2c_copy<P>(q.x, q.chunk, xpipe_buf<P>(q.c, b), p0, field);
+    return;
   }
-  cp_async_commit();
+  if (th.t == 0) ring_mark_issued(&sm.issued[b]);
+  xr2c_copy<P>(q.x, q.chunk, dst, p0, field, th);
+  cp_async_mbar_arrive(&sm.mbar[b]);
 }
-
 
 // X1[k] = (Z[k] + conj Z[N-k]) / 2, X2[k] = -i (Z[k] - conj Z[N-k]) / 2,
 // modes k < nkeep stored to the working layout (USER: the user complex
 // format, for the X-only transform).
-template <class P, bool USER>
-P3G_D void xr2c_store_t(const XParams& x, const typename P::W* sm, int p0, int field, int kb) {
+template <class P, bool USER, class TH>
+P3G_D void xr2c_store_t(const XParams& x, const typename P::W* sm, int p0, int field, int kb, const TH& th) {
   using C = typename P::C;
   using O = typename std::conditional<USER, typename P::UC, typename P::W>::type;
   const int N = x.nx, nk = x.nkeep;
   O* out = static_cast<O*>(x.out) + field * x.out_field;
   const FastDiv fnk((uint32_t)nk);
-  for (int e = threadIdx.x; e < x.M * nk; e += blockDim.x) {
+  for (int e = th.tid(); e < x.M * nk; e += th.count()) {
     const int pr = (int)fnk.div((uint32_t)e);
     const int k = e - pr * nk;
     const int line = 2 * (p0 + pr);
@@ -648,71 +597,17 @@ P3G_D void xr2c_store_t(const XParams& x, const typename P::W* sm, int p0, int f
   }
 }
 // kb: the exponent bias of the user-format output (X-only transform)
-template <class P>
-P3G_D void xr2c_store(const XParams& x, const typename P::W* sm, int p0, int field, int kb) {
-  if (x.out_user) xr2c_store_t<P, true>(x, sm, p0, field, kb);
-  else xr2c_store_t<P, false>(x, sm, p0, field, kb);
-}
-
-template <class P, int E>
-__global__ void __launch_bounds__(XPipeLimits<P, E>::kMaxThreads, XPipeLimits<P, E>::kMinBlocks)
-    k_xr2c_pipe(const __grid_constant__ XPipeParams pp, const StagePlan* __restrict__ sp,
-                const float4* __restrict__ tw_g) {
-  const int k = range_k(pp.x.range);
-  const int nb = pp.c.nbuf;
-  uint32_t amax = 0;
-  int it = 0;
-  int tile = blockIdx.x;
-  if (pp.bulk && threadIdx.x == 0) {
-    for (int i = 0; i < nb; ++i) mbar_init(xpipe_mbar<P>(pp.c) + i, 1);
-    mbar_fence_init();
-  }
-  __syncthreads();
-  for (int j = 0; j < nb - 1; ++j) {
-    const int t = tile + j * (int)gridDim.x;
-    if (t < pp.c.ntiles) xr2c_issue<P>(pp, t, j);
-    else cp_async_commit();
-  }
-  int b = 0, ph = 0;  // buffer of iteration it and the parity of its use
-#pragma unroll 1
-  for (; tile < pp.c.ntiles; tile += gridDim.x, ++it) {
-    const int ahead = tile + (nb - 1) * (int)gridDim.x;
-    if (ahead < pp.c.ntiles) xr2c_issue<P>(pp, ahead, b == 0 ? nb - 1 : b - 1);
-    else cp_async_commit();
-    cp_async_wait_ahead(nb);
-    const bool ok = !xr2c_tile_bulk(pp, tile) || mbar_wait_bounded(xpipe_mbar<P>(pp.c) + b, ph, pp.c.err);
-    if (__syncthreads_or(!ok)) break;
-    {
-      // the first FFT stage reads the raw line pairs (packing fused into it)
-      Tile<P> t{xpipe_buf<P>(pp.c, b), nullptr, pp.x.M, pp.x.log2m, pp.x.LS, 1, pp.x.ps, k, &amax};
-      cta_fft<P, -1, E, kLineMajor, kRawR2C, PipeMaxR<P, E>::value>(t, sp, tw_g, 0);
-    }
-    {
-      const int field = tile / pp.c.tiles_per_field;
-      const int p0 = (tile - field * pp.c.tiles_per_field) * pp.x.M;
-      xr2c_store<P>(pp.x, xpipe_buf<P>(pp.c, b), p0, field, k);
-    }
-    __syncthreads();
-    if (++b == nb) {
-      b = 0;
-      ph ^= 1;
-    }
-  }
-  cp_async_wait<0>();
-  // early exit after a timed-out wait: wait (bounded) for bulk copies in flight
-  if (threadIdx.x == 0)
-    for (int j = 0; j < nb; ++j) {
-      const int t = tile + j * (int)gridDim.x;
-      if (t < pp.c.ntiles && xr2c_tile_bulk(pp, t))
-        mbar_wait_bounded(xpipe_mbar<P>(pp.c) + (it + j) % nb, ((it + j) / nb) & 1, nullptr);
-    }
-  range_flush(pp.x.range, amax);
+template <class P, class TH = CtaThreads>
+P3G_D void xr2c_store(const XParams& x, const typename P::W* sm, int p0, int field, int kb, const TH& th = TH()) {
+  if (x.out_user) xr2c_store_t<P, true>(x, sm, p0, field, kb, th);
+  else xr2c_store_t<P, false>(x, sm, p0, field, kb, th);
 }
 
 // c2r: complex lines 2p, 2p+1 of nh = N/2+1 modes copied raw (pair stride
 // 2 nh) into dst, modes beyond nkeep as zeros, without a commit.
-template <class P>
-P3G_D void xc2r_copy(const XParams& x, typename P::W* dst, int p0, int field) {
+template <class P, class TH = CtaThreads>
+P3G_D void xc2r_copy(const XParams& x, typename P::W* dst, int p0, int field, const TH& th = TH()) {
+  const int tid = th.tid(), nthr = th.count();
   using W = typename P::W;
   const int M = x.M, nh = x.nx / 2 + 1;
   const W* in = static_cast<const W*>(x.in) + field * x.in_field;
@@ -720,13 +615,13 @@ P3G_D void xc2r_copy(const XParams& x, typename P::W* dst, int p0, int field) {
     // two complexes per 16-byte copy: raw stride rs even, line pitch even
     const int rs = xc2r_raw_stride(nh, 8), hp = rs >> 1;
     if ((x.in_line & 1) == 0 && (reinterpret_cast<uintptr_t>(in) & 15) == 0) {
-      if (hp >= (int)blockDim.x) {  // line by line, addresses formed once per line
+      if (hp >= nthr) {  // line by line, addresses formed once per line
         for (int lt = 0; lt < 2 * M; ++lt) {
           const int line = 2 * p0 + lt;
           const int keep = line < x.nlines ? x.nkeep : 0;
           const W* g = in + (line < x.nlines ? (long long)line * x.in_line : 0LL);
           W* d = dst + lt * rs;
-          for (int k = 2 * (int)threadIdx.x; k < rs; k += 2 * (int)blockDim.x) {
+          for (int k = 2 * tid; k < rs; k += 2 * nthr) {
             const int nv = min(max(keep - k, 0), 2);
             cp_async16(d + k, nv ? g + k : in, (uint32_t)(8 * nv));
           }
@@ -734,7 +629,7 @@ P3G_D void xc2r_copy(const XParams& x, typename P::W* dst, int p0, int field) {
         return;
       }
       const FastDiv fhp((uint32_t)hp);
-      for (int e = threadIdx.x; e < 2 * M * hp; e += blockDim.x) {
+      for (int e = tid; e < 2 * M * hp; e += nthr) {
         const int lt = (int)fhp.div((uint32_t)e);
         const int k = 2 * (e - lt * hp);
         const int line = 2 * p0 + lt;
@@ -745,7 +640,7 @@ P3G_D void xc2r_copy(const XParams& x, typename P::W* dst, int p0, int field) {
       return;
     }
     const FastDiv fnh((uint32_t)nh);
-    for (int e = threadIdx.x; e < 2 * M * nh; e += blockDim.x) {
+    for (int e = tid; e < 2 * M * nh; e += nthr) {
       const int lt = (int)fnh.div((uint32_t)e);
       const int k = e - lt * nh;
       const int line = 2 * p0 + lt;
@@ -755,13 +650,13 @@ P3G_D void xc2r_copy(const XParams& x, typename P::W* dst, int p0, int field) {
     }
     return;
   }
-  if (nh >= (int)blockDim.x) {  // line by line, addresses formed once per line
+  if (nh >= nthr) {  // line by line, addresses formed once per line
     for (int lt = 0; lt < 2 * M; ++lt) {
       const int line = 2 * p0 + lt;
       const int keep = line < x.nlines ? x.nkeep : 0;
       const W* g = in + (line < x.nlines ? (long long)line * x.in_line : 0LL);
       W* d = dst + lt * nh;
-      for (int k = threadIdx.x; k < nh; k += blockDim.x) {
+      for (int k = tid; k < nh; k += nthr) {
         const bool ok = k < keep;
         if constexpr (sizeof(W) == 16) cp_async16(d + k, ok ? g + k : in, ok ? 16u : 0u);
         else cp_async8(d + k, ok ? g + k : in, ok ? 8u : 0u);
@@ -770,7 +665,7 @@ P3G_D void xc2r_copy(const XParams& x, typename P::W* dst, int p0, int field) {
     return;
   }
   const FastDiv fnh((uint32_t)nh);
-  for (int e = threadIdx.x; e < 2 * M * nh; e += blockDim.x) {
+  for (int e = tid; e < 2 * M * nh; e += nthr) {
     const int lt = (int)fnh.div((uint32_t)e);
     const int k = e - lt * nh;
     const int line = 2 * p0 + lt;
@@ -781,38 +676,40 @@ P3G_D void xc2r_copy(const XParams& x, typename P::W* dst, int p0, int field) {
   }
 }
 
-// Copies of one c2r tile into buffer b: one bulk copy per line (the nh
-// modes rounded up to 16 bytes, into the raw line stride) by thread 0, with an
-// empty commit group, or cp.async.
+// Copies of one c2r tile into buffer b by one group: one bulk copy per line
+// (the nkeep modes rounded up to 16 bytes; the kernel zeroes the modes beyond),
+// or cp.async.
 template <class P>
-P3G_D void xc2r_issue(const XPipeParams& q, int tile, int b) {
+P3G_D void xc2r_issue(const XPipeParams& q, int tile, int b, const GroupThreads& th) {
   using W = typename P::W;
+  const RingSmem<P> sm = ring_smem<P>(q.c);
+  W* dst = sm.buf0 + b * q.c.buf_elems;
   const int field = tile / q.c.tiles_per_field;
   const int p0 = (tile - field * q.c.tiles_per_field) * q.x.M;
   if (q.bulk) {
-    if (threadIdx.x == 0) {
-      const int nh = q.x.nx / 2 + 1;
-      const int rs = xc2r_raw_stride(nh, (int)sizeof(W));
-      const uint32_t lbytes = ((uint32_t)nh * (uint32_t)sizeof(W) + 15u) & ~15u;
+    if (th.t == 0) {
+      const int rs = xc2r_raw_stride(q.x.nx / 2 + 1, (int)sizeof(W));
+      const uint32_t lbytes = ((uint32_t)q.x.nkeep * (uint32_t)sizeof(W) + 15u) & ~15u;
       const int nl = min(2 * q.x.M, q.x.nlines - 2 * p0);
-      uint64_t* bar = xpipe_mbar<P>(q.c) + b;
       const W* in = static_cast<const W*>(q.x.in) + field * q.x.in_field;
-      W* dst = xpipe_buf<P>(q.c, b);
+      ring_mark_issued(&sm.issued[b]);
       fence_proxy_async_smem();
-      mbar_arrive_expect_tx(bar, lbytes * (uint32_t)nl);
-      for (int lt = 0; lt < nl; ++lt) bulk_load(dst + lt * rs, in + (long long)(2 * p0 + lt) * q.x.in_line, lbytes, bar);
+      mbar_arrive_expect_tx(&sm.mbar[b], lbytes * (uint32_t)nl);
+      for (int lt = 0; lt < nl; ++lt)
+        bulk_load(dst + lt * rs, in + (long long)(2 * p0 + lt) * q.x.in_line, lbytes, &sm.mbar[b]);
     }
-  } else {
-    xc2r_copy<P>(q.x, xpipe_buf<P>(q.c, b), p0, field);
+    return;
   }
-  cp_async_commit();
+  if (th.t == 0) ring_mark_issued(&sm.issued[b]);
+  xc2r_copy<P>(q.x, dst, p0, field, th);
+  cp_async_mbar_arrive(&sm.mbar[b]);
 }
 
 // x1 = Re z, x2 = Im z to the user's real lines (format conversion fused).
 // Even N: each thread takes positions n, n+1 of a line pair, reads the two
 // complex values once and writes two-element vectors to both lines.
-template <class P>
-P3G_D void xc2r_store(const XParams& x, const typename P::W* sm, int p0, int field, int k) {
+template <class P, class TH = CtaThreads>
+P3G_D void xc2r_store(const XParams& x, const typename P::W* sm, int p0, int field, int k, const TH& th = TH()) {
   using W = typename P::W;
   using UR = typename P::UR;
   const int M = x.M, N = x.nx, LS = x.LS, ps = x.ps;
@@ -822,7 +719,7 @@ P3G_D void xc2r_store(const XParams& x, const typename P::W* sm, int p0, int fie
   if (vec) {
     const int NH = N >> 1;
     const FastDiv fNH((uint32_t)NH);
-    for (int e = threadIdx.x; e < M * NH; e += blockDim.x) {
+    for (int e = th.tid(); e < M * NH; e += th.count()) {
       const int pr = (int)fNH.div((uint32_t)e);
       const int n = 2 * (e - pr * NH);
       const int line = 2 * (p0 + pr);
@@ -845,7 +742,7 @@ P3G_D void xc2r_store(const XParams& x, const typename P::W* sm, int p0, int fie
   const float* smf = reinterpret_cast<const float*>(sm);
   constexpr int kW = sizeof(W) / sizeof(float);
   const FastDiv fN((uint32_t)N);
-  for (int e = threadIdx.x; e < 2 * M * N; e += blockDim.x) {
+  for (int e = th.tid(); e < 2 * M * N; e += th.count()) {
     const int lt = (int)fN.div((uint32_t)e);
     const int n = e - lt * N;
     const int line = 2 * p0 + lt;
@@ -857,55 +754,110 @@ P3G_D void xc2r_store(const XParams& x, const typename P::W* sm, int p0, int fie
   }
 }
 
-template <class P, int E>
-__global__ void __launch_bounds__(XPipeLimits<P, E>::kMaxThreads, XPipeLimits<P, E>::kMinBlocks)
-    k_xc2r_pipe(const __grid_constant__ XPipeParams pp, const StagePlan* __restrict__ sp,
-                const float4* __restrict__ tw_g) {
-  const int k = range_k(pp.x.range);
-  int it = 0;
-  const int nb = pp.c.nbuf;
-  int tile = blockIdx.x;
-  if (pp.bulk && threadIdx.x == 0) {
-    for (int i = 0; i < nb; ++i) mbar_init(xpipe_mbar<P>(pp.c) + i, 1);
-    mbar_fence_init();
+// X passes in groups over a ring of buffers, as k_strided_pipe; a tile is M
+// line pairs.  Lines are contiguous in memory, so the tiles can be as small as
+// two warps' work and eight groups keep the SM's FMA pipes, shared memory and
+// stores busy at once.  The first FFT stage reads the raw line pairs (packing
+// or Hermitian merge and format conversion fused into it).
+template <class P, bool R2C, int MODE>
+__global__ void __launch_bounds__(tile_max_threads(MODE, true), 1)
+    k_x_pipe(const __grid_constant__ XPipeParams pp, const float4* __restrict__ tw_g) {
+  const int nb = pp.c.nbuf, G = pp.c.groups;
+  const int step = (int)gridDim.x;
+  {
+    const RingSmem<P> sm = ring_smem<P>(pp.c);
+    for (int i = threadIdx.x; i < pp.c.tw_count; i += blockDim.x) sm.tw[i] = __ldg(tw_g + pp.c.tw_base + i);
+    if (threadIdx.x == 0) {
+      for (int i = 0; i < nb; ++i) {
+        mbar_init(&sm.mbar[i], pp.bulk ? 1 : pp.c.gthreads);
+        sm.issued[i] = 0;
+      }
+      sm.cta[0] = 0;
+      sm.cta[1] = range_k(pp.x.range);
+      sm.cta[2] = 0;
+      mbar_fence_init();
+    }
   }
   __syncthreads();
-  for (int j = 0; j < nb - 1; ++j) {
-    const int t = tile + j * (int)gridDim.x;
-    if (t < pp.c.ntiles) xc2r_issue<P>(pp, t, j);
-    else cp_async_commit();
-  }
-  int b = 0, ph = 0;  // buffer of iteration it and the parity of its use
+  // the exponent bias and the largest input seen live in shared memory: no
+  // register of theirs is held across the stages
+  const int g = (int)threadIdx.x / pp.c.gthreads;
+  const GroupThreads th{(int)threadIdx.x - g * pp.c.gthreads, pp.c.gthreads, 1 + g};
+  auto issue = [&](int tile, int b) {
+    if constexpr (R2C) xr2c_issue<P>(pp, tile, b, th);
+    else xc2r_issue<P>(pp, tile, b, th);
+  };
+  for (int j = 0, tile = blockIdx.x; j < nb && tile < pp.c.ntiles; ++j, tile += step)
+    if (pp.bulk ? g == 0 : j % G == g) issue(tile, j);
+  int b = g, use = 0;  // this tile's buffer and how often it was used before
 #pragma unroll 1
-  for (; tile < pp.c.ntiles; tile += gridDim.x, ++it) {
-    const int ahead = tile + (nb - 1) * (int)gridDim.x;
-    if (ahead < pp.c.ntiles) xc2r_issue<P>(pp, ahead, b == 0 ? nb - 1 : b - 1);
-    else cp_async_commit();
-    cp_async_wait_ahead(nb);
-    const bool ok = !pp.bulk || mbar_wait_bounded(xpipe_mbar<P>(pp.c) + b, ph, pp.c.err);
-    if (__syncthreads_or(!ok)) break;
-    {
-      // the first FFT stage reads the raw half spectra (Hermitian merge fused into it)
-      Tile<P> t{xpipe_buf<P>(pp.c, b), nullptr, pp.x.M, pp.x.log2m, pp.x.LS, 1, pp.x.ps};
-      cta_fft<P, 1, E, kLineMajor, kRawC2R, PipeMaxR<P, E>::value>(t, sp, tw_g, 0);
+  for (int tile = blockIdx.x + g * step; tile < pp.c.ntiles; tile += G * step) {
+    const bool ok = ring_wait(&ring_smem<P>(pp.c).mbar[b], &ring_smem<P>(pp.c).issued[b], use, pp.c.err);
+    if (th.sync_or(!ok)) {
+      if (th.t == 0) ring_smem<P>(pp.c).cta[0] = 1;
+      break;
+    }
+    const RingSmem<P> sm = ring_smem<P>(pp.c);
+    typename P::W* tb = sm.buf0 + b * pp.c.buf_elems;
+    auto place = [&](int& field, int& p0) {
+      field = tile / pp.c.tiles_per_field;
+      p0 = (tile - field * pp.c.tiles_per_field) * pp.x.M;
+    };
+    int field, p0;
+    place(field, p0);
+    if (pp.bulk && 2 * (p0 + pp.x.M) > pp.x.nlines) {  // the field's last tile: zeros for the lines it lacks
+      const int from = pp.x.nlines - 2 * p0, lines = 2 * pp.x.M - from;
+      const int words = (R2C ? pp.x.nx * (int)sizeof(typename P::UR)
+                             : xc2r_raw_stride(pp.x.nx / 2 + 1, (int)sizeof(typename P::W)) * (int)sizeof(typename P::W)) / 4;
+      float* z = reinterpret_cast<float*>(tb) + (long long)from * words;
+      for (int e = th.t; e < lines * words; e += th.n) z[e] = 0.0f;
+      th.sync();
+    }
+    if constexpr (!R2C) {
+      const int nh = pp.x.nx / 2 + 1, drop = nh - pp.x.nkeep;
+      if (pp.bulk && drop > 0) {  // the x modes the pruned spectrum lacks
+        const int rs = xc2r_raw_stride(nh, (int)sizeof(typename P::W));
+        const FastDiv fd((uint32_t)drop);
+        for (int e = th.t; e < 2 * pp.x.M * drop; e += th.n) {
+          const int lt = (int)fd.div((uint32_t)e);
+          tb[lt * rs + pp.x.nkeep + e - lt * drop] = P::to_w(P::zero());
+        }
+        th.sync();
+      }
     }
     {
-      const int field = tile / pp.c.tiles_per_field;
-      const int p0 = (tile - field * pp.c.tiles_per_field) * pp.x.M;
-      xc2r_store<P>(pp.x, xpipe_buf<P>(pp.c, b), p0, field, k);
+      constexpr int E = MODE == kTileSmall ? TileElems<P>::value / 2 : TileElems<P>::value;
+      constexpr bool kFull = MODE == kTileFull || MODE == kTileFullWide;
+      uint32_t amax = 0;
+      Tile<P, GroupThreads> t{tb, nullptr, pp.x.M, pp.x.log2m, pp.x.LS, 1, pp.x.ps, R2C ? sm.cta[1] : 0,
+                              R2C ? &amax : nullptr, th, R2C ? reinterpret_cast<unsigned*>(&sm.cta[2]) : nullptr};
+      run_families<P, R2C ? -1 : 1, E, kLineMajor, R2C ? kRawR2C : kRawC2R, E, kFull>(t, sm.tw, pp.x.nx, pp.c.fam, 0);
     }
-    __syncthreads();
-    if (++b == nb) {
-      b = 0;
-      ph ^= 1;
+    asm volatile("" : "+r"(tile));  // the tile's place again, rather than held across the stages
+    place(field, p0);
+    const int k = ring_smem<P>(pp.c).cta[1];
+    if constexpr (R2C) xr2c_store<P>(pp.x, tb, p0, field, k, th);
+    else xc2r_store<P>(pp.x, tb, p0, field, k, th);
+    th.sync();
+    if (tile + nb * step < pp.c.ntiles) issue(tile + nb * step, b);
+    b += G;
+    if (b >= nb) {
+      b -= nb;
+      ++use;
     }
   }
-  cp_async_wait<0>();
-  // early exit after a timed-out wait: wait (bounded) for bulk copies in flight
-  if (pp.bulk && threadIdx.x == 0)
-    for (int j = 0; j < nb; ++j)
-      if (tile + j * (int)gridDim.x < pp.c.ntiles)
-        mbar_wait_bounded(xpipe_mbar<P>(pp.c) + (it + j) % nb, ((it + j) / nb) & 1, nullptr);
+  if (!pp.bulk) cp_async_wait<0>();
+  __syncthreads();
+  // a wait timed out: loads may be in flight that no group waits for
+  if (threadIdx.x == 0 && pp.bulk) {
+    const RingSmem<P> sm = ring_smem<P>(pp.c);
+    if (sm.cta[0])
+      for (int i = 0; i < nb; ++i)
+        if (sm.issued[i]) mbar_wait_bounded(&sm.mbar[i], (sm.issued[i] - 1) & 1, nullptr);
+  }
+  if constexpr (R2C) {
+    if (threadIdx.x < 32) range_flush(pp.x.range, threadIdx.x == 0 ? (uint32_t)ring_smem<P>(pp.c).cta[2] : 0u);
+  }
 }
 
 }  // namespace p3g

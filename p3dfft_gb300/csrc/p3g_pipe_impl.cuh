@@ -1,0 +1,48 @@
+// Launchers of the pipelined kernels: one translation unit per path and
+// direction (the unrolled codelets dominate the build time).
+#pragma once
+
+#include "p3g_pipe.cuh"
+
+namespace p3g {
+
+template <class P, int DIR>
+cudaError_t launch_strided_pipe(const CUtensorMap* map, const CUtensorMap* omap, const SPipeParams& p,
+                                const float4* tw, TileMode mode, int threads, size_t smem, int grid,
+                                cudaStream_t st) {
+  auto kernel = k_strided_pipe<P, DIR, kTileGeneral>;
+  if (mode == kTileFull) kernel = k_strided_pipe<P, DIR, kTileFull>;
+  if (mode == kTileSmall) kernel = k_strided_pipe<P, DIR, kTileSmall>;
+  if constexpr (!P::kF64) {
+    if (mode == kTileFullWide) kernel = k_strided_pipe<P, DIR, kTileFullWide>;
+  }
+  const cudaError_t e = opt_in_smem((const void*)kernel, 227 * 1024);
+  if (e != cudaSuccess) return e;
+  kernel<<<grid, threads, smem, st>>>(*map, *omap, p, tw);
+  return cudaGetLastError();
+}
+
+template <class P, bool R2C>
+cudaError_t launch_x_pipe(const XPipeParams& p, const float4* tw, TileMode mode, int threads,
+                          size_t smem, int grid, cudaStream_t st) {
+  auto kernel = k_x_pipe<P, R2C, kTileGeneral>;
+  if (mode == kTileFull) kernel = k_x_pipe<P, R2C, kTileFull>;
+  if (mode == kTileSmall) kernel = k_x_pipe<P, R2C, kTileSmall>;
+  if constexpr (!P::kF64) {
+    if (mode == kTileFullWide) kernel = k_x_pipe<P, R2C, kTileFullWide>;
+  }
+  const cudaError_t e = opt_in_smem((const void*)kernel, 227 * 1024);
+  if (e != cudaSuccess) return e;
+  kernel<<<grid, threads, smem, st>>>(p, tw);
+  return cudaGetLastError();
+}
+
+#define P3G_X_INSTANTIATE(P, R2C)                                                                              \
+  template cudaError_t launch_x_pipe<P, R2C>(const XPipeParams&, const float4*, TileMode, int, \
+                                             size_t, int, cudaStream_t);
+#define P3G_STRIDED_INSTANTIATE(P, DIR)                                                                       \
+  template cudaError_t launch_strided_pipe<P, DIR>(const CUtensorMap*, const CUtensorMap*, const SPipeParams&, \
+                                                   const float4*, TileMode, int, size_t, int,    \
+                                                   cudaStream_t);
+
+}  // namespace p3g

@@ -273,14 +273,6 @@ static bool size_tile(AxisPlan& ap, int n, int lines_avail, bool f64, int max_m 
   return ap.smem <= 227 * 1024;
 }
 
-// Launch shape of an X pass kernel with E elements per thread: the most
-// threads per CTA and the registers per thread its launch bounds allow.
-template <class P, int E>
-static void pipe_shape(int& max_threads, int& regs) {
-  max_threads = XPipeLimits<P, E>::kMaxThreads;
-  regs = std::min(255, 65536 / (max_threads * XPipeLimits<P, E>::kMinBlocks));
-}
-
 // Strided pipelined kernel (k_strided_pipe): one CTA per SM of g groups of tg
 // threads, each group on tiles of M columns, and a ring of nbuf buffers (1 KB
 // aligned), the axis's twiddles and the buffers' mbarriers in shared memory.
@@ -304,7 +296,7 @@ static void size_strided(AxisPlan& ap, bool f64, int X, int O1, int max_m, int s
   ap.pipe_ok = false;
   if (ap.sp.nstages < 1 || ap.sp.has_generic || ap.n < 2) return;
   const size_t esize = f64 ? 16 : 8;
-  const int Emax = f64 ? StridedElems<PathF64>::value : StridedElems<PathF32>::value;
+  const int Emax = f64 ? TileElems<PathF64>::value : TileElems<PathF32>::value;
   const int n = ap.n;
   const size_t room = 227 * 1024;
   const int wide_index = ap.spw_index;
@@ -330,11 +322,11 @@ static void size_strided(AxisPlan& ap, bool f64, int X, int O1, int max_m, int s
         // of its own and groups that drift apart spread over more pages at a
         // time (Y of 1024^3, 4.2 MB apart: 1.95 ms with two groups, 1.81 ms
         // with one; of 768 x 1024 x 540, 1.7 MB apart: 0.59 against 0.73 ms)
-        const StridedMode mode =
-            E < Emax ? kStridedSmall : (!full ? kStridedGeneral : (!f64 && (tstore || far_rows) ? kStridedFullWide : kStridedFull));
-        const int max_threads = strided_max_threads(mode);
+        const TileMode mode =
+            E < Emax ? kTileSmall : (!full ? kTileGeneral : (!f64 && (tstore || far_rows) ? kTileFullWide : kTileFull));
+        const int max_threads = tile_max_threads(mode);
         const size_t buf = ((size_t)M * n * esize + 1023) / 1024 * 1024;
-        if (tg > strided_max_threads(kStridedGeneral) || fixed + 2 * buf > room) break;
+        if (tg > tile_max_threads(kTileGeneral) || fixed + 2 * buf > room) break;
         if (tg > max_threads) continue;
         const int fit = (int)std::min<size_t>((room - fixed) / buf, kMaxTileBuffers);
         const double tiles = (double)((X + M - 1) / M) * O1;
@@ -346,8 +338,8 @@ static void size_strided(AxisPlan& ap, bool f64, int X, int O1, int max_m, int s
         if (E < Emax && per_sm > g) continue;
         const size_t row = M * esize;
         const double rows = row >= 128 ? 1.0 : (row >= 64 ? 0.97 : (row >= 32 ? 0.45 : 0.25));
-        const double warps = (mode == kStridedFullWide ? 1.5 : 1.0) * g * tg / 32;
-        const double overlap = std::min(1.0, warps / 12) * (g >= 2 || mode == kStridedFullWide ? 1.0 : 0.8);
+        const double warps = (mode == kTileFullWide ? 1.5 : 1.0) * g * tg / 32;
+        const double overlap = std::min(1.0, warps / 12) * (g >= 2 || mode == kTileFullWide ? 1.0 : 0.8);
         const double clocks = (f64 ? 1.0 : 0.35) * sp.nstages;
         const double t = per_sm * tg * E * clocks / (rows * overlap) + 100.0 * E * sp.nstages / (f64 ? 1 : 2);
         if (t < best * 0.999) {
@@ -372,65 +364,68 @@ static void size_strided(AxisPlan& ap, bool f64, int X, int O1, int max_m, int s
   if (ap.pipe_ok) ap.spw_index = use_wide;
 }
 
-// X pass kernels: two or three tile buffers (1 KB aligned) and their
-// mbarriers in shared memory.  kind: 1 r2c, 2 c2r.  The elements per thread
-// follow the axis's stage plans: 8 on F64; 32 on F32 with the wide plan, else 16.
-static void size_pipe(AxisPlan& ap, int kind, bool f64, int thread_cap = 0) {
+// X pass kernels (k_x_pipe): as size_strided; a tile is M line pairs of n
+// points (line stride ls in the padded layout) or their raw lines, whichever
+// takes more.  Lines are contiguous, so the smallest tile of two warps or more
+// is taken: up to eight groups per SM.
+static void size_x(AxisPlan& ap, bool f64, long long pairs, int max_m, int sm_count) {
   ap.pipe_ok = false;
   if (ap.sp.nstages < 1 || ap.sp.has_generic || ap.n < 2) return;
   const size_t esize = f64 ? 16 : 8;
-  const int E = f64 ? (ap.spw_index >= 0 ? 16 : 8) : (ap.spw_index >= 0 ? 32 : 16);
-  ap.pipe_e = E;
-  int max_threads = 0, regs_max = 0;
-  if (f64) {
-    if (E == 16) pipe_shape<PathF64, 16>(max_threads, regs_max);
-    else pipe_shape<PathF64, 8>(max_threads, regs_max);
-  } else if (E == 32) pipe_shape<PathF32, 32>(max_threads, regs_max);
-  else pipe_shape<PathF32, 16>(max_threads, regs_max);
-  if (thread_cap > 0 && thread_cap < max_threads) max_threads = thread_cap;
+  const int Emax = f64 ? TileElems<PathF64>::value : TileElems<PathF32>::value;
   const int n = ap.n;
-  const int nh = n / 2 + 1;
-  auto threads_for = [&](int M) { return round_threads((M * n + E - 1) / E); };
-  auto smem_for = [&](int M, size_t& buf_bytes, int nbuf = 2) {
-    // buffer stride rounded to 1 KB so every buffer stays aligned
-    const int raw = 2 * xc2r_raw_stride(nh, (int)esize);  // c2r raw line pair
-    const int ls = ap.pipe_ls();
-    const size_t need = (size_t)(M * (ls > raw ? ls : raw)) * esize;
-    buf_bytes = (need + 1023) / 1024 * 1024;
-    return 1024 + nbuf * buf_bytes + 8 * nbuf + 16;
-  };
-  // resident warps per SM for tile width M: registers per thread from the
-  // kernel's launch bounds, 2048 threads and ~228 KB of shared memory per SM
-  auto warps_for = [&](int M, int nbuf = 2) {
-    const int t = threads_for(M);
-    size_t bb;
-    const size_t sm = smem_for(M, bb, nbuf);
-    int b = 65536 / (regs_max * t);
-    b = std::min(b, 2048 / t);
-    b = std::min(b, (int)((228 * 1024) / sm));
-    return b * t / 32;
-  };
-  // widest tile whose CTA fits the kernel; a narrower one (down to half of
-  // that, at least 2 lines) only when it keeps 1.5x more warps resident
-  int M = ap.M;
-  while (M > 1 && threads_for(M) > max_threads) M /= 2;
-  if (threads_for(M) > max_threads) return;
-  const int w0 = warps_for(M);
-  if (M >= 4 && 2 * warps_for(M / 2) >= 3 * w0) M /= 2;
-  ap.pipe_threads = threads_for(M);
-  ap.pipe_m = M;
-  ap.pipe_log2m = ilog2(M);
-  // a third tile buffer (loads two tiles ahead) where it fits without costing
-  // resident warps
-  size_t buf_bytes = 0;
-  ap.pipe_nbuf = 2;
-  if (smem_for(M, buf_bytes, 3) <= 227 * 1024 && warps_for(M, 3) >= warps_for(M, 2)) ap.pipe_nbuf = 3;
-  ap.pipe_smem = smem_for(M, buf_bytes, ap.pipe_nbuf);
-  ap.buf_elems = (int)(buf_bytes / esize);
-  ap.pipe_ok = ap.pipe_smem <= 227 * 1024;
+  const size_t room = 227 * 1024;
+  const int wide_index = ap.spw_index;
+  int use_wide = wide_index;
+  double best = 1e300;
+  for (int narrow = wide_index >= 0 ? 0 : 1; narrow < 2; ++narrow) {
+    const StagePlan& sp = narrow ? ap.sp : ap.spw;
+    bool pow2 = true;
+    int rmax = 0;
+    for (int i = 0; i < sp.nstages; ++i) {
+      pow2 = pow2 && (sp.radix[i] & (sp.radix[i] - 1)) == 0;
+      rmax = std::max(rmax, sp.radix[i]);
+    }
+    const size_t fixed = 1024 + (size_t)(narrow ? ap.tw_cnt : ap.tw_cnt_w) * 16 + 256;
+    const int ls = narrow ? ap.ls : ap.ls_w;
+    const int raw = 2 * xc2r_raw_stride(n / 2 + 1, (int)esize);
+    for (int E = Emax; E >= Emax / 2 && E >= rmax; E /= 2) {
+      for (int M = 1; M <= max_m && M < 2 * pairs; M *= 2) {
+        const int tg = stage_threads(sp, M, E);
+        const bool full = pow2 && (long long)M * n == (long long)tg * E;
+        const TileMode mode =
+            E < Emax ? kTileSmall : (!full ? kTileGeneral : (f64 ? kTileFull : kTileFullWide));
+        const int max_threads = tile_max_threads(mode, true);
+        const size_t buf = ((size_t)M * std::max(ls, raw) * esize + 1023) / 1024 * 1024;
+        if (tg > tile_max_threads(kTileGeneral) || fixed + 2 * buf > room) break;
+        if (tg > max_threads) continue;
+        const int fit = (int)std::min<size_t>((room - fixed) / buf, kMaxTileBuffers);
+        const double per_sm = std::ceil((double)((pairs + M - 1) / M) / sm_count);
+        const int g = (int)std::max(
+            1.0, std::min({(double)(max_threads / tg), (double)kMaxGroups, (double)(fit - 1), per_sm}));
+        if (E < Emax && per_sm > g) continue;  // every tile has a group of its own
+        const double warps = (mode == kTileFullWide ? 1.3 : 1.0) * g * tg / 32;
+        const double overlap = std::min(1.0, warps / 12) * (g >= 2 ? 1.0 : 0.8) * (tg >= 64 ? 1.0 : 0.9);
+        const double clocks = (f64 ? 1.0 : 0.35) * sp.nstages;
+        const double t = per_sm * tg * E * clocks / overlap + 100.0 * E * sp.nstages / (f64 ? 1 : 2);
+        if (t < best * 0.999) {
+          best = t;
+          use_wide = narrow ? -1 : wide_index;
+          ap.pipe_ok = true;
+          ap.pipe_m = M;
+          ap.pipe_log2m = ilog2(M);
+          ap.pipe_mode = mode;
+          ap.pipe_g = g;
+          ap.pipe_threads = g * tg;
+          ap.pipe_nbuf = std::min(fit, g + (g >= 4 ? 2 : 1));
+          ap.buf_elems = (int)(buf / esize);
+          ap.pipe_smem = fixed + ap.pipe_nbuf * buf;
+        }
+      }
+    }
+  }
+  if (ap.pipe_ok) ap.spw_index = use_wide;
 }
-
-
 
 }  // namespace p3g
 
@@ -637,6 +632,7 @@ int run_strided(p3g_plan p, SParams& s, const AxisPlan& ap, bool fwd_sign, int n
     pp.c.ntiles = pp.c.tiles_per_field * nv;
     pp.c.tw_base = ap.pipe_tw_lo();
     pp.c.tw_count = ap.pipe_tw_cnt();
+    pp.c.fam = ap.pipe_fam();
     pp.c.buf_elems = ap.buf_elems;
     pp.c.nbuf = ap.pipe_nbuf;
     pp.c.groups = ap.pipe_g;
@@ -678,7 +674,7 @@ int run_strided(p3g_plan p, SParams& s, const AxisPlan& ap, bool fwd_sign, int n
     const int slots = max_sms > 0 && max_sms < p->sm_count ? max_sms : p->sm_count;
     const int grid = pp.c.ntiles < slots ? pp.c.ntiles : slots;
     const auto launch = fwd_sign ? launch_strided_pipe<P, -1> : launch_strided_pipe<P, 1>;
-    cudaError_t e = launch(&map, &omap, pp, p->d_sp + ap.pipe_sp(), p->d_tw, ap.pipe_mode, ap.pipe_threads,
+    cudaError_t e = launch(&map, &omap, pp, p->d_tw, ap.pipe_mode, ap.pipe_threads,
                            ap.pipe_smem, grid, st);
     if (e != cudaSuccess) return fail(P3G_E_CUDA, std::string("strided pass launch: ") + cudaGetErrorString(e));
     p->launches++;
@@ -711,16 +707,19 @@ int run_x_r2c(p3g_plan p, XParams& x, int nv, cudaStream_t st, int max_sms = 0) 
     xp.c.ntiles = x.tiles * nv;
     xp.c.tw_base = ap.pipe_tw_lo();
     xp.c.tw_count = ap.pipe_tw_cnt();
+    xp.c.fam = ap.pipe_fam();
     xp.c.buf_elems = ap.buf_elems;
     xp.c.nbuf = ap.pipe_nbuf;
+    xp.c.groups = ap.pipe_g;
+    xp.c.gthreads = ap.pipe_threads / ap.pipe_g;
     xp.c.err = p->d_err;
     // the tile's 2M real lines are one contiguous run of device memory
     xp.bulk = x.in_line == x.nx && (x.nx * us) % 16 == 0 && (x.in_field * us) % 16 == 0 && aligned_to(x.in, 16) &&
               device_memory(x.in);
-    const int slots = (max_sms > 0 && max_sms < p->sm_count ? max_sms : p->sm_count) * ap.pipe_bps;
+    const int slots = max_sms > 0 && max_sms < p->sm_count ? max_sms : p->sm_count;
     const int grid = xp.c.ntiles < slots ? xp.c.ntiles : slots;
-    cudaError_t e = launch_xr2c_pipe<P>(xp, p->d_sp + ap.pipe_sp(), p->d_tw, ap.pipe_e, ap.pipe_threads,
-                                        ap.pipe_smem, grid, st);
+    cudaError_t e = launch_x_pipe<P, true>(xp, p->d_tw, ap.pipe_mode, ap.pipe_threads,
+                                            ap.pipe_smem, grid, st);
     if (e != cudaSuccess) return fail(P3G_E_CUDA, std::string("X r2c launch: ") + cudaGetErrorString(e));
     p->launches++;
     return P3G_OK;
@@ -733,7 +732,7 @@ int run_x_r2c(p3g_plan p, XParams& x, int nv, cudaStream_t st, int max_sms = 0) 
 
 template <class P>
 int run_x_c2r(p3g_plan p, XParams& x, int nv, cudaStream_t st, int max_sms = 0) {
-  const AxisPlan& ap = p->ax_xc;
+  const AxisPlan& ap = p->ax_x;
   if (p->use_pipe && ap.pipe_ok) {
     x.M = ap.pipe_m;
     x.log2m = ap.pipe_log2m;
@@ -747,22 +746,24 @@ int run_x_c2r(p3g_plan p, XParams& x, int nv, cudaStream_t st, int max_sms = 0) 
     xp.c.ntiles = x.tiles * nv;
     xp.c.tw_base = ap.pipe_tw_lo();
     xp.c.tw_count = ap.pipe_tw_cnt();
+    xp.c.fam = ap.pipe_fam();
     xp.c.buf_elems = ap.buf_elems;
     xp.c.nbuf = ap.pipe_nbuf;
+    xp.c.groups = ap.pipe_g;
+    xp.c.gthreads = ap.pipe_threads / ap.pipe_g;
     xp.c.err = p->d_err;
     {
-      // every mode of a line arrives by one bulk copy of its nh complexes
-      // rounded up to 16 bytes, which the line pitch and the raw stride hold
+      // the modes of a line arrive by one bulk copy, rounded up to 16 bytes,
+      // which the line pitch and the raw stride hold
       const long long es = (long long)sizeof(typename P::W);
-      const int nh = x.nx / 2 + 1;
-      xp.bulk = x.nkeep == nh && (x.in_line * es) % 16 == 0 && (x.in_field * es) % 16 == 0 &&
-                (long long)x.in_line * es >= ((nh * es + 15) / 16) * 16 && aligned_to(x.in, 16) &&
+      xp.bulk = (x.in_line * es) % 16 == 0 && (x.in_field * es) % 16 == 0 &&
+                (long long)x.in_line * es >= ((x.nkeep * es + 15) / 16) * 16 && aligned_to(x.in, 16) &&
                 device_memory(x.in);
     }
-    const int slots = (max_sms > 0 && max_sms < p->sm_count ? max_sms : p->sm_count) * ap.pipe_bps;
+    const int slots = max_sms > 0 && max_sms < p->sm_count ? max_sms : p->sm_count;
     const int grid = xp.c.ntiles < slots ? xp.c.ntiles : slots;
-    cudaError_t e = launch_xc2r_pipe<P>(xp, p->d_sp + ap.pipe_sp(), p->d_tw, ap.pipe_e, ap.pipe_threads,
-                                        ap.pipe_smem, grid, st);
+    cudaError_t e = launch_x_pipe<P, false>(xp, p->d_tw, ap.pipe_mode, ap.pipe_threads,
+                                            ap.pipe_smem, grid, st);
     if (e != cudaSuccess) return fail(P3G_E_CUDA, std::string("X c2r launch: ") + cudaGetErrorString(e));
     p->launches++;
     return P3G_OK;
@@ -1560,7 +1561,7 @@ int p3g_plan_create_tuned(p3g_plan* out, int nx, int ny, int nz, int nxc, int ny
   // on the Y pass only (1024 points: 8.2 -> 7.8 ms at 1024^3; the X passes'
   // 128-thread CTAs and the Z passes' user-format stores ran slower with it)
   auto wide_ok = [&](const AxisPlan& ap, int n) {
-    if (f64) return &ap != &p->ax_x && (max_radix == 0 || max_radix >= 16);
+    if (f64) return max_radix == 0 || max_radix >= 16;
     if ((n & (n - 1)) != 0) return false;
     return max_radix == 0 || max_radix >= 32;
   };
@@ -1598,20 +1599,18 @@ int p3g_plan_create_tuned(p3g_plan* out, int nx, int ny, int nz, int nxc, int ny
     return bad("a plane of more than 2^31 elements is not supported");
   const bool x_fits = add_axis(p->ax_x, nx, (ny * nz + 1) / 2);
   {
-    // line padding for the X tiles (pad_index in p3g_engine.cuh): only for
-    // all-power-of-two plans whose every N/R is a multiple of the first radix
+    // line padding for the X tiles (pad_index in p3g_engine.cuh): one element
+    // every 2^ps, the largest 2^ps that divides the first radix and every N/R
     AxisPlan& ax = p->ax_x;
     const int nh2 = 2 * (nx / 2 + 1);
     auto pad_of = [&](const StagePlan& sp, int& ps, int& ls) {
       ps = 0;
       if (sp.nstages > 0 && !sp.has_generic) {
-        const int r0 = sp.radix[0];
-        bool ok = (r0 & (r0 - 1)) == 0 && r0 >= 4;
-        for (int i = 0; ok && i < sp.nstages; ++i) {
-          const int r = sp.radix[i];
-          ok = (r & (r - 1)) == 0 && (nx / r) % r0 == 0;
-        }
-        if (ok) ps = ilog2(r0);
+        ps = 5;
+        for (int i = 0; i < sp.nstages; ++i)
+          while (ps > 0 && (nx / sp.radix[i]) % (1 << ps) != 0) --ps;
+        while (ps > 0 && sp.radix[0] % (1 << ps) != 0) --ps;
+        if (ps < 2) ps = 0;
       }
       ls = nx + (ps ? nx >> ps : 0);
       if (ls < nh2) ls = nh2;
@@ -1660,33 +1659,7 @@ int p3g_plan_create_tuned(p3g_plan* out, int nx, int ny, int nz, int nxc, int ny
     if (!size_tile(p->ax_z[3], nz, p->nxhpc, f64, strided_max_m)) p->z_ok[3] = false;
   }
   if (!p->z_ok[0] && !p->z_ok[1] && !p->z_ok[3]) return bad("z length " + std::to_string(nz) + " is too long");
-  auto size_x = [&] {  // r2c and c2r share the tile; c2r needs the larger buffer
-    size_pipe(p->ax_x, 1, f64);
-    AxisPlan c2r = p->ax_x;
-    size_pipe(c2r, 2, f64);
-    if (!c2r.pipe_ok || c2r.pipe_threads != p->ax_x.pipe_threads || c2r.pipe_m != p->ax_x.pipe_m)
-      p->ax_x.pipe_ok = false;
-    p->ax_x.buf_elems = c2r.buf_elems;
-    p->ax_x.pipe_smem = c2r.pipe_smem;
-    p->ax_x.pipe_nbuf = c2r.pipe_nbuf;
-  };
-  size_x();
-  if (!p->ax_x.pipe_ok && p->ax_x.spw_index >= 0) {
-    p->ax_x.spw_index = -1;
-    size_x();
-  }
-  // the X c2r pass: the same kernel shape, except on the F32 path, whose
-  // c2r pass runs the 16-point kernel (1024^3: 3.01 -> 2.80 ms; the r2c pass
-  // is faster with the radix-32 one, 2.56 against 2.72 ms)
-  p->ax_xc = p->ax_x;
-  if (!f64 && p->ax_xc.spw_index >= 0) {
-    // and in CTAs of at most 128 threads, six per SM, for power-of-two lines
-    // of 512 points or more (1024: 2.80 -> 2.69 ms; on 768-point lines the
-    // smaller CTAs were slower, 1.82 -> 1.88 ms)
-    p->ax_xc.spw_index = -1;
-    size_pipe(p->ax_xc, 2, f64, nx >= 512 && (nx & (nx - 1)) == 0 ? 128 : 0);
-    if (!p->ax_xc.pipe_ok) size_pipe(p->ax_xc, 2, f64);
-  }
+  size_x(p->ax_x, f64, p->xpairs(), x_max_m, p->sm_count);
   const int yx = p->nxhpc;
   const bool far_y = (long long)nz * p->pitch * p->esize() >= 3 << 20;  // the Y/Z workspace's row stride along y
   auto size_s = [&](AxisPlan& ap, int X, long long O1, bool tstore, bool far_rows) {
@@ -1705,15 +1678,6 @@ int p3g_plan_create_tuned(p3g_plan* out, int nx, int ny, int nz, int nxc, int ny
   }
   for (int i = 0; i < 4; ++i)
     if (p->z_ok[i]) size_s(p->ax_z[i], yx, nyc, !f64, false);
-  {
-    auto bps = [&](AxisPlan& ap) {
-      if (!ap.pipe_ok) return;
-      ap.pipe_bps = f64 ? pipe_blocks_per_sm<PathF64>(2, ap.pipe_e, ap.pipe_threads, ap.pipe_smem)
-                        : pipe_blocks_per_sm<PathF32>(2, ap.pipe_e, ap.pipe_threads, ap.pipe_smem);
-    };
-    bps(p->ax_x);
-    bps(p->ax_xc);
-  }
   {
     const char* e = std::getenv("P3G_NO_PIPE");
     p->use_pipe = !(e && *e && *e != '0');

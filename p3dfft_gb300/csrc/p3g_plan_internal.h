@@ -28,9 +28,7 @@ struct AxisPlan {
   int pipe_threads = 0;
   int buf_elems = 0;
   size_t pipe_smem = 0;
-  int pipe_bps = 1;  // resident CTAs per SM of the pipelined kernel
-  int pipe_e = 8;    // X passes: elements per thread of the pipelined kernel (PipeLimits)
-  StridedMode pipe_mode = kStridedGeneral;
+  TileMode pipe_mode = kTileGeneral;
   int pipe_nbuf = 2; // tile buffers of the pipelined kernel
   int pipe_g = 1;    // strided kernel: thread groups per CTA (pipe_threads over all of them)
   // F64 wide pipelined kernels (16 points per thread): a second stage plan
@@ -40,7 +38,7 @@ struct AxisPlan {
   int tw_lo_w = 0, tw_cnt_w = 0;
   int ls_w = 0, ps_w = 0;  // X axis: line-pair stride and padding of the wide tiles
   // the pipelined kernel's stage plan index, twiddle slice and X tile layout
-  int pipe_sp() const { return spw_index >= 0 ? spw_index : sp_index; }
+  unsigned long long pipe_fam() const { return spw_index >= 0 ? spw.fam : sp.fam; }
   int pipe_tw_lo() const { return spw_index >= 0 ? tw_lo_w : tw_lo; }
   int pipe_tw_cnt() const { return spw_index >= 0 ? tw_cnt_w : tw_cnt; }
   int pipe_ls() const { return spw_index >= 0 ? ls_w : ls; }
@@ -89,7 +87,6 @@ struct p3g_plan_s {
   int nxh, nxhp, nxhc, nxhpc, nycph, nzcph;
   long long pitch;
   AxisPlan ax_x, ax_y, ax_z[4];  // z: 0 fft, 1 dct (2(nz-1)), 2 dst (2(nz+1)), 3 none
-  AxisPlan ax_xc;                 // the X c2r pass's pipelined kernel (ax_x for the rest)
   bool z_ok[4];
   float4* d_tw = nullptr;
   StagePlan* d_sp = nullptr;

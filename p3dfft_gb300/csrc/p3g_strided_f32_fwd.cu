@@ -1,5 +1,5 @@
 // Strided Y/Z pass kernels, F32 path, forward sign.
-#include "p3g_strided_impl.cuh"
+#include "p3g_pipe_impl.cuh"
 
 namespace p3g {
 P3G_STRIDED_INSTANTIATE(PathF32, -1)

@@ -1,5 +1,5 @@
 // Strided Y/Z pass kernels, F64 path, backward sign.
-#include "p3g_strided_impl.cuh"
+#include "p3g_pipe_impl.cuh"
 
 namespace p3g {
 P3G_STRIDED_INSTANTIATE(PathF64, 1)

@@ -1,0 +1,6 @@
+// X c2r pass kernels, F64 path.
+#include "p3g_pipe_impl.cuh"
+
+namespace p3g {
+P3G_X_INSTANTIATE(PathF64, false)
+}  // namespace p3g
