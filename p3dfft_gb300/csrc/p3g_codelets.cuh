@@ -1,4 +1,4 @@
-// Register-resident DFT codelets of radix 2, 3, 4, 5, 8, 16 and 32.
+// Register-resident DFT codelets of radix 2 to 10, 12, 15, 16 and 32.
 //
 // DIR = -1 computes X_k = sum_n a_n exp(-2 pi i n k / R) (FFTW_FORWARD),
 // DIR = +1 the exp(+...) transform (FFTW_BACKWARD).  Inputs and outputs are in
@@ -20,6 +20,15 @@ namespace p3g {
 #define P3G_S5_1 0x1.e6f0e2p-1f, -0x1.97756p-26f
 #define P3G_S5_2 0x1.2cf23p-1f, 0x1.1d5698p-27f
 #define P3G_SQRT1_2 0x1.6a09e6p-1f, 0x1.9fcef4p-27f
+#define P3G_C7_1 0x1.3f3a0ep-1f, 0x1.45f6e8p-28f
+#define P3G_C7_2 -0x1.c7b90ep-3f, -0x1.8122c2p-30f
+#define P3G_C7_3 -0x1.cd4bcap-1f, -0x1.396b8ep-26f
+#define P3G_S7_1 0x1.904c38p-1f, -0x1.5f4436p-26f
+#define P3G_S7_2 0x1.f329cp-1f, 0x1.563a5ap-27f
+#define P3G_S7_3 0x1.bc4c04p-2f, 0x1.ae3578p-27f
+#define P3G_C9_1 0x1.8836fap-1f, 0x1.67a81cp-28f
+#define P3G_C9_2 0x1.63a1a8p-3f, -0x1.f48c76p-31f
+#define P3G_C9_4 -0x1.e11f64p-1f, -0x1.29168ep-28f
 #define P3G_C16_1 0x1.d906bcp-1f, 0x1.e651a8p-26f
 #define P3G_S16_1 0x1.87de2ap-2f, 0x1.abaa58p-28f
 
@@ -55,15 +64,60 @@ P3G_D void dft4(C* a) {
 template <int DIR, class C>
 P3G_D void dft5(C* a) {
   const C t1 = a[1] + a[4], t2 = a[2] + a[3], t3 = a[1] - a[4], t4 = a[2] - a[3];
-  const C b1 = a[0] + addmulr(mulr(t1, P3G_C5_1), t2, P3G_C5_2);
-  const C b2 = a[0] + addmulr(mulr(t1, P3G_C5_2), t2, P3G_C5_1);
-  const C d1 = rot<DIR>(addmulr(mulr(t3, P3G_S5_1), t4, P3G_S5_2));
-  const C d2 = rot<DIR>(addmulr(mulr(t3, P3G_S5_2), cneg(t4), P3G_S5_1));
+  const C b1 = a[0] + (mulr(t1, P3G_C5_1) + mulr(t2, P3G_C5_2));
+  const C b2 = a[0] + (mulr(t1, P3G_C5_2) + mulr(t2, P3G_C5_1));
+  const C d1 = rot<DIR>(mulr(t3, P3G_S5_1) + mulr(t4, P3G_S5_2));
+  const C d2 = rot<DIR>(mulr(t3, P3G_S5_2) - mulr(t4, P3G_S5_1));
   a[0] = a[0] + (t1 + t2);
   a[1] = b1 + d1;
   a[4] = b1 - d1;
   a[2] = b2 + d2;
   a[3] = b2 - d2;
+}
+
+// Outputs k and 7-k share the cosine sum r_k and the sine sum i_k of the input
+// pairs' sums and differences.
+template <int DIR, class C>
+P3G_D void dft7(C* a) {
+  const C s1 = a[1] + a[6], s2 = a[2] + a[5], s3 = a[3] + a[4];
+  const C d1 = a[1] - a[6], d2 = a[2] - a[5], d3 = a[3] - a[4];
+  const C r1 = a[0] + addmulr(addmulr(mulr(s1, P3G_C7_1), s2, P3G_C7_2), s3, P3G_C7_3);
+  const C r2 = a[0] + addmulr(addmulr(mulr(s1, P3G_C7_2), s2, P3G_C7_3), s3, P3G_C7_1);
+  const C r3 = a[0] + addmulr(addmulr(mulr(s1, P3G_C7_3), s2, P3G_C7_1), s3, P3G_C7_2);
+  const C i1 = rot<DIR>(addmulr(addmulr(mulr(d1, P3G_S7_1), d2, P3G_S7_2), d3, P3G_S7_3));
+  const C i2 = rot<DIR>(addmulr(addmulr(mulr(d1, P3G_S7_2), cneg(d2), P3G_S7_3), cneg(d3), P3G_S7_1));
+  const C i3 = rot<DIR>(addmulr(addmulr(mulr(d1, P3G_S7_3), cneg(d2), P3G_S7_1), d3, P3G_S7_2));
+  a[0] = a[0] + (s1 + (s2 + s3));
+  a[1] = r1 + i1;
+  a[6] = r1 - i1;
+  a[2] = r2 + i2;
+  a[5] = r2 - i2;
+  a[3] = r3 + i3;
+  a[4] = r3 - i3;
+}
+
+// 9 = 3 x 3: DFT3 over the inputs three apart, twiddles w9^(n1 k2), DFT3.
+template <int DIR, class C>
+P3G_D void dft9(C* a) {
+  constexpr float S = DIR > 0 ? 1.0f : -1.0f;
+  C b[3][3];
+#pragma unroll
+  for (int n1 = 0; n1 < 3; ++n1) {
+#pragma unroll
+    for (int n2 = 0; n2 < 3; ++n2) b[n1][n2] = a[n1 + 3 * n2];
+    dft3<DIR>(b[n1]);
+  }
+  b[1][1] = mulcc(b[1][1], P3G_C9_1, S * 0x1.491b76p-1f, S * -0x1.b87d3cp-26f);
+  b[1][2] = mulcc(b[1][2], P3G_C9_2, S * 0x1.f838b8p-1f, S * 0x1.902382p-26f);
+  b[2][1] = mulcc(b[2][1], P3G_C9_2, S * 0x1.f838b8p-1f, S * 0x1.902382p-26f);
+  b[2][2] = mulcc(b[2][2], P3G_C9_4, S * 0x1.5e3a88p-2f, S * -0x1.6ebe82p-27f);
+#pragma unroll
+  for (int k2 = 0; k2 < 3; ++k2) {
+    C t[3] = {b[0][k2], b[1][k2], b[2][k2]};
+    dft3<DIR>(t);
+#pragma unroll
+    for (int k1 = 0; k1 < 3; ++k1) a[k2 + 3 * k1] = t[k1];
+  }
 }
 
 // multiply by w8^1 = (1 + DIR i)/sqrt2 and w8^3 = (-1 + DIR i)/sqrt2
@@ -191,12 +245,53 @@ P3G_D void dft32(C* a) {
 }
 
 template <int R, int DIR, class C>
+P3G_D void dft(C* a);
+
+// x^-1 mod m for the prime factor maps
+P3G_HD constexpr int inv_mod(int x, int m) {
+  for (int i = 1; i < m; ++i)
+    if (x * i % m == 1) return i;
+  return 0;
+}
+
+// N1 N2 points, N1 and N2 coprime: with the input map n = N2 n1 + N1 n2 and
+// the output map k = N2 (N2^-1 mod N1) k1 + N1 (N1^-1 mod N2) k2 (all mod
+// N1 N2) the transform is a DFT of N1 points by a DFT of N2 points without
+// twiddles between them (Good's prime factor algorithm).
+template <int N1, int N2, int DIR, class C>
+P3G_D void dft_coprime(C* a) {
+  constexpr int N = N1 * N2, K1 = N2 * inv_mod(N2 % N1, N1), K2 = N1 * inv_mod(N1 % N2, N2);
+  C b[N1][N2];
+#pragma unroll
+  for (int n1 = 0; n1 < N1; ++n1) {
+#pragma unroll
+    for (int n2 = 0; n2 < N2; ++n2) b[n1][n2] = a[(N2 * n1 + N1 * n2) % N];
+    dft<N2, DIR>(b[n1]);
+  }
+#pragma unroll
+  for (int k2 = 0; k2 < N2; ++k2) {
+    C t[N1];
+#pragma unroll
+    for (int n1 = 0; n1 < N1; ++n1) t[n1] = b[n1][k2];
+    dft<N1, DIR>(t);
+#pragma unroll
+    for (int k1 = 0; k1 < N1; ++k1) a[(K1 * k1 + K2 * k2) % N] = t[k1];
+  }
+}
+
+template <int R, int DIR, class C>
 P3G_D void dft(C* a) {
   if constexpr (R == 2) dft2<DIR>(a);
   else if constexpr (R == 3) dft3<DIR>(a);
   else if constexpr (R == 4) dft4<DIR>(a);
   else if constexpr (R == 5) dft5<DIR>(a);
+  else if constexpr (R == 6) dft_coprime<2, 3, DIR>(a);
+  else if constexpr (R == 7) dft7<DIR>(a);
   else if constexpr (R == 8) dft8<DIR>(a);
+  else if constexpr (R == 9) dft9<DIR>(a);
+  else if constexpr (R == 10) dft_coprime<2, 5, DIR>(a);
+  else if constexpr (R == 12) dft_coprime<4, 3, DIR>(a);
+  else if constexpr (R == 15) dft_coprime<3, 5, DIR>(a);
   else if constexpr (R == 16) dft16<DIR>(a);
   else if constexpr (R == 32) dft32<DIR>(a);
 }

@@ -13,7 +13,7 @@
 // butterflies of the stage in registers (at most stage_butterflies, for which
 // the launch has enough threads).
 //
-// Radices 2, 3, 4, 5, 8, 16, 32 are register codelets.  Any other prime p runs a
+// Radices 2 to 10, 12, 15, 16 and 32 are register codelets.  Any other prime p runs a
 // generic direct-DFT stage through a second shared-memory buffer (O(N p) work).
 #pragma once
 
@@ -28,21 +28,23 @@ constexpr int kElemsPerThread = 16;  // E
 
 // The register codelets in the order their stages run: powers of two first,
 // so that the sub-transform length before any of them is a power of two.
-constexpr int kFamilies[] = {32, 16, 8, 4, 2, 3, 5};
+constexpr int kFamilies[] = {32, 16, 8, 4, 2, 12, 10, 15, 9, 6, 3, 5, 7};
 constexpr int kNumFamilies = sizeof(kFamilies) / sizeof(kFamilies[0]);
 P3G_HD int family_count(unsigned long long fam, int i) { return (int)(fam >> (4 * i)) & 15; }
 
 // Most butterflies of radix r that a thread of E elements runs per stage: as
 // many as cover E elements or, where the launch can have the threads for it
-// (the grouped kernels), as many as E elements hold.
+// (the grouped kernels), as many as E elements hold (with E = 16, two
+// butterflies of 9 points rather than one).
 P3G_HD constexpr int stage_butterflies(int E, int r, bool hold) {
-  return hold ? (E / r > 1 ? E / r : 1) : (E + r - 1) / r;
+  const int h = (E == 16 && r == 9 ? 18 : E) / r;
+  return hold ? (h > 1 ? h : 1) : (E + r - 1) / r;
 }
 
 struct StagePlan {
   int n;                   // transform length (1 allowed: no stages)
   int nstages;
-  int has_generic;         // a stage with a radix outside {2,3,4,5,8,16}
+  int has_generic;         // a stage with a radix outside kFamilies
   unsigned long long fam;  // stages of each radix family, 4 bits each in the order of kFamilies, then generic
   int radix[kMaxStages];
   int ns[kMaxStages];      // sub-transform length before the stage
@@ -464,8 +466,16 @@ __device__ __forceinline__ void run_families(const Tile<P, TH>& t, const float4*
   run_family<P, DIR, 4, E, LAY, FULL, RAW>(t, tw, N, family_count(fam, 3), ns, off);
   run_family<P, DIR, 2, E, LAY, FULL, RAW>(t, tw, N, family_count(fam, 4), ns, off);
   if constexpr (!FULL) {
-    run_family<P, DIR, 3, E, LAY, false, RAW>(t, tw, N, family_count(fam, 5), ns, off);
-    run_family<P, DIR, 5, E, LAY, false, RAW>(t, tw, N, family_count(fam, 6), ns, off);
+    if constexpr (MAXR >= 16 && TH::kHold) {
+      run_family<P, DIR, 12, E, LAY, false, RAW>(t, tw, N, family_count(fam, 5), ns, off);
+      run_family<P, DIR, 10, E, LAY, false, RAW>(t, tw, N, family_count(fam, 6), ns, off);
+      run_family<P, DIR, 15, E, LAY, false, RAW>(t, tw, N, family_count(fam, 7), ns, off);
+      run_family<P, DIR, 9, E, LAY, false, RAW>(t, tw, N, family_count(fam, 8), ns, off);
+    }
+    run_family<P, DIR, 6, E, LAY, false, RAW>(t, tw, N, family_count(fam, 9), ns, off);
+    run_family<P, DIR, 3, E, LAY, false, RAW>(t, tw, N, family_count(fam, 10), ns, off);
+    run_family<P, DIR, 5, E, LAY, false, RAW>(t, tw, N, family_count(fam, 11), ns, off);
+    run_family<P, DIR, 7, E, LAY, false, RAW>(t, tw, N, family_count(fam, 12), ns, off);
   }
 }
 

@@ -195,7 +195,11 @@ struct XPipeParams;
 // and more registers (binary32 only), kTileGeneral any plan, kTileSmall any
 // narrow plan with half the points per thread.
 enum TileMode { kTileGeneral = 0, kTileFull = 1, kTileFullWide = 2, kTileSmall = 3 };
-constexpr int tile_max_threads(int mode, bool x_pass = false) { return mode == kTileFullWide ? (x_pass ? 384 : 256) : 512; }
+// Threads per CTA: 512 with 128 registers each, or fewer where the binary32
+// kernels' 32 points per thread would spill.
+constexpr int tile_max_threads(int mode, bool f64, bool x_pass) {
+  return mode == kTileFullWide ? (x_pass ? 384 : 256) : (mode == kTileGeneral && !f64 ? 384 : 512);
+}
 template <class P, int DIR>
 cudaError_t launch_strided_pipe(const CUtensorMap* map, const CUtensorMap* omap, const SPipeParams& p,
                                 const float4* tw, TileMode mode, int threads, size_t smem, int grid,

@@ -378,7 +378,7 @@ P3G_D void strided_store(const SParams& s, const typename P::W* sm, int xt, int 
 // shared-memory exchanges and barriers; two or more groups drift apart and
 // fill each other's gaps.
 template <class P, int DIR, int MODE>
-__global__ void __launch_bounds__(tile_max_threads(MODE), 1)
+__global__ void __launch_bounds__(tile_max_threads(MODE, P::kF64, false), 1)
     k_strided_pipe(const __grid_constant__ CUtensorMap tin, const __grid_constant__ CUtensorMap tout,
                    const __grid_constant__ SPipeParams pp, const float4* __restrict__ tw_g) {
   const int nb = pp.c.nbuf, G = pp.c.groups;
@@ -760,7 +760,7 @@ P3G_D void xc2r_store(const XParams& x, const typename P::W* sm, int p0, int fie
 // stores busy at once.  The first FFT stage reads the raw line pairs (packing
 // or Hermitian merge and format conversion fused into it).
 template <class P, bool R2C, int MODE>
-__global__ void __launch_bounds__(tile_max_threads(MODE, true), 1)
+__global__ void __launch_bounds__(tile_max_threads(MODE, P::kF64, true), 1)
     k_x_pipe(const __grid_constant__ XPipeParams pp, const float4* __restrict__ tw_g) {
   const int nb = pp.c.nbuf, G = pp.c.groups;
   const int step = (int)gridDim.x;

@@ -12,6 +12,7 @@
 // replacing ftran.F90:489-780 / btran.F90:396-679, whose 1x1 path runs the
 // same FFTs with seg_copy/seg_zero passes (module.F90:502-706) in between.
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -59,14 +60,85 @@ cudaError_t opt_in_smem(const void* func, int bytes) {
   } while (0)
 
 // ------------------------------------------------------------ factorisation
-// Stage radices for length n, ordered by family (32, 16, 8, 4, 2, 3, 5,
-// other primes) as cta_fft expects.  Powers of two use the largest radix
-// allowed (max_pow2: 16, or 32 for the wide plans, on the F32 path; 8, or 16
-// for the wide plans, on F64; 4 or 2 when a tuner asks) with a smaller
-// remainder; with 32 the 2^a factor is
-// split into the fewest stages of at most 32, as evenly as possible
-// (1024 = 32 x 32, 512 = 32 x 16, 256 = 16 x 16, 128 = 16 x 8).
-static bool factor(int n, int max_pow2, std::vector<int>& radices) {
+// Cheapest split of 2^e[0] 3^e[1] 5^e[2] 7^e[3] into codelet radices, powers
+// of two of at most rmax and others of at most odd_max: the operations per point of a codelet (packed double-float ones;
+// the binary32 ratios are alike), of the twiddles before every stage but one,
+// and of a stage's shared-memory exchange.
+struct Split {
+  double cost = 1e300;
+  std::vector<int> radices;
+};
+static const Split& best_split(const std::array<int, 4>& e, int rmax, int odd_max, std::map<std::array<int, 4>, Split>& memo) {
+  const auto known = memo.find(e);
+  if (known != memo.end()) return known->second;
+  struct Codelet {
+    int r;
+    std::array<int, 4> e;
+    double ops;
+  };
+  static const Codelet codelets[] = {
+      {16, {4, 0, 0, 0}, 40}, {15, {0, 1, 1, 0}, 52}, {12, {2, 1, 0, 0}, 36}, {10, {1, 0, 1, 0}, 40},
+      {9, {0, 2, 0, 0}, 42},  {8, {3, 0, 0, 0}, 26},  {7, {0, 0, 0, 1}, 50},  {6, {1, 1, 0, 0}, 28},
+      {5, {0, 0, 1, 0}, 32},  {4, {2, 0, 0, 0}, 16},  {3, {0, 1, 0, 0}, 20},  {2, {1, 0, 0, 0}, 8},
+  };
+  Split best;
+  if (e == std::array<int, 4>{0, 0, 0, 0}) best.cost = 0;
+  for (const Codelet& c : codelets) {
+    if (c.r > ((c.r & (c.r - 1)) == 0 ? rmax : odd_max)) continue;
+    std::array<int, 4> rest = e;
+    bool ok = true;
+    for (int i = 0; i < 4; ++i) ok = ok && (rest[i] -= c.e[i]) >= 0;
+    if (!ok) continue;
+    const Split& sub = best_split(rest, rmax, odd_max, memo);
+    const double cost = sub.cost + c.ops + 30 + (sub.radices.empty() ? 0.0 : 16.0 * (1.0 - 1.0 / c.r));
+    if (cost < best.cost) {
+      best.cost = cost;
+      best.radices = sub.radices;
+      best.radices.push_back(c.r);
+    }
+  }
+  return memo[e] = best;
+}
+
+// Stage radices for length n in the order of kFamilies, other primes last.
+// Powers of two use the largest radix allowed (max_pow2: 16, or 32 for the
+// wide plans, on the F32 path; 8, or 16 for the wide plans, on F64; 4 or 2
+// when a tuner asks) with a smaller remainder; with 32 the 2^a factor is split
+// into the fewest stages of at most 32, as evenly as possible (1024 = 32 x 32,
+// 512 = 32 x 16, 256 = 16 x 16, 128 = 16 x 8).  Lengths with factors 3, 5 and
+// 7 take the cheapest split into codelets of at most 16 points (the narrow
+// plans: of at most 8 besides the powers of two).
+//
+// kSplitFixed: radices 3 and 5 after the powers of two and other primes as
+// generic stages.  The binary32 STRIDE1 plans keep it: their output goes into
+// the shell spectrum, whose binary64 sums callers compare far below binary32's
+// rounding, and another split rounds otherwise.
+enum SplitKind { kSplitNarrow = 0, kSplitWide = 1, kSplitFixed = 2 };
+static bool factor(int n, int max_pow2, SplitKind kind, std::vector<int>& radices) {
+  if (kind != kSplitFixed && n > 1 && (n & (n - 1)) != 0 && max_pow2 >= 8) {
+    std::array<int, 4> e{};
+    const int primes[4] = {2, 3, 5, 7};
+    int rest = n;
+    for (int i = 0; i < 4; ++i)
+      for (; rest % primes[i] == 0; rest /= primes[i]) ++e[i];
+    std::map<std::array<int, 4>, Split> memo;
+    const Split& s = best_split(e, std::min(max_pow2, 16), kind == kSplitWide ? 16 : 8, memo);
+    radices.clear();
+    for (int f : kFamilies)
+      for (int r : s.radices)
+        if (r == f) radices.push_back(r);
+    for (int p = 11; rest > 1; p += 2) {
+      while (rest % p == 0) {
+        radices.push_back(p);
+        rest /= p;
+      }
+      if ((long long)p * p > rest && rest > 1) {
+        radices.push_back(rest);
+        rest = 1;
+      }
+    }
+    return (int)radices.size() <= kMaxStages;
+  }
   radices.clear();
   int a = 0;
   while (n % 2 == 0) {
@@ -115,8 +187,8 @@ static bool factor(int n, int max_pow2, std::vector<int>& radices) {
   for (int r : {32, 16, 8, 4, 2})
     for (int x : pow2)
       if (x == r) radices.push_back(r);
-  for (int p : {3, 5}) {
-    while (n % p == 0) {
+  for (int p : {3, 5, 7}) {
+    while (n % p == 0 && !(p == 7 && kind == kSplitFixed)) {
       radices.push_back(p);
       n /= p;
     }
@@ -147,7 +219,7 @@ struct HostTw {
     StagePlan sp;
     int lo, cnt;
   };
-  std::map<std::pair<int, int>, Built> built;  // by (length, largest power-of-two radix)
+  std::map<std::pair<int, int>, Built> built;  // by length and kind of plan
 
   // exp(-2 pi i t / n) for 0 <= t < n, split into hi/lo
   static float4 root(long long t, long long n) {
@@ -191,8 +263,9 @@ struct HostTw {
   }
 };
 
-static bool build_stages(int n, int max_pow2, HostTw& tw, StagePlan& sp) {
-  const auto known = tw.built.find({n, max_pow2});
+static bool build_stages(int n, int max_pow2, SplitKind kind, HostTw& tw, StagePlan& sp) {
+  const int key = 4 * max_pow2 + (int)kind;
+  const auto known = tw.built.find({n, key});
   if (known != tw.built.end()) {
     sp = known->second.sp;
     tw.mark = known->second.lo;
@@ -203,7 +276,7 @@ static bool build_stages(int n, int max_pow2, HostTw& tw, StagePlan& sp) {
   tw.mark = (int)tw.v.size();
   sp.n = n;
   std::vector<int> rad;
-  if (n > 1 && !factor(n, max_pow2, rad)) return false;
+  if (n > 1 && !factor(n, max_pow2, kind, rad)) return false;
   sp.nstages = (int)rad.size();
   int ns = 1;
   for (int s = 0; s < sp.nstages; ++s) {
@@ -212,6 +285,7 @@ static bool build_stages(int n, int max_pow2, HostTw& tw, StagePlan& sp) {
     sp.ns[s] = ns;
     int fam = 0;
     while (fam < kNumFamilies && kFamilies[fam] != r) ++fam;
+    if (r == 7 && kind == kSplitFixed) fam = kNumFamilies;
     if (fam < kNumFamilies) sp.fam += 1ull << (4 * fam);
     else sp.has_generic = 1;
     sp.tw_off[s] = (int)tw.v.size();
@@ -227,7 +301,7 @@ static bool build_stages(int n, int max_pow2, HostTw& tw, StagePlan& sp) {
     ns *= r;
   }
   tw.count = (int)tw.v.size() - tw.mark;
-  tw.built[{n, max_pow2}] = HostTw::Built{sp, tw.mark, tw.count};
+  tw.built[{n, key}] = HostTw::Built{sp, tw.mark, tw.count};
   return true;
 }
 
@@ -291,18 +365,19 @@ static bool size_tile(AxisPlan& ap, int n, int lines_avail, bool f64, int max_m 
 // group of 256 threads, 5.3 ms with two).  The latency term matters when the
 // grid has fewer tiles than the GPU has groups: half the points per thread
 // halve the length of a thread's serial chain.
-static void size_strided(AxisPlan& ap, bool f64, int X, int O1, int max_m, int sm_count, bool tstore,
-                         bool far_rows) {
-  ap.pipe_ok = false;
-  if (ap.sp.nstages < 1 || ap.sp.has_generic || ap.n < 2) return;
+static TileShape size_strided(const AxisPlan& ap, long long nv) {
+  TileShape best_shape;
+  if (ap.sp.nstages < 1 || ap.sp.has_generic || ap.n < 2) return best_shape;
+  const bool f64 = ap.ext.f64, tstore = ap.ext.tstore, far_rows = ap.ext.far_rows;
+  const long long X = ap.ext.cols, O1 = ap.ext.rows * nv;
+  const int max_m = ap.ext.max_m, sm_count = ap.ext.sm_count;
   const size_t esize = f64 ? 16 : 8;
   const int Emax = f64 ? TileElems<PathF64>::value : TileElems<PathF32>::value;
   const int n = ap.n;
   const size_t room = 227 * 1024;
   const int wide_index = ap.spw_index;
-  int use_wide = wide_index;
   double best = 1e300;
-  for (int narrow = wide_index >= 0 ? 0 : 1; narrow < 2; ++narrow) {
+  for (int narrow = wide_index >= 0 ? 0 : 1; narrow < (ap.fixed_plan && wide_index >= 0 ? 1 : 2); ++narrow) {
     const StagePlan& sp = narrow ? ap.sp : ap.spw;
     bool pow2 = true;
     int rmax = 0;
@@ -312,7 +387,7 @@ static void size_strided(AxisPlan& ap, bool f64, int X, int O1, int max_m, int s
     }
     const size_t fixed = 1024 + (size_t)(narrow ? ap.tw_cnt : ap.tw_cnt_w) * 16 + 256;
     for (int E = Emax; E >= Emax / 2 && E >= rmax; E /= 2) {
-      for (int M = 1; M <= max_m && M <= (1 << ilog2(X)); M *= 2) {
+      for (int M = 1; M <= max_m && M < 2 * X; M *= 2) {
         const int tg = stage_threads(sp, M, E);
         const bool full = pow2 && (long long)M * n == (long long)tg * E && E == Emax;
         // binary32 FULL passes that store by threads run one group with twice
@@ -324,9 +399,9 @@ static void size_strided(AxisPlan& ap, bool f64, int X, int O1, int max_m, int s
         // with one; of 768 x 1024 x 540, 1.7 MB apart: 0.59 against 0.73 ms)
         const TileMode mode =
             E < Emax ? kTileSmall : (!full ? kTileGeneral : (!f64 && (tstore || far_rows) ? kTileFullWide : kTileFull));
-        const int max_threads = tile_max_threads(mode);
+        const int max_threads = tile_max_threads(mode, f64, false);
         const size_t buf = ((size_t)M * n * esize + 1023) / 1024 * 1024;
-        if (tg > tile_max_threads(kTileGeneral) || fixed + 2 * buf > room) break;
+        if (tg > 512 || fixed + 2 * buf > room) break;
         if (tg > max_threads) continue;
         const int fit = (int)std::min<size_t>((room - fixed) / buf, kMaxTileBuffers);
         const double tiles = (double)((X + M - 1) / M) * O1;
@@ -344,41 +419,49 @@ static void size_strided(AxisPlan& ap, bool f64, int X, int O1, int max_m, int s
         const double t = per_sm * tg * E * clocks / (rows * overlap) + 100.0 * E * sp.nstages / (f64 ? 1 : 2);
         if (t < best * 0.999) {
           best = t;
-          use_wide = narrow ? -1 : wide_index;
-          ap.pipe_ok = true;
-          ap.pipe_m = M;
-          ap.pipe_log2m = ilog2(M);
-          ap.pipe_mode = mode;
-          ap.pipe_g = g;
-          ap.pipe_threads = g * tg;
+          TileShape& o = best_shape;
+          o.ok = true;
+          o.wide = !narrow;
+          o.m = M;
+          o.log2m = ilog2(M);
+          o.mode = mode;
+          o.g = g;
+          o.threads = g * tg;
           // more loads in flight than one beyond the groups pay off only where
           // the tiles leave by TMA (binary32 512^3 Y: 0.19 ms with two, 0.26
           // with one; 540-point binary32 Z: 1.60 with two, 1.55 with one)
-          ap.pipe_nbuf = std::min(fit, g + (tstore ? 1 : 2));
-          ap.buf_elems = (int)(buf / esize);
-          ap.pipe_smem = fixed + ap.pipe_nbuf * buf;
+          o.nbuf = std::min(fit, g + (tstore ? 1 : 2));
+          o.buf_elems = (int)(buf / esize);
+          o.smem = fixed + o.nbuf * buf;
+          o.fam = sp.fam;
+          o.tw_lo = narrow ? ap.tw_lo : ap.tw_lo_w;
+          o.tw_cnt = narrow ? ap.tw_cnt : ap.tw_cnt_w;
+          o.ls = narrow ? ap.ls : ap.ls_w;
+          o.ps = narrow ? ap.ps : ap.ps_w;
         }
       }
     }
   }
-  if (ap.pipe_ok) ap.spw_index = use_wide;
+  return best_shape;
 }
 
 // X pass kernels (k_x_pipe): as size_strided; a tile is M line pairs of n
 // points (line stride ls in the padded layout) or their raw lines, whichever
 // takes more.  Lines are contiguous, so the smallest tile of two warps or more
 // is taken: up to eight groups per SM.
-static void size_x(AxisPlan& ap, bool f64, long long pairs, int max_m, int sm_count) {
-  ap.pipe_ok = false;
-  if (ap.sp.nstages < 1 || ap.sp.has_generic || ap.n < 2) return;
+static TileShape size_x(const AxisPlan& ap, long long nv) {
+  TileShape best_shape;
+  if (ap.sp.nstages < 1 || ap.sp.has_generic || ap.n < 2) return best_shape;
+  const bool f64 = ap.ext.f64;
+  const long long pairs = ap.ext.cols;
+  const int max_m = ap.ext.max_m, sm_count = ap.ext.sm_count;
   const size_t esize = f64 ? 16 : 8;
   const int Emax = f64 ? TileElems<PathF64>::value : TileElems<PathF32>::value;
   const int n = ap.n;
   const size_t room = 227 * 1024;
   const int wide_index = ap.spw_index;
-  int use_wide = wide_index;
   double best = 1e300;
-  for (int narrow = wide_index >= 0 ? 0 : 1; narrow < 2; ++narrow) {
+  for (int narrow = wide_index >= 0 ? 0 : 1; narrow < (ap.fixed_plan && wide_index >= 0 ? 1 : 2); ++narrow) {
     const StagePlan& sp = narrow ? ap.sp : ap.spw;
     bool pow2 = true;
     int rmax = 0;
@@ -395,12 +478,12 @@ static void size_x(AxisPlan& ap, bool f64, long long pairs, int max_m, int sm_co
         const bool full = pow2 && (long long)M * n == (long long)tg * E;
         const TileMode mode =
             E < Emax ? kTileSmall : (!full ? kTileGeneral : (f64 ? kTileFull : kTileFullWide));
-        const int max_threads = tile_max_threads(mode, true);
+        const int max_threads = tile_max_threads(mode, f64, true);
         const size_t buf = ((size_t)M * std::max(ls, raw) * esize + 1023) / 1024 * 1024;
-        if (tg > tile_max_threads(kTileGeneral) || fixed + 2 * buf > room) break;
+        if (tg > 512 || fixed + 2 * buf > room) break;
         if (tg > max_threads) continue;
         const int fit = (int)std::min<size_t>((room - fixed) / buf, kMaxTileBuffers);
-        const double per_sm = std::ceil((double)((pairs + M - 1) / M) / sm_count);
+        const double per_sm = std::ceil((double)((pairs + M - 1) / M) * nv / sm_count);
         const int g = (int)std::max(
             1.0, std::min({(double)(max_threads / tg), (double)kMaxGroups, (double)(fit - 1), per_sm}));
         if (E < Emax && per_sm > g) continue;  // every tile has a group of its own
@@ -410,21 +493,35 @@ static void size_x(AxisPlan& ap, bool f64, long long pairs, int max_m, int sm_co
         const double t = per_sm * tg * E * clocks / overlap + 100.0 * E * sp.nstages / (f64 ? 1 : 2);
         if (t < best * 0.999) {
           best = t;
-          use_wide = narrow ? -1 : wide_index;
-          ap.pipe_ok = true;
-          ap.pipe_m = M;
-          ap.pipe_log2m = ilog2(M);
-          ap.pipe_mode = mode;
-          ap.pipe_g = g;
-          ap.pipe_threads = g * tg;
-          ap.pipe_nbuf = std::min(fit, g + (g >= 4 ? 2 : 1));
-          ap.buf_elems = (int)(buf / esize);
-          ap.pipe_smem = fixed + ap.pipe_nbuf * buf;
+          TileShape& o = best_shape;
+          o.ok = true;
+          o.wide = !narrow;
+          o.m = M;
+          o.log2m = ilog2(M);
+          o.mode = mode;
+          o.g = g;
+          o.threads = g * tg;
+          o.nbuf = std::min(fit, g + (g >= 4 ? 2 : 1));
+          o.buf_elems = (int)(buf / esize);
+          o.smem = fixed + o.nbuf * buf;
+          o.fam = sp.fam;
+          o.tw_lo = narrow ? ap.tw_lo : ap.tw_lo_w;
+          o.tw_cnt = narrow ? ap.tw_cnt : ap.tw_cnt_w;
+          o.ls = narrow ? ap.ls : ap.ls_w;
+          o.ps = narrow ? ap.ps : ap.ps_w;
         }
       }
     }
   }
-  if (ap.pipe_ok) ap.spw_index = use_wide;
+  return best_shape;
+}
+
+// The axis's tile shape for calls with nv fields (under the plan's lock).
+static const TileShape& tile_shape(AxisPlan& ap, int nv) {
+  const auto known = ap.shapes.find(nv);
+  if (known != ap.shapes.end()) return known->second;
+  if (ap.shapes.size() >= 64) ap.shapes.clear();
+  return ap.shapes[nv] = ap.ext.x_pass ? size_x(ap, nv) : size_strided(ap, nv);
 }
 
 }  // namespace p3g
@@ -595,7 +692,7 @@ bool device_memory(const void* ptr) {
 }
 
 template <class P>
-int run_strided(p3g_plan p, SParams& s, const AxisPlan& ap, bool fwd_sign, int nv, cudaStream_t st,
+int run_strided(p3g_plan p, SParams& s, AxisPlan& ap, bool fwd_sign, int nv, cudaStream_t st,
                 int max_sms = 0) {
   s.M = ap.M;
   s.log2m = ap.log2m;
@@ -603,8 +700,9 @@ int run_strided(p3g_plan p, SParams& s, const AxisPlan& ap, bool fwd_sign, int n
   s.xtiles = (s.X + ap.M - 1) / ap.M;
   const int esize = (int)sizeof(typename P::W);
   if (p->use_pipe && ap.pipe_ok && aligned_to(s.in, esize)) {
-    s.M = ap.pipe_m;
-    s.log2m = ap.pipe_log2m;
+    const TileShape& ts = tile_shape(ap, nv);
+    s.M = ts.m;
+    s.log2m = ts.log2m;
     s.xtiles = (s.X + s.M - 1) / s.M;
     SPipeParams pp{};
     pp.s = s;
@@ -630,13 +728,13 @@ int run_strided(p3g_plan p, SParams& s, const AxisPlan& ap, bool fwd_sign, int n
     }
     pp.c.tiles_per_field = pp.s.xtiles * pp.s.O1;
     pp.c.ntiles = pp.c.tiles_per_field * nv;
-    pp.c.tw_base = ap.pipe_tw_lo();
-    pp.c.tw_count = ap.pipe_tw_cnt();
-    pp.c.fam = ap.pipe_fam();
-    pp.c.buf_elems = ap.buf_elems;
-    pp.c.nbuf = ap.pipe_nbuf;
-    pp.c.groups = ap.pipe_g;
-    pp.c.gthreads = ap.pipe_threads / ap.pipe_g;
+    pp.c.tw_base = ts.tw_lo;
+    pp.c.tw_count = ts.tw_cnt;
+    pp.c.fam = ts.fam;
+    pp.c.buf_elems = ts.buf_elems;
+    pp.c.nbuf = ts.nbuf;
+    pp.c.groups = ts.g;
+    pp.c.gthreads = ts.threads / ts.g;
     pp.c.err = p->d_err;
     pp.chunk = esize;
     CUtensorMap map, omap;
@@ -674,8 +772,7 @@ int run_strided(p3g_plan p, SParams& s, const AxisPlan& ap, bool fwd_sign, int n
     const int slots = max_sms > 0 && max_sms < p->sm_count ? max_sms : p->sm_count;
     const int grid = pp.c.ntiles < slots ? pp.c.ntiles : slots;
     const auto launch = fwd_sign ? launch_strided_pipe<P, -1> : launch_strided_pipe<P, 1>;
-    cudaError_t e = launch(&map, &omap, pp, p->d_tw, ap.pipe_mode, ap.pipe_threads,
-                           ap.pipe_smem, grid, st);
+    cudaError_t e = launch(&map, &omap, pp, p->d_tw, ts.mode, ts.threads, ts.smem, grid, st);
     if (e != cudaSuccess) return fail(P3G_E_CUDA, std::string("strided pass launch: ") + cudaGetErrorString(e));
     p->launches++;
     return P3G_OK;
@@ -688,38 +785,38 @@ int run_strided(p3g_plan p, SParams& s, const AxisPlan& ap, bool fwd_sign, int n
 
 template <class P>
 int run_x_r2c(p3g_plan p, XParams& x, int nv, cudaStream_t st, int max_sms = 0) {
-  const AxisPlan& ap = p->ax_x;
+  AxisPlan& ap = p->ax_x;
   using UR = typename P::UR;
   if (p->use_pipe && ap.pipe_ok) {
     const long long us = sizeof(UR);
     int chunk = (int)us;
     if ((x.nx * us) % 16 == 0 && (x.in_field * us) % 16 == 0 && aligned_to(x.in, 16)) chunk = 16;
     else if ((x.nx * us) % 8 == 0 && (x.in_field * us) % 8 == 0 && aligned_to(x.in, 8)) chunk = 8;
-    x.M = ap.pipe_m;
-    x.log2m = ap.pipe_log2m;
-    x.LS = ap.pipe_ls();
-    x.ps = ap.pipe_ps();
+    const TileShape& ts = tile_shape(ap, nv);
+    x.M = ts.m;
+    x.log2m = ts.log2m;
+    x.LS = ts.ls;
+    x.ps = ts.ps;
     x.tiles = ((x.nlines + 1) / 2 + x.M - 1) / x.M;
     XPipeParams xp{};
     xp.x = x;
     xp.chunk = chunk;
     xp.c.tiles_per_field = x.tiles;
     xp.c.ntiles = x.tiles * nv;
-    xp.c.tw_base = ap.pipe_tw_lo();
-    xp.c.tw_count = ap.pipe_tw_cnt();
-    xp.c.fam = ap.pipe_fam();
-    xp.c.buf_elems = ap.buf_elems;
-    xp.c.nbuf = ap.pipe_nbuf;
-    xp.c.groups = ap.pipe_g;
-    xp.c.gthreads = ap.pipe_threads / ap.pipe_g;
+    xp.c.tw_base = ts.tw_lo;
+    xp.c.tw_count = ts.tw_cnt;
+    xp.c.fam = ts.fam;
+    xp.c.buf_elems = ts.buf_elems;
+    xp.c.nbuf = ts.nbuf;
+    xp.c.groups = ts.g;
+    xp.c.gthreads = ts.threads / ts.g;
     xp.c.err = p->d_err;
     // the tile's 2M real lines are one contiguous run of device memory
     xp.bulk = x.in_line == x.nx && (x.nx * us) % 16 == 0 && (x.in_field * us) % 16 == 0 && aligned_to(x.in, 16) &&
               device_memory(x.in);
     const int slots = max_sms > 0 && max_sms < p->sm_count ? max_sms : p->sm_count;
     const int grid = xp.c.ntiles < slots ? xp.c.ntiles : slots;
-    cudaError_t e = launch_x_pipe<P, true>(xp, p->d_tw, ap.pipe_mode, ap.pipe_threads,
-                                            ap.pipe_smem, grid, st);
+    cudaError_t e = launch_x_pipe<P, true>(xp, p->d_tw, ts.mode, ts.threads, ts.smem, grid, st);
     if (e != cudaSuccess) return fail(P3G_E_CUDA, std::string("X r2c launch: ") + cudaGetErrorString(e));
     p->launches++;
     return P3G_OK;
@@ -732,25 +829,26 @@ int run_x_r2c(p3g_plan p, XParams& x, int nv, cudaStream_t st, int max_sms = 0) 
 
 template <class P>
 int run_x_c2r(p3g_plan p, XParams& x, int nv, cudaStream_t st, int max_sms = 0) {
-  const AxisPlan& ap = p->ax_x;
+  AxisPlan& ap = p->ax_x;
   if (p->use_pipe && ap.pipe_ok) {
-    x.M = ap.pipe_m;
-    x.log2m = ap.pipe_log2m;
-    x.LS = ap.pipe_ls();
-    x.ps = ap.pipe_ps();
+    const TileShape& ts = tile_shape(ap, nv);
+    x.M = ts.m;
+    x.log2m = ts.log2m;
+    x.LS = ts.ls;
+    x.ps = ts.ps;
     x.tiles = ((x.nlines + 1) / 2 + x.M - 1) / x.M;
     XPipeParams xp{};
     xp.x = x;
     xp.chunk = (int)sizeof(typename P::W);
     xp.c.tiles_per_field = x.tiles;
     xp.c.ntiles = x.tiles * nv;
-    xp.c.tw_base = ap.pipe_tw_lo();
-    xp.c.tw_count = ap.pipe_tw_cnt();
-    xp.c.fam = ap.pipe_fam();
-    xp.c.buf_elems = ap.buf_elems;
-    xp.c.nbuf = ap.pipe_nbuf;
-    xp.c.groups = ap.pipe_g;
-    xp.c.gthreads = ap.pipe_threads / ap.pipe_g;
+    xp.c.tw_base = ts.tw_lo;
+    xp.c.tw_count = ts.tw_cnt;
+    xp.c.fam = ts.fam;
+    xp.c.buf_elems = ts.buf_elems;
+    xp.c.nbuf = ts.nbuf;
+    xp.c.groups = ts.g;
+    xp.c.gthreads = ts.threads / ts.g;
     xp.c.err = p->d_err;
     {
       // the modes of a line arrive by one bulk copy, rounded up to 16 bytes,
@@ -762,8 +860,7 @@ int run_x_c2r(p3g_plan p, XParams& x, int nv, cudaStream_t st, int max_sms = 0) 
     }
     const int slots = max_sms > 0 && max_sms < p->sm_count ? max_sms : p->sm_count;
     const int grid = xp.c.ntiles < slots ? xp.c.ntiles : slots;
-    cudaError_t e = launch_x_pipe<P, false>(xp, p->d_tw, ap.pipe_mode, ap.pipe_threads,
-                                            ap.pipe_smem, grid, st);
+    cudaError_t e = launch_x_pipe<P, false>(xp, p->d_tw, ts.mode, ts.threads, ts.smem, grid, st);
     if (e != cudaSuccess) return fail(P3G_E_CUDA, std::string("X c2r launch: ") + cudaGetErrorString(e));
     p->launches++;
     return P3G_OK;
@@ -1554,29 +1651,32 @@ int p3g_plan_create_tuned(p3g_plan* out, int nx, int ny, int nz, int nxc, int ny
     if (f64) return 8;
     return (n & (n - 1)) == 0 ? 32 : 16;
   };
-  // Every axis has a stage plan of radices up to 8 (F64) or 16 (F32) for the
-  // kernels that run 8 or 16 points per thread (and the single-tile and batch
-  // kernels); power-of-two lines add a wide plan for the wide pipelined
-  // kernels: radix 32 on F32 (every axis), radix 16 on F64, where it pays off
-  // on the Y pass only (1024 points: 8.2 -> 7.8 ms at 1024^3; the X passes'
-  // 128-thread CTAs and the Z passes' user-format stores ran slower with it)
-  auto wide_ok = [&](const AxisPlan& ap, int n) {
+  // Every axis has a narrow stage plan (radices up to 8 on F64, 16 on F32) for
+  // the single-tile and batch kernels and for few tiles, and, unless a tuner
+  // caps the radix, a wide one for the grouped kernels: up to 16 on F64, 32
+  // for powers of two on F32.
+  const bool fixed_split = !f64 && layout == P3G_LAYOUT_STRIDE1;
+  auto wide_ok = [&](const AxisPlan&, int n) {
+    if (fixed_split && (n & (n - 1)) != 0) return false;
     if (f64) return max_radix == 0 || max_radix >= 16;
-    if ((n & (n - 1)) != 0) return false;
-    return max_radix == 0 || max_radix >= 32;
+    return max_radix == 0 || max_radix >= ((n & (n - 1)) == 0 ? 32 : 16);
   };
   auto add_axis = [&](AxisPlan& ap, int n, int lines) -> bool {
-    if (!build_stages(n, std::min(axis_pow2(n), f64 ? 8 : 16), tw, ap.sp)) return false;
+    ap.fixed_plan = fixed_split;
+    if (!build_stages(n, std::min(axis_pow2(n), f64 ? 8 : 16), fixed_split ? kSplitFixed : kSplitNarrow, tw, ap.sp)) return false;
     ap.tw_lo = tw.mark;
     ap.tw_cnt = tw.count;
     if (!size_tile(ap, n, lines, f64, &ap == &p->ax_x ? x_max_m : strided_max_m)) return false;
     ap.sp_index = (int)sps.size();
     sps.push_back(ap.sp);
     // the wide plan (1024 = 16 x 16 x 4 against 8 x 8 x 4 x 4 on F64, 32 x 32
-    // against 16 x 16 x 4 on F32), kept when it has a wide stage
+    // against 16 x 16 x 4 on F32; 540 = 12 x 9 x 5 against 6 x 6 x 5 x 3),
+    // where it is another
     if (wide_ok(ap, n)) {
       StagePlan w;
-      if (build_stages(n, f64 ? 16 : 32, tw, w) && family_count(w.fam, f64 ? 1 : 0) > 0) {
+
+      if (build_stages(n, f64 ? 16 : 32, kSplitWide, tw, w) && w.fam != ap.sp.fam &&
+          (f64 || (n & (n - 1)) != 0 || family_count(w.fam, 0) > 0)) {
         ap.spw = w;
         ap.tw_lo_w = tw.mark;
         ap.tw_cnt_w = tw.count;
@@ -1659,22 +1759,18 @@ int p3g_plan_create_tuned(p3g_plan* out, int nx, int ny, int nz, int nxc, int ny
     if (!size_tile(p->ax_z[3], nz, p->nxhpc, f64, strided_max_m)) p->z_ok[3] = false;
   }
   if (!p->z_ok[0] && !p->z_ok[1] && !p->z_ok[3]) return bad("z length " + std::to_string(nz) + " is too long");
-  size_x(p->ax_x, f64, p->xpairs(), x_max_m, p->sm_count);
+  p->ax_x.ext = TileExtents{true, f64, false, false, p->xpairs(), 1, x_max_m, p->sm_count};
+  p->ax_x.pipe_ok = tile_shape(p->ax_x, 1).ok;
   const int yx = p->nxhpc;
   const bool far_y = (long long)nz * p->pitch * p->esize() >= 3 << 20;  // the Y/Z workspace's row stride along y
   auto size_s = [&](AxisPlan& ap, int X, long long O1, bool tstore, bool far_rows) {
-    size_strided(ap, f64, X, (int)std::min<long long>(O1, 1 << 30), strided_max_m, p->sm_count, tstore,
-                 far_rows);
-    if (!ap.pipe_ok && ap.spw_index >= 0) {
-      ap.spw_index = -1;
-      size_strided(ap, f64, X, (int)std::min<long long>(O1, 1 << 30), strided_max_m, p->sm_count, tstore,
-                 far_rows);
-    }
+    ap.ext = TileExtents{false, f64, tstore, far_rows, X, O1, strided_max_m, p->sm_count};
+    ap.pipe_ok = tile_shape(ap, 1).ok;
   };
   size_s(p->ax_y, yx, nz, false, far_y);
   for (int i = 0; i < 2; ++i) {
-    if (p->four_y) size_s(p->ly[i], yx, (long long)nz * p->ly[1 - i].n, false, far_y);
-    if (p->four_z) size_s(p->lz[i], yx, (long long)nyc * p->lz[1 - i].n, !f64, false);
+    if (p->four_y) size_s(p->ly[i], yx, p->ly[1 - i].n, false, far_y);
+    if (p->four_z) size_s(p->lz[i], yx, p->lz[1 - i].n, !f64, false);
   }
   for (int i = 0; i < 4; ++i)
     if (p->z_ok[i]) size_s(p->ax_z[i], yx, nyc, !f64, false);

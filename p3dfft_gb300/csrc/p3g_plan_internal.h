@@ -2,6 +2,7 @@
 // units of libp3dfft_gb300.so (not part of the public headers).
 #pragma once
 
+#include <map>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -14,6 +15,25 @@ namespace p3g {
 // Records msg as the calling thread's p3g_last_error() and returns code.
 int fail(int code, const std::string& msg);
 
+// A pipelined kernel's tiles and launch: tiles of m lines (columns), g groups
+// over `threads` threads, a ring of nbuf buffers; wide: the stage plan spw.
+struct TileShape {
+  bool ok = false, wide = false;
+  int m = 1, log2m = 0, g = 1, threads = 32, nbuf = 2, buf_elems = 0;
+  TileMode mode = kTileGeneral;
+  size_t smem = 0;
+  unsigned long long fam = 0;  // the plan's stages, its twiddle slice and X tile layout
+  int tw_lo = 0, tw_cnt = 0, ls = 0, ps = 0;
+};
+
+// What a pass's tiles cover per field: cols columns (X passes: line pairs) of
+// rows row sets.
+struct TileExtents {
+  bool x_pass = false, f64 = false, tstore = false, far_rows = false;
+  long long cols = 1, rows = 1;
+  int max_m = 1, sm_count = 1;
+};
+
 struct AxisPlan {
   StagePlan sp{};
   int n = 0;
@@ -22,27 +42,18 @@ struct AxisPlan {
   int sp_index = 0;  // index into the device StagePlan array
   int tw_lo = 0, tw_cnt = 0;  // this axis's contiguous slice of the twiddle table
   int ls = 0, ps = 0;         // X axis: shared-memory line-pair stride and padding shift
-  // pipelined kernels (p3g_pipe.cuh): same tile, double buffered
+  // pipelined kernels (p3g_pipe.cuh): the pass's extents, and the tile shape
+  // for each number of fields that a call has asked for
   bool pipe_ok = false;
-  int pipe_m = 1, pipe_log2m = 0;  // lines (columns) per pipelined tile
-  int pipe_threads = 0;
-  int buf_elems = 0;
-  size_t pipe_smem = 0;
-  TileMode pipe_mode = kTileGeneral;
-  int pipe_nbuf = 2; // tile buffers of the pipelined kernel
-  int pipe_g = 1;    // strided kernel: thread groups per CTA (pipe_threads over all of them)
+  TileExtents ext;
+  std::map<int, TileShape> shapes;
   // F64 wide pipelined kernels (16 points per thread): a second stage plan
   // with radix-16 stages and its twiddle slice; every other kernel runs sp
   StagePlan spw{};
-  int spw_index = -1;  // -1: none, the pipelined kernel runs sp
+  int spw_index = -1;  // -1: none, the pipelined kernels run sp
+  bool fixed_plan = false;  // kSplitFixed: no choice between spw and sp
   int tw_lo_w = 0, tw_cnt_w = 0;
   int ls_w = 0, ps_w = 0;  // X axis: line-pair stride and padding of the wide tiles
-  // the pipelined kernel's stage plan index, twiddle slice and X tile layout
-  unsigned long long pipe_fam() const { return spw_index >= 0 ? spw.fam : sp.fam; }
-  int pipe_tw_lo() const { return spw_index >= 0 ? tw_lo_w : tw_lo; }
-  int pipe_tw_cnt() const { return spw_index >= 0 ? tw_cnt_w : tw_cnt; }
-  int pipe_ls() const { return spw_index >= 0 ? ls_w : ls; }
-  int pipe_ps() const { return spw_index >= 0 ? ps_w : ps; }
 };
 
 struct TimerRec {

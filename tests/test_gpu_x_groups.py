@@ -78,3 +78,31 @@ def test_x_long_conversion_values(precision):
         assert orc.normalised_linf(got, want) <= 1e-12
     else:
         assert orc.relative_l2(got, want) <= 1e-6
+
+
+@pytest.mark.parametrize("precision", ["f64", "f32"])
+@pytest.mark.parametrize("shape", [(64, 31, 41), (128, 150, 67, 86, 100, 44)], ids=lambda s: "x".join(map(str, s)))
+def test_many_fields_with_partial_last_tile(shape, precision):
+    """nv fields whose line count leaves each field's last tile partial: the
+    tiles after it, of the next field, must not be affected."""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import p3dfft_gb300 as pg
+    nx, ny, nz = shape[:3]
+    pruned = shape[3:] or (nx, ny, nz)
+    f64 = precision == "f64"
+    plan = pg.Plan(nx, ny, nz, *pruned, precision=pg.F64 if f64 else pg.F32)
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(3)
+    x = torch.rand((5, nz, ny, nx), dtype=torch.float64 if f64 else torch.float32, device="cuda", generator=gen)
+    b = plan.ftran_r2c(x, nv=5)
+    r = plan.btran_c2r(b, nv=5)
+    plan.check()
+    for i in range(5):
+        bi = plan.ftran_r2c(x[i].contiguous())
+        ri = plan.btran_c2r(bi)
+        assert torch.equal(b[i], bi)
+        assert torch.equal(r[i], ri)
+    plan.check()
+    plan.close()
