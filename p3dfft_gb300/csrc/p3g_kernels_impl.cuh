@@ -223,43 +223,59 @@ __global__ void __launch_bounds__(PathLimits<P>::kMaxThreads, PathLimits<P>::kMi
 }
 
 // ------------------------------------------------------------- Chebyshev
-// out(k) = L k old + out(k+2), ftran.F90:412-451, one thread per (x, y)
-// pencil.  The F64 path runs this recurrence in binary64 itself (a few
-// multiply-adds per mode on a pass bound by its 2 x 16 bytes per mode), so
-// it has binary64's range and rounding like the reference; the F32 path in
-// binary32.
+// out(k) = L k old + out(k+2), ftran.F90:412-451.  The F64 path runs this
+// recurrence in binary64 itself, so it has binary64's range and rounding like
+// the reference; the F32 path in binary32.
+//
+// One thread per real component of an (x, y) pencil: a chain of one multiply-
+// add per mode, bound by the binary64 rate (about 1/70 of binary32's) where it
+// does more than that.  The factors L (k+1) / (nx ny (nz-1)) come from a table
+// the CTA makes once (a conversion and two multiplies per mode and component
+// before: 512x512x257, 0.97 -> 0.36 ms), and the loads run a block of modes
+// ahead of the chain.
+constexpr int kChebyThreads = 128;
+constexpr int kChebyAhead = 8;
+
 template <class P>
-__global__ void k_cheby(const ChebyParams prm) {
-  using UC = typename P::UC;
-  using R = typename std::conditional<P::kF64, double, float>::type;
-  const int pcl = blockIdx.x * blockDim.x + threadIdx.x;
-  if (pcl >= prm.npencil) return;
-  UC* d = static_cast<UC*>(prm.data) + blockIdx.y * prm.field + pcl * prm.pstride;
+__global__ void __launch_bounds__(kChebyThreads) k_cheby(const ChebyParams prm) {
+  using R = typename P::UR;
+  extern __shared__ double p3g_cheby_f[];
+  R* f = reinterpret_cast<R*>(p3g_cheby_f);
   const int n = prm.nzc;
-  const long long zs = prm.zstride;
   const R sc = (R)prm.sc, lf = (R)prm.lfac;
-  auto scaled = [&](int k) {
-    const UC v = d[k * zs];
-    return UC{(R)v.x * sc, (R)v.y * sc};
-  };
-  UC old = scaled(n - 2);
-  const UC top = scaled(n - 1);
-  const R f1 = lf * (R)(n - 1) * (R)0.5;
-  UC o1{f1 * top.x, f1 * top.y};  // out(nzc-1)
-  UC o2{(R)0, (R)0};               // out(nzc)
-  d[(n - 2) * zs] = o1;
+  for (int k = threadIdx.x; k < n; k += kChebyThreads) f[k] = lf * (R)(k + 1) * sc;
+  __syncthreads();
+  const long long e = (long long)blockIdx.x * kChebyThreads + threadIdx.x;
+  if (e >= 2LL * prm.npencil) return;
+  R* d = static_cast<R*>(prm.data) + 2 * (blockIdx.y * prm.field + (e >> 1) * prm.pstride) + (e & 1);
+  const long long zs = 2 * prm.zstride;
+  R old = d[(n - 2) * zs];
+  R o1 = f[n - 2] * (R)0.5 * d[(n - 1) * zs];  // out(nzc-1)
+  R o2 = (R)0;                                 // out(nzc)
+  d[(n - 2) * zs] = n == 2 ? o1 * (R)0.5 : o1;
   d[(n - 1) * zs] = o2;
-  for (int k = n - 3; k >= 0; --k) {
-    const UC nw = scaled(k);
-    const R f = lf * (R)(k + 1);
-    const UC val{f * old.x + o2.x, f * old.y + o2.y};
-    d[k * zs] = val;
-    o2 = o1;
-    o1 = val;
-    old = nw;
+  R cur[kChebyAhead], nxt[kChebyAhead];
+#pragma unroll
+  for (int u = 0; u < kChebyAhead; ++u) cur[u] = n - 3 - u >= 0 ? d[(n - 3 - u) * zs] : (R)0;
+  for (int k0 = n - 3; k0 >= 0; k0 -= kChebyAhead) {
+#pragma unroll
+    for (int u = 0; u < kChebyAhead; ++u) {
+      const int k = k0 - kChebyAhead - u;
+      nxt[u] = k >= 0 ? d[k * zs] : (R)0;
+    }
+#pragma unroll
+    for (int u = 0; u < kChebyAhead; ++u) {
+      const int k = k0 - u;
+      if (k < 0) break;
+      const R val = f[k] * old + o2;
+      d[k * zs] = k == 0 ? val * (R)0.5 : val;
+      o2 = o1;
+      o1 = val;
+      old = cur[u];
+    }
+#pragma unroll
+    for (int u = 0; u < kChebyAhead; ++u) cur[u] = nxt[u];
   }
-  const UC v0 = d[0];
-  d[0] = UC{v0.x * (R)0.5, v0.y * (R)0.5};
 }
 
 // ------------------------------------------------- long X lines (four-step)
@@ -409,8 +425,8 @@ cudaError_t launch_strided(const SParams& p, const StagePlan* sp, const float4* 
 }
 template <class P>
 cudaError_t launch_cheby(const ChebyParams& p, int nfields, cudaStream_t st) {
-  const int threads = 128;
-  k_cheby<P><<<dim3((p.npencil + threads - 1) / threads, nfields), threads, 0, st>>>(p);
+  const long long blocks = (2LL * p.npencil + kChebyThreads - 1) / kChebyThreads;
+  k_cheby<P><<<dim3((unsigned)blocks, nfields), kChebyThreads, (size_t)p.nzc * sizeof(typename P::UR), st>>>(p);
   return cudaGetLastError();
 }
 
