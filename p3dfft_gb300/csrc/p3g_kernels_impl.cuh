@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(PathLimits<P>::kMaxThreads, PathLimits<P>::kMi
 // add per mode, bound by the binary64 rate (about 1/70 of binary32's) where it
 // does more than that.  The factors L (k+1) / (nx ny (nz-1)) come from a table
 // the CTA makes once (a conversion and two multiplies per mode and component
-// before: 512x512x257, 0.97 -> 0.36 ms), and the loads run a block of modes
+// before: 512x512x257, 0.97 -> 0.27 ms), and the loads run a block of modes
 // ahead of the chain.
 constexpr int kChebyThreads = 128;
 constexpr int kChebyAhead = 8;

@@ -8,17 +8,14 @@
 // The serving form's power spectrum uses the same binning with unit weight
 // and counts the conjugate partner of every mode with 0 < kx and 2 kx != nx.
 //
-// Arithmetic: each warp takes one row of the fast axis (x, or z in the
-// STRIDE1 layout) 32 modes at a time.  The mode weight w = k^2 |B|^2 is formed
+// Arithmetic: each warp takes one row of the fast axis (x, or z in the STRIDE1
+// layout), each lane a run of its modes.  The mode weight w = k^2 |B|^2 is formed
 // in double-float (binary32 pairs with FMA-exact products; GB300 runs binary64
-// FMA at about 1/70 of the binary32 rate), equal bins among the 32 lanes are
-// contiguous (|k| is monotone along x, and monotone on each side of the fold
-// along z), so a segmented shuffle reduction gives one partial sum per run of
-// equal bins; the run head converts its sum to binary64 and adds it to the
-// warp's private binary64 histogram in shared memory.  At the end the CTA sums
-// its warps' histograms and adds them to E with binary64 atomics.  Summation
-// order differs from the sample's sequential loop, so results agree to
-// rounding, not bitwise.
+// FMA at about 1/70 of the binary32 rate), runs of equal bins are added up in
+// double-float, and each run's sum goes in binary64 to the warp's private
+// histogram in shared memory.  At the end the CTA sums its warps' histograms
+// and adds them to E with binary64 atomics.  Summation order differs from the
+// sample's sequential loop, so results agree to rounding, not bitwise.
 #include <cuda_runtime.h>
 
 #include <cmath>
