@@ -80,8 +80,16 @@ struct RingSmem {
   float4* tw;
   uint64_t* mbar;  // one per buffer: its load has landed
   int* issued;     // loads issued into each buffer so far
-  int* cta;        // [0] failure flag; X passes: [1] exponent bias, [2] largest |high word| seen
+  int* cta;        // [0] failure flag, [1] exponent bias, [2] largest |high word| seen
 };
+// Start of a pass kernel: lets the next pass's CTAs launch (they fit beside
+// this one's on grids that leave SMs or shared memory free) and, after the
+// part that only reads the plan's own tables, waits for the kernel before this
+// one in the stream to complete (launch_pass; 32^3 FP64 forward 24.6 us per
+// call without, 21.4 us with; 128^3 round trip 120 and 108 us).
+P3G_D void pass_launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+P3G_D void pass_begin() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 template <class P>
 P3G_D RingSmem<P> ring_smem(const PipeCommon& pc) {
   extern __shared__ unsigned char p3g_pipe_smem[];
@@ -381,6 +389,7 @@ template <class P, int DIR, int MODE>
 __global__ void __launch_bounds__(tile_max_threads(MODE, P::kF64, false), 1)
     k_strided_pipe(const __grid_constant__ CUtensorMap tin, const __grid_constant__ CUtensorMap tout,
                    const __grid_constant__ SPipeParams pp, const float4* __restrict__ tw_g) {
+  pass_launch_next();
   const int nb = pp.c.nbuf, G = pp.c.groups;
   const int step = (int)gridDim.x;
   {
@@ -395,9 +404,12 @@ __global__ void __launch_bounds__(tile_max_threads(MODE, P::kF64, false), 1)
       mbar_fence_init();
     }
   }
+  pass_begin();
+  if (threadIdx.x == 0) {  // held in shared memory, not in registers across the stages
+    ring_smem<P>(pp.c).cta[1] = range_k(pp.s.range);
+    ring_smem<P>(pp.c).cta[2] = 0;
+  }
   __syncthreads();
-  const int k = range_k(pp.s.range);
-  uint32_t amax = 0;
   const int g = (int)threadIdx.x / pp.c.gthreads;
   const GroupThreads th{(int)threadIdx.x - g * pp.c.gthreads, pp.c.gthreads, 1 + g};
   // one group alone (nb >= 3) loads one tile ahead, into the buffer whose store
@@ -425,7 +437,15 @@ __global__ void __launch_bounds__(tile_max_threads(MODE, P::kF64, false), 1)
       bulk_wait_read<0>();
       strided_issue<P>(pp, &tin, rtile, rbuf, th);
     }
-    strided_fix<P>(pp.s, pp.use_tma != 0, ring_smem<P>(pp.c).buf0 + b * pp.c.buf_elems, k, amax, th);
+    {
+      const RingSmem<P> sm = ring_smem<P>(pp.c);
+      uint32_t amax = 0;
+      strided_fix<P>(pp.s, pp.use_tma != 0, sm.buf0 + b * pp.c.buf_elems, sm.cta[1], amax, th);
+      if (P::kF64 && pp.s.in_user) {
+        amax = __reduce_max_sync(0xFFFFFFFFu, amax);
+        if ((th.t & 31) == 0) atomicMax(reinterpret_cast<unsigned*>(&sm.cta[2]), amax);
+      }
+    }
     {
       const RingSmem<P> sm = ring_smem<P>(pp.c);
       Tile<P, GroupThreads> t{sm.buf0 + b * pp.c.buf_elems, nullptr, pp.s.M, pp.s.log2m, 1, pp.s.M, 0, 0, nullptr, th};
@@ -437,6 +457,7 @@ __global__ void __launch_bounds__(tile_max_threads(MODE, P::kF64, false), 1)
       int xt, o1, o2;
       strided_decode(pp, tile, xt, o1, o2);
       typename P::W* tb = ring_smem<P>(pp.c).buf0 + b * pp.c.buf_elems;
+      const int k = ring_smem<P>(pp.c).cta[1];
       rtile = !lag && tile + nb * step < pp.c.ntiles ? tile + nb * step : -1;
       rbuf = b;
       if (pp.tma_store) {
@@ -485,7 +506,8 @@ __global__ void __launch_bounds__(tile_max_threads(MODE, P::kF64, false), 1)
       for (int i = 0; i < nb; ++i)
         if (sm.issued[i]) mbar_wait_bounded(&sm.mbar[i], (sm.issued[i] - 1) & 1, nullptr);
   }
-  range_flush(pp.s.range, amax);
+  if (P::kF64 && pp.s.in_user && threadIdx.x < 32)
+    range_flush(pp.s.range, threadIdx.x == 0 ? (uint32_t)ring_smem<P>(pp.c).cta[2] : 0u);
 }
 
 // ---------------------------------------------------------------- X passes
@@ -762,6 +784,7 @@ P3G_D void xc2r_store(const XParams& x, const typename P::W* sm, int p0, int fie
 template <class P, bool R2C, int MODE>
 __global__ void __launch_bounds__(tile_max_threads(MODE, P::kF64, true), 1)
     k_x_pipe(const __grid_constant__ XPipeParams pp, const float4* __restrict__ tw_g) {
+  pass_launch_next();
   const int nb = pp.c.nbuf, G = pp.c.groups;
   const int step = (int)gridDim.x;
   {
@@ -773,11 +796,12 @@ __global__ void __launch_bounds__(tile_max_threads(MODE, P::kF64, true), 1)
         sm.issued[i] = 0;
       }
       sm.cta[0] = 0;
-      sm.cta[1] = range_k(pp.x.range);
       sm.cta[2] = 0;
       mbar_fence_init();
     }
   }
+  pass_begin();
+  if (threadIdx.x == 0) ring_smem<P>(pp.c).cta[1] = range_k(pp.x.range);
   __syncthreads();
   // the exponent bias and the largest input seen live in shared memory: no
   // register of theirs is held across the stages

@@ -2,9 +2,30 @@
 // direction (the unrolled codelets dominate the build time).
 #pragma once
 
+#include <utility>
+
 #include "p3g_pipe.cuh"
 
 namespace p3g {
+
+// Launch with programmatic stream serialization: the kernel may start while
+// the one before it in the stream still runs, and waits (pass_begin) before it
+// touches anything that kernel reads or writes.
+template <class... Params, class... Args>
+cudaError_t launch_pass(void (*kernel)(Params...), int grid, int threads, size_t smem, cudaStream_t st,
+                        Args&&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
 
 template <class P, int DIR>
 cudaError_t launch_strided_pipe(const CUtensorMap* map, const CUtensorMap* omap, const SPipeParams& p,
@@ -18,8 +39,7 @@ cudaError_t launch_strided_pipe(const CUtensorMap* map, const CUtensorMap* omap,
   }
   const cudaError_t e = opt_in_smem((const void*)kernel, 227 * 1024);
   if (e != cudaSuccess) return e;
-  kernel<<<grid, threads, smem, st>>>(*map, *omap, p, tw);
-  return cudaGetLastError();
+  return launch_pass(kernel, grid, threads, smem, st, *map, *omap, p, tw);
 }
 
 template <class P, bool R2C>
@@ -33,8 +53,7 @@ cudaError_t launch_x_pipe(const XPipeParams& p, const float4* tw, TileMode mode,
   }
   const cudaError_t e = opt_in_smem((const void*)kernel, 227 * 1024);
   if (e != cudaSuccess) return e;
-  kernel<<<grid, threads, smem, st>>>(p, tw);
-  return cudaGetLastError();
+  return launch_pass(kernel, grid, threads, smem, st, p, tw);
 }
 
 #define P3G_X_INSTANTIATE(P, R2C)                                                                              \
