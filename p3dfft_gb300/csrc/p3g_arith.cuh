@@ -171,8 +171,10 @@ P3G_HD uint32_t shl3_funnel(uint32_t lo, uint32_t hi) {
 #endif
 }
 
+constexpr uint32_t kD2dfMidLow = 949u << 20;   // |high word| of the short route's smallest values
+constexpr uint32_t kD2dfMidSpan = 202u << 20;  // and the span of its window
 P3G_HD bool d2df_is_edge(uint32_t hw) {  // e < 949 or e > 1150
-  return (hw & 0x7FFFFFFFu) - (949u << 20) >= (202u << 20);
+  return (hw & 0x7FFFFFFFu) - kD2dfMidLow >= kD2dfMidSpan;
 }
 // The short route alone (x must not be an edge value).
 P3G_HD df d2df_mid(double x) {
@@ -530,10 +532,12 @@ struct PathF64 {
   P3G_D static C from_uc(double2 v, int k) { return make_cdf(d2df_scaled(v.x, k), d2df_scaled(v.y, k)); }
   P3G_D static double2 to_uc(C c, int k) { return make_double2(to_ur(re(c), k), to_ur(im(c), k)); }
   P3G_D static df from_ur(double v, int k) { return d2df_scaled(v, k); }
-  // z = x1 + i x2 for values of the short route; `edge` collects whether the
-  // caller has to convert again with make_slow
-  P3G_D static C make_mid(double x1, double x2, bool& edge) {
-    edge = edge || d2df_is_edge((uint32_t)__double2hiint(x1)) || d2df_is_edge((uint32_t)__double2hiint(x2));
+  // z = x1 + i x2 for values of the short route; `off` becomes the largest
+  // |high word| - kD2dfMidLow (unsigned): from kD2dfMidSpan on, the caller has
+  // to convert again with make_slow
+  P3G_D static C make_mid(double x1, double x2, uint32_t& off) {
+    off = max(off, ((uint32_t)__double2hiint(x1) & 0x7FFFFFFFu) - kD2dfMidLow);
+    off = max(off, ((uint32_t)__double2hiint(x2) & 0x7FFFFFFFu) - kD2dfMidLow);
     return make_cdf(d2df_mid(x1), d2df_mid(x2));
   }
   static __device__ __noinline__ float4 make_slow(double x1, double x2, int k) {
@@ -571,7 +575,7 @@ struct PathF32 {
   P3G_D static C from_uc(float2 v, int) { return from_w(v); }
   P3G_D static float2 to_uc(C c, int) { return to_w(c); }
   P3G_D static float from_ur(float v, int) { return v; }
-  P3G_D static C make_mid(float x1, float x2, bool&) { return make(x1, x2); }
+  P3G_D static C make_mid(float x1, float x2, uint32_t&) { return make(x1, x2); }
   P3G_D static float2 make_slow(float x1, float x2, int) { return make_float2(x1, x2); }
   P3G_D static float to_ur(float v, int) { return v; }
   P3G_D static void track(uint32_t&, float) {}

@@ -286,21 +286,28 @@ __device__ __forceinline__ void stage_reg(const Tile<P, TH>& t, int N, int ns, c
         // one branch per butterfly for the values (or bias) that need the long
         // conversion, out of line: with one per value the inlined long route
         // made the stage's code several times larger
-        bool edge = false;
-        uint32_t am = 0;
+        // the fast route keeps the largest |high word| less that of 2^-74, as an
+        // unsigned number: one value outside the route's window makes it too
+        // large, and without one it gives the tracked maximum
+        uint32_t off = 0;
 #pragma unroll
         for (int q = 0; q < R; ++q) {
           const UR x1 = lds1(ra + q * rstep, (UR*)nullptr), x2 = lds1(ra + lstep + q * rstep, (UR*)nullptr);
-          P::track(am, x1);
-          P::track(am, x2);
-          v[i][q] = P::make_mid(x1, x2, edge);
+          v[i][q] = P::make_mid(x1, x2, off);
         }
-        if (t.amax) *t.amax = max(*t.amax, am);
-        if (P::kF64 && (edge || t.ebias != 0)) {
+        if constexpr (P::kF64) {
+          uint32_t am = off + kD2dfMidLow;
+          if (off >= kD2dfMidSpan || t.ebias != 0) {
+            am = 0;
 #pragma unroll
-          for (int q = 0; q < R; ++q)
-            v[i][q] = P::from_w(P::make_slow(lds1(ra + q * rstep, (UR*)nullptr),
-                                             lds1(ra + lstep + q * rstep, (UR*)nullptr), t.ebias));
+            for (int q = 0; q < R; ++q) {
+              const UR x1 = lds1(ra + q * rstep, (UR*)nullptr), x2 = lds1(ra + lstep + q * rstep, (UR*)nullptr);
+              P::track(am, x1);
+              P::track(am, x2);
+              v[i][q] = P::from_w(P::make_slow(x1, x2, t.ebias));
+            }
+          }
+          if (t.amax) *t.amax = max(*t.amax, am);
         }
       } else if constexpr (RAW == kRawC2R) {
         const int nh = N / 2 + 1;
