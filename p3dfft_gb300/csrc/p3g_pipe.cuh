@@ -71,7 +71,7 @@ struct TileElems {
   static constexpr int value = P::kF64 ? 16 : 32;
 };
 constexpr int kMaxGroups = 8;        // named barriers 1..8
-constexpr int kMaxTileBuffers = 12;  // ring of tile buffers
+constexpr int kMaxTileBuffers = 16;  // ring of tile buffers
 
 // ------------------------------------------------------------ strided Y/Z
 template <class P>

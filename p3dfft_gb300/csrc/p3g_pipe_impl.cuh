@@ -10,10 +10,13 @@ namespace p3g {
 
 // Launch with programmatic stream serialization: the kernel may start while
 // the one before it in the stream still runs, and waits (pass_begin) before it
-// touches anything that kernel reads or writes.
+// touches anything that kernel reads or writes.  Only for passes of few tiles
+// per group, whose start is a good part of their time: the long binary32
+// passes ran 4-8 % slower with it (1024^3 forward 6.28 -> 6.57 ms).
+constexpr int kOverlapTiles = 16;
 template <class... Params, class... Args>
-cudaError_t launch_pass(void (*kernel)(Params...), int grid, int threads, size_t smem, cudaStream_t st,
-                        Args&&... args) {
+cudaError_t launch_pass(void (*kernel)(Params...), const PipeCommon& pc, int grid, int threads, size_t smem,
+                        cudaStream_t st, Args&&... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(threads);
@@ -23,7 +26,7 @@ cudaError_t launch_pass(void (*kernel)(Params...), int grid, int threads, size_t
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = (long long)pc.ntiles <= (long long)kOverlapTiles * grid * pc.groups ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 
@@ -39,7 +42,7 @@ cudaError_t launch_strided_pipe(const CUtensorMap* map, const CUtensorMap* omap,
   }
   const cudaError_t e = opt_in_smem((const void*)kernel, 227 * 1024);
   if (e != cudaSuccess) return e;
-  return launch_pass(kernel, grid, threads, smem, st, *map, *omap, p, tw);
+  return launch_pass(kernel, p.c, grid, threads, smem, st, *map, *omap, p, tw);
 }
 
 template <class P, bool R2C>
@@ -53,7 +56,7 @@ cudaError_t launch_x_pipe(const XPipeParams& p, const float4* tw, TileMode mode,
   }
   const cudaError_t e = opt_in_smem((const void*)kernel, 227 * 1024);
   if (e != cudaSuccess) return e;
-  return launch_pass(kernel, grid, threads, smem, st, p, tw);
+  return launch_pass(kernel, p.c, grid, threads, smem, st, p, tw);
 }
 
 #define P3G_X_INSTANTIATE(P, R2C)                                                                              \

@@ -390,15 +390,16 @@ static TileShape size_strided(const AxisPlan& ap, long long nv) {
       for (int M = 1; M <= max_m && M < 2 * X; M *= 2) {
         const int tg = stage_threads(sp, M, E);
         const bool full = pow2 && (long long)M * n == (long long)tg * E && E == Emax;
-        // binary32 FULL passes that store by threads run one group with twice
-        // the registers: at 128 the spilled words and the stores share what is
-        // left of the L1 (1024-point Z forward 5.4 ms against 2.5 ms).  So do
+        // binary32 FULL passes of 512 points or more that store by threads run
+        // one group with twice the registers: at 128 the spilled words and the
+        // stores share what is left of the L1 (1024-point Z forward 5.4 ms against
+        // 2.5 ms; 256 points: 0.043 against 0.049 ms the other way).  So do
         // those with far rows, where every row of a tile is in a memory page
         // of its own and groups that drift apart spread over more pages at a
         // time (Y of 1024^3, 4.2 MB apart: 1.95 ms with two groups, 1.81 ms
         // with one; of 768 x 1024 x 540, 1.7 MB apart: 0.59 against 0.73 ms)
         const TileMode mode =
-            E < Emax ? kTileSmall : (!full ? kTileGeneral : (!f64 && (tstore || far_rows) ? kTileFullWide : kTileFull));
+            E < Emax ? kTileSmall : (!full ? kTileGeneral : (!f64 && ((tstore && n >= 512) || far_rows) ? kTileFullWide : kTileFull));
         const int max_threads = tile_max_threads(mode, f64, false);
         const size_t buf = ((size_t)M * n * esize + 1023) / 1024 * 1024;
         if (tg > 512 || fixed + 2 * buf > room) break;
@@ -427,10 +428,13 @@ static TileShape size_strided(const AxisPlan& ap, long long nv) {
           o.mode = mode;
           o.g = g;
           o.threads = g * tg;
-          // more loads in flight than one beyond the groups pay off only where
-          // the tiles leave by TMA (binary32 512^3 Y: 0.19 ms with two, 0.26
-          // with one; 540-point binary32 Z: 1.60 with two, 1.55 with one)
-          o.nbuf = std::min(fit, g + (tstore ? 1 : 2));
+          // buffers beyond the groups (loads in flight): two, one where the
+          // tiles leave by threads (binary32 512^3 Y: 0.19 ms with two, 0.26
+          // with one; 540-point binary32 Z: 1.42 with two, 1.34 with one), and
+          // twice as many for the small tiles of short binary32 lines (256^3 Y:
+          // 0.046 -> 0.040 ms with four, Z 0.051 -> 0.049 with two)
+          const bool small_tile = !f64 && buf <= (tstore ? 24 : 16) * 1024;
+          o.nbuf = std::min(fit, g + (tstore ? 1 : 2) * (small_tile ? 2 : 1));
           o.buf_elems = (int)(buf / esize);
           o.smem = fixed + o.nbuf * buf;
           o.fam = sp.fam;
