@@ -61,43 +61,59 @@ cudaError_t opt_in_smem(const void* func, int bytes) {
 
 // ------------------------------------------------------------ factorisation
 // Cheapest split of 2^e[0] 3^e[1] 5^e[2] 7^e[3] into codelet radices, powers
-// of two of at most rmax and others of at most odd_max: the operations per point of a codelet (packed double-float ones;
-// the binary32 ratios are alike), of the twiddles before every stage but one,
-// and of a stage's shared-memory exchange.
+// of two of at most rmax and others of at most odd_max.  A stage costs the
+// operations per point of its codelet (packed double-float ones; the binary32
+// ratios are alike), of the twiddles before every stage but one, and of its
+// shared-memory exchange.  E > 0 (binary32 grouped kernels, E elements per
+// thread): the stage that fits a thread's elements worst sets the threads per
+// tile, and the others leave as much idle (768 points as 16 x 16 x 3 rather
+// than 8 x 8 x 12: X r2c of 768 x 1024 x 540 1.26 -> 1.18 ms; on F64, where more
+// threads per tile pay, 8 x 4 x 12 runs 384-point Y in 0.327 against 0.353 ms).
 struct Split {
   double cost = 1e300;
   std::vector<int> radices;
 };
-static const Split& best_split(const std::array<int, 4>& e, int rmax, int odd_max, std::map<std::array<int, 4>, Split>& memo) {
-  const auto known = memo.find(e);
-  if (known != memo.end()) return known->second;
-  struct Codelet {
-    int r;
-    std::array<int, 4> e;
-    double ops;
-  };
-  static const Codelet codelets[] = {
-      {16, {4, 0, 0, 0}, 40}, {15, {0, 1, 1, 0}, 52}, {12, {2, 1, 0, 0}, 36}, {10, {1, 0, 1, 0}, 40},
-      {9, {0, 2, 0, 0}, 42},  {8, {3, 0, 0, 0}, 26},  {7, {0, 0, 0, 1}, 50},  {6, {1, 1, 0, 0}, 28},
-      {5, {0, 0, 1, 0}, 32},  {4, {2, 0, 0, 0}, 16},  {3, {0, 1, 0, 0}, 20},  {2, {1, 0, 0, 0}, 8},
-  };
-  Split best;
-  if (e == std::array<int, 4>{0, 0, 0, 0}) best.cost = 0;
-  for (const Codelet& c : codelets) {
+struct Codelet {
+  int r;
+  std::array<int, 4> e;
+  double ops;
+};
+static const Codelet kCodelets[] = {
+    {16, {4, 0, 0, 0}, 40}, {15, {0, 1, 1, 0}, 52}, {12, {2, 1, 0, 0}, 36}, {10, {1, 0, 1, 0}, 40},
+    {9, {0, 2, 0, 0}, 42},  {8, {3, 0, 0, 0}, 26},  {7, {0, 0, 0, 1}, 50},  {6, {1, 1, 0, 0}, 28},
+    {5, {0, 0, 1, 0}, 32},  {4, {2, 0, 0, 0}, 16},  {3, {0, 1, 0, 0}, 20},  {2, {1, 0, 0, 0}, 8},
+};
+static double split_cost(const std::vector<const Codelet*>& c, int E) {
+  auto fill = [&](int r) { return E > 0 ? (double)(r * stage_butterflies(E, r, true)) / E : 1.0; };
+  double worst = 1.0, cost = 0;
+  for (const Codelet* s : c) worst = std::min(worst, fill(s->r));
+  for (size_t i = 0; i < c.size(); ++i)
+    cost += fill(c[i]->r) / worst * (c[i]->ops + 30 + (i == 0 ? 0.0 : 16.0 * (1.0 - 1.0 / c[i]->r)));
+  return cost;
+}
+static void best_split(std::array<int, 4> e, int rmax, int odd_max, int E, size_t from,
+                       std::vector<const Codelet*>& cur, Split& best) {
+  if (e == std::array<int, 4>{0, 0, 0, 0}) {
+    const double cost = split_cost(cur, E);
+    if (cost < best.cost) {
+      best.cost = cost;
+      best.radices.clear();
+      for (const Codelet* c : cur) best.radices.push_back(c->r);
+    }
+    return;
+  }
+  if (cur.size() >= 6 && cur.size() * 30 > best.cost) return;
+  for (size_t i = from; i < sizeof(kCodelets) / sizeof(kCodelets[0]); ++i) {
+    const Codelet& c = kCodelets[i];
     if (c.r > ((c.r & (c.r - 1)) == 0 ? rmax : odd_max)) continue;
     std::array<int, 4> rest = e;
     bool ok = true;
-    for (int i = 0; i < 4; ++i) ok = ok && (rest[i] -= c.e[i]) >= 0;
+    for (int k = 0; k < 4; ++k) ok = ok && (rest[k] -= c.e[k]) >= 0;
     if (!ok) continue;
-    const Split& sub = best_split(rest, rmax, odd_max, memo);
-    const double cost = sub.cost + c.ops + 30 + (sub.radices.empty() ? 0.0 : 16.0 * (1.0 - 1.0 / c.r));
-    if (cost < best.cost) {
-      best.cost = cost;
-      best.radices = sub.radices;
-      best.radices.push_back(c.r);
-    }
+    cur.push_back(&c);
+    best_split(rest, rmax, odd_max, E, i, cur, best);
+    cur.pop_back();
   }
-  return memo[e] = best;
 }
 
 // Stage radices for length n in the order of kFamilies, other primes last.
@@ -121,8 +137,10 @@ static bool factor(int n, int max_pow2, SplitKind kind, std::vector<int>& radice
     int rest = n;
     for (int i = 0; i < 4; ++i)
       for (; rest % primes[i] == 0; rest /= primes[i]) ++e[i];
-    std::map<std::array<int, 4>, Split> memo;
-    const Split& s = best_split(e, std::min(max_pow2, 16), kind == kSplitWide ? 16 : 8, memo);
+    Split s;
+    std::vector<const Codelet*> cur;
+    best_split(e, std::min(max_pow2, 16), kind == kSplitWide ? 16 : 8,
+               kind == kSplitWide && max_pow2 == 32 ? TileElems<PathF32>::value : 0, 0, cur, s);
     radices.clear();
     for (int f : kFamilies)
       for (int r : s.radices)
