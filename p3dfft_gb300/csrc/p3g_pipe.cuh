@@ -1,16 +1,16 @@
 // Pipelined (persistent, multi-buffered) pass kernels.
 //
-// Each CTA walks a strided list of tiles (grid = SMs x resident CTAs).  While
-// it transforms tile i in one shared buffer, the copy of the next tile (two
-// tiles ahead in the X kernels with three buffers) is already in flight (TMA
-// tensor tiles, bulk copies or cp.async), so HBM traffic overlaps the
-// butterflies.  Each strided tile goes through: a fix-up step in shared
+// One CTA per SM walks a strided list of tiles.  Its threads form groups that
+// each transform tiles of their own; the tiles go round a ring of more buffers
+// than groups, and the copies into the free ones are in flight (TMA tensor
+// tiles, bulk copies or cp.async) while the groups work, so HBM traffic
+// overlaps the butterflies.  Each strided tile goes through: a fix-up step in shared
 // memory (format conversion of user data, DCT-I/DST-I extension), the
 // Stockham stages of p3g_engine.cuh with the pass's twiddles held in shared
 // memory for the life of the CTA, and a store step with the pruning map and
 // output format conversion fused in, or, for rows stored one to one, TMA
-// tensor stores issued by one thread (with a third buffer, so a buffer is
-// reloaded only after its store has read it).
+// tensor stores issued by one thread (a buffer is reloaded only after its
+// store has read it).
 #pragma once
 
 #include <type_traits>

@@ -379,8 +379,8 @@ static bool size_tile(AxisPlan& ap, int n, int lines_avail, bool f64, int max_m 
 // row efficiency being that of the tile's row segments in memory: 32-byte
 // segments ran the 1024-point binary32 Y pass at 4.0 ms against 1.95 ms with
 // 64 bytes.  Fewer than 12 busy warps or a single group leave the FMA pipes
-// idle through the tiles' exchanges (1024-point binary64 Y: 6.9 ms with one
-// group of 256 threads, 5.3 ms with two).  The latency term matters when the
+// idle through the tiles' exchanges (1024^3 binary64 Y: 6.5 ms with one
+// group of 256 threads, 5.3 ms with groups).  The latency term matters when the
 // grid has fewer tiles than the GPU has groups: half the points per thread
 // halve the length of a thread's serial chain.
 static TileShape size_strided(const AxisPlan& ap, long long nv) {

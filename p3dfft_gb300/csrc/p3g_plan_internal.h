@@ -47,8 +47,8 @@ struct AxisPlan {
   bool pipe_ok = false;
   TileExtents ext;
   std::map<int, TileShape> shapes;
-  // F64 wide pipelined kernels (16 points per thread): a second stage plan
-  // with radix-16 stages and its twiddle slice; every other kernel runs sp
+  // the grouped pass kernels: a second stage plan with the large codelets and
+  // its twiddle slice; the other kernels, and grids of few tiles, run sp
   StagePlan spw{};
   int spw_index = -1;  // -1: none, the pipelined kernels run sp
   bool fixed_plan = false;  // kSplitFixed: no choice between spw and sp
