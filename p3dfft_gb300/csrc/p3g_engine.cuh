@@ -476,11 +476,9 @@ __device__ __forceinline__ void run_families(const Tile<P, TH>& t, const float4*
   run_family<P, DIR, 4, E, LAY, FULL, RAW>(t, tw, N, family_count(fam, 3), ns, off);
   run_family<P, DIR, 2, E, LAY, FULL, RAW>(t, tw, N, family_count(fam, 4), ns, off);
   if constexpr (!FULL) {
-    if constexpr (MAXR >= 16) {
+    if constexpr (MAXR >= 16 && TH::kHold) {
       run_family<P, DIR, 12, E, LAY, false, RAW>(t, tw, N, family_count(fam, 5), ns, off);
       run_family<P, DIR, 10, E, LAY, false, RAW>(t, tw, N, family_count(fam, 6), ns, off);
-    }
-    if constexpr (MAXR >= 16 && TH::kHold) {
       run_family<P, DIR, 15, E, LAY, false, RAW>(t, tw, N, family_count(fam, 7), ns, off);
       run_family<P, DIR, 9, E, LAY, false, RAW>(t, tw, N, family_count(fam, 8), ns, off);
     }

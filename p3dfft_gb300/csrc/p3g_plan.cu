@@ -105,7 +105,7 @@ static void best_split(std::array<int, 4> e, int rmax, int odd_max, int E, size_
   if (cur.size() >= 6 && cur.size() * 30 > best.cost) return;
   for (size_t i = from; i < sizeof(kCodelets) / sizeof(kCodelets[0]); ++i) {
     const Codelet& c = kCodelets[i];
-    if (c.r > ((c.r & (c.r - 1)) == 0 ? rmax : odd_max) || (c.r == 9 && odd_max < 15)) continue;
+    if (c.r > ((c.r & (c.r - 1)) == 0 ? rmax : odd_max)) continue;
     std::array<int, 4> rest = e;
     bool ok = true;
     for (int k = 0; k < 4; ++k) ok = ok && (rest[k] -= c.e[k]) >= 0;
@@ -123,7 +123,7 @@ static void best_split(std::array<int, 4> e, int rmax, int odd_max, int E, size_
 // into the fewest stages of at most 32, as evenly as possible (1024 = 32 x 32,
 // 512 = 32 x 16, 256 = 16 x 16, 128 = 16 x 8).  Lengths with factors 3, 5 and
 // 7 take the cheapest split into codelets of at most 16 points (the narrow
-// plans, besides the powers of two: of at most 8 points, and 10 and 12 on F32).
+// plans: of at most 8 besides the powers of two).
 //
 // kSplitFixed: radices 3 and 5 after the powers of two and other primes as
 // generic stages.  The binary32 STRIDE1 plans keep it: their output goes into
@@ -139,7 +139,7 @@ static bool factor(int n, int max_pow2, SplitKind kind, std::vector<int>& radice
       for (; rest % primes[i] == 0; rest /= primes[i]) ++e[i];
     Split s;
     std::vector<const Codelet*> cur;
-    best_split(e, std::min(max_pow2, 16), kind == kSplitWide ? 16 : (max_pow2 >= 16 ? 12 : 8),
+    best_split(e, std::min(max_pow2, 16), kind == kSplitWide ? 16 : 8,
                kind == kSplitWide && max_pow2 == 32 ? TileElems<PathF32>::value : 0, 0, cur, s);
     radices.clear();
     for (int f : kFamilies)
