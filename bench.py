@@ -47,15 +47,15 @@ CONFIGS = {
 MODES = {"pipe_tma": (True, True), "pipe_cpasync": (True, False), "single_tile": (False, False)}
 
 # DRAM bytes (read + write) per algorithmic byte of one launch of the
-# dominant kernel, from ncu captures of its Y pass on a 1024x1024x32 grid
-# (273.69 MB read + 225.91 MB written) and its Z passes on a 1024x32x1024
-# grid (273.93 + 222.29 and 270.01 + 224.63 MB), each for 538.97 MB of 2C
-# model traffic; the four launches of a round trip (Y, Z, Z, Y) averaged.
-# The full-size launches move the same bytes per line, so traffic scales
-# with the model.
+# dominant kernel, from ncu captures of its Y passes on a 1024x1024x32 grid
+# (forward 273.67 MB read + 221.91 MB written, backward 273.69 + 218.90) and
+# its Z passes on a 1024x32x1024 grid (275.79 + 217.86 and 270.10 + 218.32 MB),
+# each for 538.97 MB of 2C model traffic; the four launches of a round trip
+# averaged.  The full-size launches move the same bytes per line, so traffic
+# scales with the model.
 TRAFFIC_PER_ALGO_BYTE = {
-    "k_strided_pipe": (2 * (273.687040e6 + 225.914880e6) + (273.926656e6 + 222.291712e6) +
-                       (270.008320e6 + 224.634880e6)) / (4 * 538968064.0)}
+    "k_strided_pipe": (273.671168e6 + 221.905664e6 + 273.686784e6 + 218.902784e6 +
+                       275.788544e6 + 217.860096e6 + 270.095872e6 + 218.322688e6) / (4 * 538968064.0)}
 
 
 def load_peaks():
@@ -429,9 +429,8 @@ def run_ours(args):
     pass_bytes = {"x_r2c": bm["x"], "y_fwd": bm["y"], "z_fwd": bm["z"], "z_bwd": bm["z"], "y_bwd": bm["y"],
                   "x_c2r": bm["x"]}
     # passes grouped by kernel; the dominant kernel is the one with the largest
-    # total time per round trip (4 strided launches, 1 r2c, 1 c2r)
-    groups = {"k_strided_pipe": ["y_fwd", "z_fwd", "z_bwd", "y_bwd"], "k_xr2c_pipe": ["x_r2c"],
-              "k_xc2r_pipe": ["x_c2r"]}
+    # total time per round trip (4 strided launches, 2 X launches)
+    groups = {"k_strided_pipe": ["y_fwd", "z_fwd", "z_bwd", "y_bwd"], "k_x_pipe": ["x_r2c", "x_c2r"]}
     dom = max(groups, key=lambda k: sum(pass_ms[p] for p in groups[k]))
     nl = len(groups[dom])
     dom_ms = sum(pass_ms[p] for p in groups[dom]) / nl
@@ -493,7 +492,7 @@ def run_ours(args):
                      "peak": peak, "unit": "GB/s", "frac": round(achieved / peak, 4) if achieved else None,
                      "peak_kind": peak_kind, "traffic": traffic,
                      "traffic_source": "ncu DRAM read+write of the Y pass (1024x1024x32) and Z passes "
-                                       "(1024x32x1024), 0.923 per algorithmic byte, scaled to this launch",
+                                       "(1024x32x1024), 0.914 per algorithmic byte, scaled to this launch",
                      "step_bytes_model": bm["rt"],
                      "step_frac": round(bm["rt"] / (ms64 * 1e-3) / 1e9 / peak, 4)},
         "gpu_launches": launches,
