@@ -289,6 +289,17 @@ P3G_HD double scale_pow2(double d, int k) {
   return u2d(((uint64_t)((hw & 0x800FFFFFu) | ((uint32_t)e2 << 20)) << 32) | (uint32_t)b);
 }
 
+// hi + lo rounded to binary64 for every pair, also the sums below 2^-75 that
+// df2d cuts (squares of modes carry no exponent bias): those below 2^-70 go
+// through it scaled by 2^100, which is exact, and back in the exponent field.
+// (double)hi + (double)lo is the same value on the binary64 pipe.
+P3G_HD double df2d_any(float hi, float lo) {
+  const bool low = (f2u(hi) & 0x7FFFFFFFu) < (57u << 23);
+  const float m = low ? 0x1p100f : 1.0f;
+  const uint64_t d = d2u(df2d(hi * m, lo * m));
+  return u2d(low && d != 0 ? d - (100ull << 52) : d);
+}
+
 // The window of largest magnitudes the F64 path transforms without a bias:
 // 2^kRangeLo <= max |x| < 2^(kRangeTop - log2n + 1), where 2^log2n bounds the
 // transform's gain (nx ny 2 (nz + 1) covers the DCT-I/DST-I extensions).

@@ -92,7 +92,7 @@ P3G_D void spectrum_rows(const SpecParams& prm, double* hist_all, int r_first, i
       auto flush = [&] {
         // modes beyond kmax are dropped (the sample would write past E); the sum
         // is widened with integer instructions, which leaves one binary64 add
-        if (bin >= 0 && bin <= prm.kmax) atomicAdd(hist + bin, df2d(acc.hi, acc.lo));
+        if (bin >= 0 && bin <= prm.kmax) atomicAdd(hist + bin, df2d_any(acc.hi, acc.lo));
       };
 #pragma unroll 4
       for (int i = i0; i < i1; ++i) {
