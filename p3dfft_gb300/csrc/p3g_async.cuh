@@ -58,6 +58,8 @@ P3G_D void mbar_arrive_expect_tx(uint64_t* b, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_u32(b)), "r"(bytes)
                : "memory");
 }
+// Waits for every cp.async this thread has issued, committed to a group or not.
+P3G_D void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 // Arrives on the barrier once every cp.async this thread issued before has
 // completed (counts as one of the barrier's expected arrivals).
 P3G_D void cp_async_mbar_arrive(uint64_t* b) {
@@ -84,6 +86,19 @@ P3G_D bool mbar_wait_bounded(uint64_t* b, uint32_t parity, int* err) {
   }
   if (err) atomicExch(err, kErrMbarTimeout);
   return false;
+}
+// Bounded wait for the loads issued last into each of n buffers (issued[i]
+// loads, barrier bar[i]): one limit of kMbarWaitNs for all of them.
+P3G_D void mbar_drain_bounded(uint64_t* bar, const int* issued, int n) {
+  const uint64_t t0 = global_ns();
+  for (int i = 0; i < n; ++i) {
+    if (issued[i] == 0) continue;
+    const uint32_t parity = (issued[i] - 1) & 1;
+    for (uint32_t k = 0; k < kMbarSpinLimit && !mbar_try_wait(bar + i, parity); ++k) {
+      if (global_ns() - t0 > kMbarWaitNs) break;
+      if (k > 16) __nanosleep(32);
+    }
+  }
 }
 // Orders this thread's generic-proxy shared-memory accesses before later
 // async-proxy (TMA) writes to the same buffer.

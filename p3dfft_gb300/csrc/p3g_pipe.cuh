@@ -495,16 +495,14 @@ __global__ void __launch_bounds__(tile_max_threads(MODE, P::kF64, false), 1)
       ++use;
     }
   }
-  if (!pp.use_tma) cp_async_wait<0>();
+  if (!pp.use_tma) cp_async_wait_all();
   // the tile stores must have completed before the CTA's shared memory goes
   if (pp.tma_store && th.t == 0) bulk_wait_all();
   __syncthreads();
   // a wait timed out: loads may be in flight that no group waits for
   if (threadIdx.x == 0 && pp.use_tma) {
     const RingSmem<P> sm = ring_smem<P>(pp.c);
-    if (sm.cta[0])
-      for (int i = 0; i < nb; ++i)
-        if (sm.issued[i]) mbar_wait_bounded(&sm.mbar[i], (sm.issued[i] - 1) & 1, nullptr);
+    if (sm.cta[0]) mbar_drain_bounded(sm.mbar, sm.issued, nb);
   }
   if (P::kF64 && pp.s.in_user && threadIdx.x < 32)
     range_flush(pp.s.range, threadIdx.x == 0 ? (uint32_t)ring_smem<P>(pp.c).cta[2] : 0u);
@@ -870,14 +868,12 @@ __global__ void __launch_bounds__(tile_max_threads(MODE, P::kF64, true), 1)
       ++use;
     }
   }
-  if (!pp.bulk) cp_async_wait<0>();
+  if (!pp.bulk) cp_async_wait_all();
   __syncthreads();
   // a wait timed out: loads may be in flight that no group waits for
   if (threadIdx.x == 0 && pp.bulk) {
     const RingSmem<P> sm = ring_smem<P>(pp.c);
-    if (sm.cta[0])
-      for (int i = 0; i < nb; ++i)
-        if (sm.issued[i]) mbar_wait_bounded(&sm.mbar[i], (sm.issued[i] - 1) & 1, nullptr);
+    if (sm.cta[0]) mbar_drain_bounded(sm.mbar, sm.issued, nb);
   }
   if constexpr (R2C) {
     if (threadIdx.x < 32) range_flush(pp.x.range, threadIdx.x == 0 ? (uint32_t)ring_smem<P>(pp.c).cta[2] : 0u);
