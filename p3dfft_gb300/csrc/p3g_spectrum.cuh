@@ -58,16 +58,42 @@ P3G_D void load_mode(const float2* p, df& re, df& im) {
   im = df{v.y, 0.0f};
 }
 
+// Adds the lanes' last sums to their bins.  Where the other wavenumbers are much
+// larger than the fast axis's, nearly all lanes end in the same bin and their
+// additions to it would follow one another, so neighbours of one bin add up
+// theirs first (z rows of 64 modes of 600 x 64 x 64 STRIDE1: 30.8 us without, 20.6
+// with).  Out of line: inlined, it slowed the loop over the modes (200 x 180 x
+// 150 binary32 41 against 34.6 us).
+static __device__ __noinline__ void flush_lanes(double* hist, int kmax, int bin, df acc) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t le_mask = 0xFFFFFFFFu >> (31 - lane);
+  const int prev = __shfl_up_sync(0xFFFFFFFFu, bin, 1);
+  const uint32_t heads = __ballot_sync(0xFFFFFFFFu, lane == 0 || prev != bin);
+  if (heads != 0xFFFFFFFFu) {
+    const int seg = __popc(heads & le_mask);
+#pragma unroll 1
+    for (int d = 1; d < 32; d <<= 1) {
+      const float oh = __shfl_down_sync(0xFFFFFFFFu, acc.hi, d);
+      const float ol = __shfl_down_sync(0xFFFFFFFFu, acc.lo, d);
+      const int os = __shfl_down_sync(0xFFFFFFFFu, seg, d);
+      const bool same = lane + d < 32 && os == seg;
+      if (same) acc = dadd(acc, df{oh, ol});
+      if (!__any_sync(0xFFFFFFFFu, same)) break;
+    }
+    if (!((heads >> lane) & 1u)) bin = -1;
+  }
+  if (bin >= 0 && bin <= kmax) atomicAdd(hist + bin, df2d_any(acc.hi, acc.lo));
+}
+
 // Rows r_first, r_first + r_step, ... below r_end of field `field`, one warp
 // per row; hist_all holds one histogram of kmax + 1 bins per warp (zeroed by
 // the caller).  Each lane takes a run of consecutive modes, whose bins change
 // by at most one from mode to mode, adds them up in double-float and adds the
-// sum to its warp's histogram when the bin changes.  Lanes are a run apart, so
-// they rarely meet in a bin.  (A segmented reduction over 32 adjacent modes
-// took five rounds of three shuffles and a double-float add per mode and as
-// many histogram additions, each with two conversions on the binary64 pipe:
-// 256^3 STRIDE1 spectrum 118 us, 69 us now; with the conversions alone it is 118
-// again.)
+// sum to its warp's histogram when the bin changes; the last sums of all lanes
+// go through flush_lanes.  (A segmented reduction over 32 adjacent modes took
+// five rounds of three shuffles and a double-float add per mode and as many
+// histogram additions, each with two conversions on the binary64 pipe: 256^3
+// STRIDE1 spectrum 118 us, 70 us now; with the conversions alone it is 118 again.)
 constexpr int kSpecRun = 8;
 template <class P, bool CG>
 P3G_D void spectrum_rows(const SpecParams& prm, double* hist_all, int r_first, int r_end, int r_step, int field) {
@@ -117,7 +143,7 @@ P3G_D void spectrum_rows(const SpecParams& prm, double* hist_all, int r_first, i
           acc = dadd(acc, w);
         }
       }
-      flush();
+      flush_lanes(hist, prm.kmax, bin, acc);
     }
   }
 }

@@ -88,3 +88,26 @@ def test_spectrum_of_a_small_field(torch_cuda, amplitude, form):
     plan.close()
     want = orc.shell_spectrum(b.cpu().numpy(), n, n, n)
     assert orc.normalised_linf(e.cpu().numpy(), want) <= REL
+
+
+@pytest.mark.parametrize("stride1", [False, True])
+@pytest.mark.parametrize("precision", ["f64", "f32"])
+@pytest.mark.parametrize("flags", ["0", "K2", "HERMITIAN", "both"])
+@pytest.mark.parametrize("grid", [(256, 9, 10), (257, 8, 7), (600, 7, 9), (9, 8, 256), (10, 9, 257), (7, 6, 600), (512, 5, 34),
+                                  (34, 512, 6), (2, 40, 30), (2, 3, 2)], ids=lambda s: "x".join(map(str, s)))
+def test_long_rows_and_shared_bins(torch_cuda, grid, flags, precision, stride1):
+    """Rows of more modes than a warp takes at once, full runs per lane, and rows
+    along which the bin hardly changes (all lanes end in it)."""
+    import p3dfft_gb300 as pg
+    nx, ny, nz = grid
+    b = _modes((nz, ny, nx // 2 + 1), precision, 17, 1.0)
+    if stride1:
+        b = np.ascontiguousarray(b.transpose(2, 1, 0))
+    plan = pg.Plan(nx, ny, nz, precision=pg.F64 if precision == "f64" else pg.F32,
+                   layout=pg.LAYOUT_STRIDE1 if stride1 else pg.LAYOUT_XYZ)
+    t = torch_cuda.from_numpy(b).to("cuda", torch_cuda.complex128 if precision == "f64" else torch_cuda.complex64)
+    k2, herm = flags in ("K2", "both"), flags in ("HERMITIAN", "both")
+    got = plan.spectrum(t, flags=(pg.SPEC_K2 if k2 else 0) | (pg.SPEC_HERMITIAN if herm else 0)).cpu().numpy()
+    plan.close()
+    want = orc.shell_spectrum(b, nx, ny, nz, stride1=stride1, k2_weight=k2, hermitian=herm)
+    assert np.all(np.abs(got - want) <= REL * want + 2.0 ** -147 * b.size)
