@@ -368,31 +368,88 @@ static bool size_tile(AxisPlan& ap, int n, int lines_avail, bool f64, int max_m 
 // Strided pipelined kernel (k_strided_pipe): one CTA per SM of g groups of tg
 // threads, each group on tiles of M columns, and a ring of nbuf buffers (1 KB
 // aligned), the axis's twiddles and the buffers' mbarriers in shared memory.
-// X columns and O1 row sets are the pass's extents; tstore: the tiles leave by
-// thread stores (binary32 user rows); far_rows: a line's points lie 3 MB or
-// more apart in the pass's input or output.
+// X columns and O1 row sets are the pass's extents.
 //
 // The stage plan (wide, or narrow with half the points per thread), the tile
 // width M and the groups are those with the least estimate of
 //   (tiles per SM) x (points per tile, idle lanes included) x (clocks per
 //   point) / (row efficiency x overlap) + latency of one tile,
-// row efficiency being that of the tile's row segments in memory: 32-byte
-// segments ran the 1024-point binary32 Y pass at 4.0 ms against 1.95 ms with
-// 64 bytes.  Fewer than 12 busy warps or a single group leave the FMA pipes
-// idle through the tiles' exchanges (1024^3 binary64 Y: 6.5 ms with one
-// group of 256 threads, 5.3 ms with groups).  The latency term matters when the
-// grid has fewer tiles than the GPU has groups: half the points per thread
-// halve the length of a thread's serial chain.
+// row efficiency being that of the tile's row segments in memory.  Too few busy
+// warps or a single group leave the FMA pipes idle through the tiles' exchanges
+// (1024^3 binary64 Y: 6.5 ms with one group of 256 threads, 5.3 ms with
+// groups).  The latency term matters when the grid has fewer tiles than the GPU
+// has groups: half the points per thread halve the length of a thread's serial
+// chain.
+struct StridedModel {
+  double rows[6];    // efficiency of row segments of 8, 16, 32, 64, 128, 256 bytes or more
+  double warps;      // busy warps per SM that keep the pipes busy
+  double one_group;  // overlap of a single group
+  double full;       // clocks per point of the unguarded form against the others
+  double small;      // and of half the points per thread
+  double latency;    // clocks of one tile per point of a thread and stage
+};
+constexpr StridedModel kStridedF64 = {{0.25, 0.25, 0.45, 0.97, 1.0, 1.0}, 12, 0.8, 1.0, 1.0, 100};
+// binary32, fitted to the times of every tile width, group count and stage plan
+// of 33 lengths from 64 to 4096 on Y and Z (4000 timed shapes; the choices are
+// within 3 % of the fastest shape in the mean).  Rows of 32 bytes cost little
+// beside more groups of a long line: 1000-point Y of 256 x 1000 x 512, M = 8 in
+// one group 0.41 ms, M = 4 in two 0.38; narrower ones are ruinous in DRAM
+// (1536-point Y of 256 x 1536 x 512: 1.97 ms with M = 1, 0.67 with M = 4) and
+// milder where the whole pass stays in the L2 cache, as half the points per
+// thread are worth more there (80-point Y of 64 x 80 x 2048: 54 us with 32
+// points, 42 with 16; of 256 x 80 x 8192: 339 and 337).  Thread stores of user
+// rows split their first and last sector, so they want wider tiles; those of
+// STRIDE1 (points adjacent) want more threads (96 points of 256 x 8192 x 96:
+// 0.83 ms with 32 points, 0.72 with 16).  Where a line's points lie 1.5 MB apart,
+// every row of a tile is in a memory page of its own and rows of 32 bytes are
+// ruinous too (800^3 Z, 2.6 MB: M = 8 1.83 ms, M = 4 3.1; 1 MB apart: equal).
+constexpr StridedModel kStridedF32 = {{0.08, 0.44, 0.92, 0.97, 1.0, 1.0}, 14, 0.85, 0.9, 1.3, 50};
+constexpr StridedModel kStridedF32User = {{0.08, 0.41, 0.85, 0.95, 1.0, 1.0}, 14, 0.85, 0.9, 1.3, 50};
+constexpr StridedModel kStridedF32Stride1 = {{0.08, 0.44, 0.92, 0.97, 1.0, 1.0}, 14, 0.85, 0.9, 0.95, 50};
+constexpr StridedModel kStridedF32Apart = {{0.08, 0.25, 0.45, 0.9, 1.0, 1.0}, 14, 0.85, 0.9, 1.3, 50};
+constexpr StridedModel kStridedF32L2 = {{0.08, 0.55, 0.95, 0.97, 1.0, 1.0}, 14, 0.85, 0.9, 1.05, 50};
+static const StridedModel& strided_model(const TileExtents& e, bool in_l2) {
+  if (e.f64) return kStridedF64;
+  if (in_l2) return kStridedF32L2;
+  if (e.stride1) return kStridedF32Stride1;
+  if (e.row_bytes >= 3 << 19) return kStridedF32Apart;
+  return e.tstore ? kStridedF32User : kStridedF32;
+}
+// Half the points per thread (16 of 32) in passes of more tiles than groups: for
+// mixed radices whose largest fills 12 to 16 of a thread's 16 points.  The
+// unguarded powers of two are faster with 32 (256-point Y of 512 x 256 x 512:
+// 0.104 against 0.124 ms), and a 10 leaves 6 of 16 idle and a 9 takes 18 (900-
+// point Y of 256 x 900 x 128: 0.100 against 0.140 ms).
+static bool small_form(bool f64, const StagePlan& sp, bool pow2, int rmax) {
+  bool nine = false;
+  for (int i = 0; i < sp.nstages; ++i) nine = nine || sp.radix[i] == 9;
+  return !f64 && !pow2 && !nine && 16 / rmax * rmax >= 12;
+}
+constexpr double kL2Bytes = 128 << 20;
+
 static TileShape size_strided(const AxisPlan& ap, long long nv) {
   TileShape best_shape;
   if (ap.sp.nstages < 1 || ap.sp.has_generic || ap.n < 2) return best_shape;
-  const bool f64 = ap.ext.f64, tstore = ap.ext.tstore, far_rows = ap.ext.far_rows;
+  const bool f64 = ap.ext.f64, tstore = ap.ext.tstore, far_rows = ap.ext.row_bytes >= 3 << 20;
   const long long X = ap.ext.cols, O1 = ap.ext.rows * nv;
   const int max_m = ap.ext.max_m, sm_count = ap.ext.sm_count;
   const size_t esize = f64 ? 16 : 8;
   const int Emax = f64 ? TileElems<PathF64>::value : TileElems<PathF32>::value;
   const int n = ap.n;
   const size_t room = 227 * 1024;
+  const bool in_l2 = 2.0 * esize * n * X * O1 <= kL2Bytes;  // the pass's input and output
+  const StridedModel& md = strided_model(ap.ext, in_l2);
+  // binary32 FULL passes of 256 points or more that store user rows by threads
+  // run half the groups with twice the registers where the data comes from
+  // DRAM: at 128 the spilled words and the stores share what is left of the L1
+  // (1024-point Z forward 5.4 ms against 2.5 ms; 512-point of 256 x 1024 x 512
+  // 0.31 against 0.29 ms, but 78 against 67 us of 64 x 256 x 512, in the L2
+  // cache).  So do those with far rows of more than 512 points, where every row
+  // of a tile is in a memory page of its own and groups that drift apart spread
+  // over more pages at a time (Y of 1024^3, 4.2 MB apart: 1.95 ms with two
+  // groups, 1.81 ms with one; 256 points of 1024 x 256 x 2048: 0.73 ms with four
+  // groups, 0.95 with two)
+  const bool wide_regs = !f64 && ((far_rows && n > 512) || (tstore && !in_l2 && n >= 256));
   const int wide_index = ap.spw_index;
   double best = 1e300;
   for (int narrow = wide_index >= 0 ? 0 : 1; narrow < (ap.fixed_plan && wide_index >= 0 ? 1 : 2); ++narrow) {
@@ -408,16 +465,8 @@ static TileShape size_strided(const AxisPlan& ap, long long nv) {
       for (int M = 1; M <= max_m && M < 2 * X; M *= 2) {
         const int tg = stage_threads(sp, M, E);
         const bool full = pow2 && (long long)M * n == (long long)tg * E && E == Emax;
-        // binary32 FULL passes of 512 points or more that store by threads run
-        // one group with twice the registers: at 128 the spilled words and the
-        // stores share what is left of the L1 (1024-point Z forward 5.4 ms against
-        // 2.5 ms; 256 points: 0.043 against 0.049 ms the other way).  So do
-        // those with far rows, where every row of a tile is in a memory page
-        // of its own and groups that drift apart spread over more pages at a
-        // time (Y of 1024^3, 4.2 MB apart: 1.95 ms with two groups, 1.81 ms
-        // with one; of 768 x 1024 x 540, 1.7 MB apart: 0.59 against 0.73 ms)
         const TileMode mode =
-            E < Emax ? kTileSmall : (!full ? kTileGeneral : (!f64 && ((tstore && n >= 512) || far_rows) ? kTileFullWide : kTileFull));
+            E < Emax ? kTileSmall : (!full ? kTileGeneral : (wide_regs ? kTileFullWide : kTileFull));
         const int max_threads = tile_max_threads(mode, f64, false);
         const size_t buf = ((size_t)M * n * esize + 1023) / 1024 * 1024;
         if (tg > 512 || fixed + 2 * buf > room) break;
@@ -428,14 +477,15 @@ static TileShape size_strided(const AxisPlan& ap, long long nv) {
         // groups: as many as the threads, one spare buffer and the tiles allow
         const int g = (int)std::max(
             1.0, std::min({(double)(max_threads / tg), (double)kMaxGroups, (double)(fit - 1), per_sm}));
-        // half the points per thread: only where every tile has a group of its own
-        if (E < Emax && per_sm > g) continue;
+        // half the points per thread: where every tile has a group of its own, or small_form
+        if (E < Emax && per_sm > g && !small_form(f64, sp, pow2, rmax)) continue;
         const size_t row = M * esize;
-        const double rows = row >= 128 ? 1.0 : (row >= 64 ? 0.97 : (row >= 32 ? 0.45 : 0.25));
+        const double rows = md.rows[row >= 256 ? 5 : ilog2((int)row) - 3];
         const double warps = (mode == kTileFullWide ? 1.5 : 1.0) * g * tg / 32;
-        const double overlap = std::min(1.0, warps / 12) * (g >= 2 || mode == kTileFullWide ? 1.0 : 0.8);
-        const double clocks = (f64 ? 1.0 : 0.35) * sp.nstages;
-        const double t = per_sm * tg * E * clocks / (rows * overlap) + 100.0 * E * sp.nstages / (f64 ? 1 : 2);
+        const double overlap = std::min(1.0, warps / md.warps) * (g >= 2 || mode == kTileFullWide ? 1.0 : md.one_group);
+        const double clocks = (f64 ? 1.0 : 0.35) * sp.nstages *
+                              (mode == kTileSmall ? md.small : (mode == kTileGeneral ? 1.0 : md.full));
+        const double t = per_sm * tg * E * clocks / (rows * overlap) + md.latency * E * sp.nstages;
         if (t < best * 0.999) {
           best = t;
           TileShape& o = best_shape;
@@ -448,11 +498,14 @@ static TileShape size_strided(const AxisPlan& ap, long long nv) {
           o.threads = g * tg;
           // buffers beyond the groups (loads in flight): two, one where the
           // tiles leave by threads (binary32 512^3 Y: 0.19 ms with two, 0.26
-          // with one; 540-point binary32 Z: 1.42 with two, 1.34 with one), and
-          // twice as many for the small tiles of short binary32 lines (256^3 Y:
+          // with one; 540-point binary32 Z: 1.42 with two, 1.34 with one) or
+          // one or two groups hold a guarded binary32 plan (640-point Y of
+          // 256 x 640 x 1024: 0.45 ms with two, 0.38 with one), and twice as
+          // many for the small tiles of short binary32 lines (256^3 Y:
           // 0.046 -> 0.040 ms with four, Z 0.051 -> 0.049 with two)
           const bool small_tile = !f64 && buf <= (tstore ? 24 : 16) * 1024;
-          o.nbuf = std::min(fit, g + (tstore ? 1 : 2) * (small_tile ? 2 : 1));
+          const bool one = tstore || (!f64 && mode == kTileGeneral && g <= 2);
+          o.nbuf = std::min(fit, g + (one ? 1 : 2) * (small_tile ? 2 : 1));
           o.buf_elems = (int)(buf / esize);
           o.smem = fixed + o.nbuf * buf;
           o.fam = sp.fam;
@@ -470,7 +523,12 @@ static TileShape size_strided(const AxisPlan& ap, long long nv) {
 // X pass kernels (k_x_pipe): as size_strided; a tile is M line pairs of n
 // points (line stride ls in the padded layout) or their raw lines, whichever
 // takes more.  Lines are contiguous, so the smallest tile of two warps or more
-// is taken: up to eight groups per SM.
+// is taken: up to eight groups per SM.  Half the points per thread is for
+// grids where every tile has a group of its own, and on binary32 for passes of
+// at most kXSmallBytes, which the L2 cache largely holds: c2r + r2c of 80 x 512
+// x 512 0.158 against 0.177 ms, of 320 x 256 x 256 0.168 against 0.186, but of
+// 400 x 256 x 256 0.224 against 0.210 and of 640 x 512 x 512 1.15 against 1.03.
+constexpr double kXSmallBytes = 192 << 20;
 static TileShape size_x(const AxisPlan& ap, long long nv) {
   TileShape best_shape;
   if (ap.sp.nstages < 1 || ap.sp.has_generic || ap.n < 2) return best_shape;
@@ -481,6 +539,7 @@ static TileShape size_x(const AxisPlan& ap, long long nv) {
   const int Emax = f64 ? TileElems<PathF64>::value : TileElems<PathF32>::value;
   const int n = ap.n;
   const size_t room = 227 * 1024;
+  const bool small_ok = !f64 && 2.0 * esize * n * pairs * nv <= kXSmallBytes;  // real lines and modes
   const int wide_index = ap.spw_index;
   double best = 1e300;
   for (int narrow = wide_index >= 0 ? 0 : 1; narrow < (ap.fixed_plan && wide_index >= 0 ? 1 : 2); ++narrow) {
@@ -508,10 +567,10 @@ static TileShape size_x(const AxisPlan& ap, long long nv) {
         const double per_sm = std::ceil((double)((pairs + M - 1) / M) * nv / sm_count);
         const int g = (int)std::max(
             1.0, std::min({(double)(max_threads / tg), (double)kMaxGroups, (double)(fit - 1), per_sm}));
-        if (E < Emax && per_sm > g) continue;  // every tile has a group of its own
+        if (E < Emax && per_sm > g && !(small_ok && per_sm >= 4 * g && small_form(f64, sp, pow2, rmax))) continue;
         const double warps = (mode == kTileFullWide ? 1.3 : 1.0) * g * tg / 32;
         const double overlap = std::min(1.0, warps / 12) * (g >= 2 ? 1.0 : 0.8) * (tg >= 64 ? 1.0 : 0.9);
-        const double clocks = (f64 ? 1.0 : 0.35) * sp.nstages;
+        const double clocks = (f64 ? 1.0 : 0.35) * sp.nstages * (E < Emax && per_sm > g ? 0.85 : 1.0);
         const double t = per_sm * tg * E * clocks / overlap + 100.0 * E * sp.nstages / (f64 ? 1 : 2);
         if (t < best * 0.999) {
           best = t;
@@ -1781,21 +1840,24 @@ int p3g_plan_create_tuned(p3g_plan* out, int nx, int ny, int nz, int nxc, int ny
     if (!size_tile(p->ax_z[3], nz, p->nxhpc, f64, strided_max_m)) p->z_ok[3] = false;
   }
   if (!p->z_ok[0] && !p->z_ok[1] && !p->z_ok[3]) return bad("z length " + std::to_string(nz) + " is too long");
-  p->ax_x.ext = TileExtents{true, f64, false, false, p->xpairs(), 1, x_max_m, p->sm_count};
+  p->ax_x.ext = TileExtents{true, f64, false, false, 0, p->xpairs(), 1, x_max_m, p->sm_count};
   p->ax_x.pipe_ok = tile_shape(p->ax_x, 1).ok;
   const int yx = p->nxhpc;
-  const bool far_y = (long long)nz * p->pitch * p->esize() >= 3 << 20;  // the Y/Z workspace's row stride along y
-  auto size_s = [&](AxisPlan& ap, int X, long long O1, bool tstore, bool far_rows) {
-    ap.ext = TileExtents{false, f64, tstore, far_rows, X, O1, strided_max_m, p->sm_count};
+  // bytes between the points of a line: the Y/Z workspace's rows, and the user's planes
+  const long long y_rows = (long long)nz * p->pitch * p->esize();
+  const bool s1 = layout == P3G_LAYOUT_STRIDE1;
+  const long long z_rows = s1 ? 0 : (long long)nyc * p->nxhpc * p->esize();
+  auto size_s = [&](AxisPlan& ap, int X, long long O1, bool user, long long row_bytes) {
+    ap.ext = TileExtents{false, f64, user && !f64, user && s1, row_bytes, X, O1, strided_max_m, p->sm_count};
     ap.pipe_ok = tile_shape(ap, 1).ok;
   };
-  size_s(p->ax_y, yx, nz, false, far_y);
+  size_s(p->ax_y, yx, nz, false, y_rows);
   for (int i = 0; i < 2; ++i) {
-    if (p->four_y) size_s(p->ly[i], yx, p->ly[1 - i].n, false, far_y);
-    if (p->four_z) size_s(p->lz[i], yx, p->lz[1 - i].n, !f64, false);
+    if (p->four_y) size_s(p->ly[i], yx, p->ly[1 - i].n, false, y_rows);
+    if (p->four_z) size_s(p->lz[i], yx, p->lz[1 - i].n, true, 0);
   }
   for (int i = 0; i < 4; ++i)
-    if (p->z_ok[i]) size_s(p->ax_z[i], yx, nyc, !f64, false);
+    if (p->z_ok[i]) size_s(p->ax_z[i], yx, nyc, true, z_rows);
   {
     const char* e = std::getenv("P3G_NO_PIPE");
     p->use_pipe = !(e && *e && *e != '0');

@@ -27,9 +27,12 @@ struct TileShape {
 };
 
 // What a pass's tiles cover per field: cols columns (X passes: line pairs) of
-// rows row sets.
+// rows row sets.  tstore: the tiles leave by thread stores (binary32 user rows);
+// stride1: Z passes of the STRIDE1 layout; row_bytes: how far a line's points lie
+// apart in the pass's input or output, whichever is farther.
 struct TileExtents {
-  bool x_pass = false, f64 = false, tstore = false, far_rows = false;
+  bool x_pass = false, f64 = false, tstore = false, stride1 = false;
+  long long row_bytes = 0;
   long long cols = 1, rows = 1;
   int max_m = 1, sm_count = 1;
 };
