@@ -933,9 +933,11 @@ int run_x_c2r(p3g_plan p, XParams& x, int nv, cudaStream_t st, int max_sms = 0) 
     xp.c.err = p->d_err;
     {
       // the modes of a line arrive by one bulk copy, rounded up to 16 bytes,
-      // which the line pitch and the raw stride hold
+      // which the line pitch and the raw stride hold; short lines by cp.async:
+      // one thread issues a tile's copies, and 64 of 264 bytes cost it more than
+      // the group's own (64-point binary32 X c2r of 16 x 64^3: 33 against 27 us)
       const long long es = (long long)sizeof(typename P::W);
-      xp.bulk = (x.in_line * es) % 16 == 0 && (x.in_field * es) % 16 == 0 &&
+      xp.bulk = x.nkeep * es >= 512 && (x.in_line * es) % 16 == 0 && (x.in_field * es) % 16 == 0 &&
                 (long long)x.in_line * es >= ((x.nkeep * es + 15) / 16) * 16 && aligned_to(x.in, 16) &&
                 device_memory(x.in);
     }

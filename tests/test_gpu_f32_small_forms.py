@@ -1,8 +1,9 @@
-"""Binary32 passes with half the points per thread and several tiles per group.
+"""Binary32 passes with half the points per thread and several tiles per group,
+and X c2r passes whose short lines arrive by cp.async.
 
 Lengths whose largest radix fills 16 points on each axis, with enough tiles
 that the ring of buffers wraps; the narrowest and the long rows of the strided
-tiles.
+tiles; lines of a few modes, pruned ones and an odd number of them.
 
 Tolerances: the transform's bounds, normalised L-inf 1e-12 (binary64) and
 relative L2 1e-6 (binary32).
@@ -57,3 +58,12 @@ def test_strided_small_forms(shape, stride1):
                          ids=lambda s: "x".join(map(str, s)))
 def test_x_small_forms(shape):
     _check(shape, "f32")
+
+
+@pytest.mark.parametrize("precision", ["f64", "f32"])
+@pytest.mark.parametrize("shape", [(16, 33, 31), (24, 65, 40), (48, 64, 60), (60, 40, 41), (64, 63, 65), (64, 64, 64),
+                                   (62, 17, 19), (61, 17, 19), (126, 20, 21), (128, 20, 21),
+                                   (96, 30, 31, 30, 30, 31), (192, 20, 22, 90, 14, 16)],
+                         ids=lambda s: "x".join(map(str, s)))
+def test_short_c2r_lines(shape, precision):
+    _check(shape, precision)
