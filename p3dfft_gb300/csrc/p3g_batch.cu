@@ -86,18 +86,34 @@ size_t fit_s(SParams& s, const AxisPlan& ap, size_t esize, int threads) {
   return (size_t)s.M * s.N * esize * (ap.sp.has_generic ? 2 : 1);
 }
 
+// c67: a plan of the batch has a 6- or 7-point stage (binary64 has the one kernel)
+template <class P, int T>
+cudaError_t batch_config_c(bool c67, size_t smem, int& per_sm, size_t& max_dyn) {
+  if constexpr (!P::kF64) {
+    if (!c67) return batch_config_t<P, T, false>(smem, per_sm, max_dyn);
+  }
+  return batch_config_t<P, T, true>(smem, per_sm, max_dyn);
+}
 template <class P>
-cudaError_t batch_config(size_t smem, int threads, int& per_sm, size_t& max_dyn) {
-  return threads == kBatchThreadsSmall ? batch_config_t<P, kBatchThreadsSmall>(smem, per_sm, max_dyn)
-                                       : batch_config_t<P, kBatchThreadsLarge>(smem, per_sm, max_dyn);
+cudaError_t batch_config(bool c67, size_t smem, int threads, int& per_sm, size_t& max_dyn) {
+  return threads == kBatchThreadsSmall ? batch_config_c<P, kBatchThreadsSmall>(c67, smem, per_sm, max_dyn)
+                                       : batch_config_c<P, kBatchThreadsLarge>(c67, smem, per_sm, max_dyn);
 }
 
+template <class P, int T>
+cudaError_t batch_launch_c(bool c67, const BatchPass* d_pass, int npass, int nitems, int* ctl, int buf_elems, int grid,
+                           size_t smem, cudaStream_t st) {
+  if constexpr (!P::kF64) {
+    if (!c67) return batch_launch_t<P, T, false>(d_pass, npass, nitems, ctl, buf_elems, grid, smem, st);
+  }
+  return batch_launch_t<P, T, true>(d_pass, npass, nitems, ctl, buf_elems, grid, smem, st);
+}
 template <class P>
-cudaError_t batch_launch(const BatchPass* d_pass, int npass, int nitems, int* ctl, int buf_elems, int grid,
+cudaError_t batch_launch(bool c67, const BatchPass* d_pass, int npass, int nitems, int* ctl, int buf_elems, int grid,
                          int threads, size_t smem, cudaStream_t st) {
   return threads == kBatchThreadsSmall
-             ? batch_launch_t<P, kBatchThreadsSmall>(d_pass, npass, nitems, ctl, buf_elems, grid, smem, st)
-             : batch_launch_t<P, kBatchThreadsLarge>(d_pass, npass, nitems, ctl, buf_elems, grid, smem, st);
+             ? batch_launch_c<P, kBatchThreadsSmall>(c67, d_pass, npass, nitems, ctl, buf_elems, grid, smem, st)
+             : batch_launch_c<P, kBatchThreadsLarge>(c67, d_pass, npass, nitems, ctl, buf_elems, grid, smem, st);
 }
 
 size_t round256(size_t b) { return (b + 255) / 256 * 256; }
@@ -155,6 +171,7 @@ struct p3g_batch_s {
   size_t smem = 0;
   int buf_elems = 0;
   int threads = 0, grid = 0;
+  bool c67 = true;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   long long launches = 0;
@@ -396,10 +413,15 @@ int p3g_batch_set_jobs(p3g_batch b, int njobs, const p3g_job* jobs, int window) 
       }
   }
   if (items > 0x7FFFFFF0LL) return fail(P3G_E_UNSUPPORTED, "too many work items");
+  bool c67 = false;
+  for (int j = 0; j < njobs; ++j) {
+    const p3g_plan p = jobs[j].plan;
+    c67 = c67 || has_c67(p->ax_x.sp.fam) || has_c67(p->ax_y.sp.fam) || has_c67(p->ax_z[0].sp.fam);
+  }
   int per_sm = 1;
   size_t max_dyn = 0;
-  cudaError_t e = f64 ? batch_config<PathF64>(smem, threads, per_sm, max_dyn)
-                      : batch_config<PathF32>(smem, threads, per_sm, max_dyn);
+  cudaError_t e = f64 ? batch_config<PathF64>(c67, smem, threads, per_sm, max_dyn)
+                      : batch_config<PathF32>(c67, smem, threads, per_sm, max_dyn);
   if (e != cudaSuccess && smem > max_dyn && max_dyn > 0)
     return fail(P3G_E_UNSUPPORTED, "a job's tile needs " + std::to_string(smem) + " bytes of shared memory, above " +
                                        std::to_string(max_dyn));
@@ -472,6 +494,7 @@ int p3g_batch_set_jobs(p3g_batch b, int njobs, const p3g_job* jobs, int window) 
   b->smem = smem;
   b->buf_elems = (int)buf_elems;
   b->threads = threads;
+  b->c67 = c67;
   const long long slots = (long long)b->sm_count * per_sm;
   b->grid = (int)std::max(1LL, std::min(slots, items));
   return P3G_OK;
@@ -498,9 +521,9 @@ static int batch_enqueue(p3g_batch b, cudaStream_t st) {
   cudaError_t e = cudaMemsetAsync(b->d_ctl, 0, ctl_bytes, st);
   if (e != cudaSuccess) return fail(P3G_E_CUDA, std::string("batch clear: ") + cudaGetErrorString(e));
   e = b->prec == P3G_F64
-          ? batch_launch<PathF64>(b->d_pass, b->npass, b->nitems, b->d_ctl, b->buf_elems, b->grid, b->threads,
+          ? batch_launch<PathF64>(b->c67, b->d_pass, b->npass, b->nitems, b->d_ctl, b->buf_elems, b->grid, b->threads,
                                   b->smem, st)
-          : batch_launch<PathF32>(b->d_pass, b->npass, b->nitems, b->d_ctl, b->buf_elems, b->grid, b->threads,
+          : batch_launch<PathF32>(b->c67, b->d_pass, b->npass, b->nitems, b->d_ctl, b->buf_elems, b->grid, b->threads,
                                   b->smem, st);
   if (e != cudaSuccess) return fail(P3G_E_CUDA, std::string("batch launch: ") + cudaGetErrorString(e));
   e = cudaMemcpyAsync(b->h_err, b->d_ctl + 1, sizeof(int), cudaMemcpyDeviceToHost, st);

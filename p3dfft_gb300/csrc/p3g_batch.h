@@ -47,10 +47,11 @@ __host__ __device__ constexpr int batch_pipe_elems() { return F64 ? 8 : 16; }
 // instantiated in the p3g_batch_<path>_<threads>.cu units.  batch_config_t
 // opts the kernel in to the largest dynamic shared memory the current device
 // allows next to its static shared variables and reads the occupancy for a
-// tile of smem bytes.
-template <class P, int T>
+// tile of smem bytes.  C67: the 6- and 7-point codelets are compiled in
+// (has_c67), on binary64 always.
+template <class P, int T, bool C67>
 cudaError_t batch_config_t(size_t smem, int& per_sm, size_t& max_dyn);
-template <class P, int T>
+template <class P, int T, bool C67>
 cudaError_t batch_launch_t(const BatchPass* d_pass, int npass, int nitems, int* ctl, int buf_elems, int grid,
                            size_t smem, cudaStream_t st);
 

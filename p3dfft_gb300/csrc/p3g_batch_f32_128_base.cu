@@ -1,0 +1,7 @@
+// Batch kernel for the F32 path with 128-thread CTAs,
+// plans without 6- and 7-point stages.
+#include "p3g_batch_kernels.cuh"
+
+namespace p3g {
+P3G_BATCH_INSTANTIATE(PathF32, 128, false)
+}  // namespace p3g

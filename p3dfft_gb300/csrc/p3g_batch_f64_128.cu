@@ -2,5 +2,5 @@
 #include "p3g_batch_kernels.cuh"
 
 namespace p3g {
-P3G_BATCH_INSTANTIATE(PathF64, 128)
+P3G_BATCH_INSTANTIATE(PathF64, 128, true)
 }  // namespace p3g

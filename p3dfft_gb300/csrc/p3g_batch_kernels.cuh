@@ -67,7 +67,7 @@ P3G_D void batch_issue(const BatchPass& bp, int tile, typename P::W* buf) {
 }
 
 // Transform and store a double-buffered item whose tile is in buf.
-template <class P>
+template <class P, bool C67>
 P3G_D void batch_process_pipe(const BatchPass& bp, int tile, typename P::W* buf) {
   constexpr int E = batch_pipe_elems<P::kF64>();
   switch (bp.kind) {
@@ -75,14 +75,14 @@ P3G_D void batch_process_pipe(const BatchPass& bp, int tile, typename P::W* buf)
       const int k = range_k(bp.x.range);
       uint32_t amax = 0;
       Tile<P> t{buf, nullptr, bp.x.M, bp.x.log2m, bp.x.LS, 1, bp.x.ps, k, &amax};
-      cta_fft<P, -1, E, kLineMajor, kRawR2C>(t, bp.sp, bp.tw);
+      cta_fft<P, C67, -1, E, kLineMajor, kRawR2C>(t, bp.sp, bp.tw);
       xr2c_store<P>(bp.x, buf, tile * bp.x.M, 0, k);
       range_flush(bp.x.range, amax);
       break;
     }
     case kBXc2r: {  // the first FFT stage reads the raw half spectra
       Tile<P> t{buf, nullptr, bp.x.M, bp.x.log2m, bp.x.LS, 1, bp.x.ps};
-      cta_fft<P, 1, E, kLineMajor, kRawC2R>(t, bp.sp, bp.tw);
+      cta_fft<P, C67, 1, E, kLineMajor, kRawC2R>(t, bp.sp, bp.tw);
       xc2r_store<P>(bp.x, buf, tile * bp.x.M, 0, range_k(bp.x.range));
       break;
     }
@@ -92,8 +92,8 @@ P3G_D void batch_process_pipe(const BatchPass& bp, int tile, typename P::W* buf)
       uint32_t amax = 0;
       strided_fix<P>(bp.s, false, buf, k, amax);
       Tile<P> t{buf, nullptr, bp.s.M, bp.s.log2m, 1, bp.s.M};
-      if (bp.kind == kBFwd) cta_fft<P, -1, E, kPointMajor>(t, bp.sp, bp.tw);
-      else cta_fft<P, 1, E, kPointMajor>(t, bp.sp, bp.tw);
+      if (bp.kind == kBFwd) cta_fft<P, C67, -1, E, kPointMajor>(t, bp.sp, bp.tw);
+      else cta_fft<P, C67, 1, E, kPointMajor>(t, bp.sp, bp.tw);
       strided_store<P>(bp.s, buf, tile - o1 * bp.s.xtiles, o1, 0, k);
       range_flush(bp.s.range, amax);
       break;
@@ -104,24 +104,24 @@ P3G_D void batch_process_pipe(const BatchPass& bp, int tile, typename P::W* buf)
 // Single-tile items (plans with generic prime stages, which need a scratch
 // tile), spectrum chunks and histogram clears; sm spans both buffers.  Kept
 // out of line so that its registers do not weigh on the double-buffered path.
-template <class P>
+template <class P, bool C67>
 __device__ __noinline__ void batch_process_single(const BatchPass& bp, int tile, typename P::W* sm) {
   switch (bp.kind) {
     case kBXr2c: {
       uint32_t amax = 0;
-      x_r2c_tile<P, true>(bp.x, bp.sp, bp.tw, sm, tile, 0, amax);
+      x_r2c_tile<P, true, C67>(bp.x, bp.sp, bp.tw, sm, tile, 0, amax);
       range_flush(bp.x.range, amax);
       break;
     }
     case kBFwd:
     case kBBwd: {
       uint32_t amax = 0;
-      if (bp.kind == kBFwd) strided_tile<P, -1, true>(bp.s, bp.sp, bp.tw, sm, tile, amax);
-      else strided_tile<P, 1, true>(bp.s, bp.sp, bp.tw, sm, tile, amax);
+      if (bp.kind == kBFwd) strided_tile<P, -1, true, C67>(bp.s, bp.sp, bp.tw, sm, tile, amax);
+      else strided_tile<P, 1, true, C67>(bp.s, bp.sp, bp.tw, sm, tile, amax);
       range_flush(bp.s.range, amax);
       break;
     }
-    case kBXc2r: x_c2r_tile<P, true>(bp.x, bp.sp, bp.tw, sm, tile, 0); break;
+    case kBXc2r: x_c2r_tile<P, true, C67>(bp.x, bp.sp, bp.tw, sm, tile, 0); break;
     case kBSpec: {
       double* hist = reinterpret_cast<double*>(sm);
       const int nwarps = blockDim.x >> 5;
@@ -152,7 +152,7 @@ __device__ __noinline__ void batch_process_single(const BatchPass& bp, int tile,
 // item and the start of the next, warp 1 publishes the finished item (fence +
 // counter) while thread 0 looks up the item after next, whose ticket was
 // fetched an item earlier: neither latency waits for the other.
-template <class P, int T>
+template <class P, int T, bool C67>
 __global__ void __launch_bounds__(T, batch_min_blocks<T>())
     k_batch(const BatchPass* __restrict__ passes, int npass, int nitems, int* __restrict__ ctl, int buf_elems) {
   using W = typename P::W;
@@ -215,9 +215,9 @@ __global__ void __launch_bounds__(T, batch_min_blocks<T>())
     if (pipe) {
       cp_async_wait<1>();
       __syncthreads();
-      batch_process_pipe<P>(bc, cur - bc.first, buf0 + b * buf_elems);
+      batch_process_pipe<P, C67>(bc, cur - bc.first, buf0 + b * buf_elems);
     } else {
-      batch_process_single<P>(bc, cur - bc.first, buf0);
+      batch_process_single<P, C67>(bc, cur - bc.first, buf0);
     }
     // the barrier orders every thread's stores before warp 1's gpu-scope
     // fence and counter increment (the grid-barrier pattern)
@@ -261,34 +261,34 @@ __global__ void __launch_bounds__(T, batch_min_blocks<T>())
   cp_async_wait<0>();
 }
 
-template <class P, int T>
+template <class P, int T, bool C67>
 cudaError_t batch_config_t(size_t smem, int& per_sm, size_t& max_dyn) {
   cudaFuncAttributes fa{};
   int dev = 0, optin = 0;
-  cudaError_t e = cudaFuncGetAttributes(&fa, k_batch<P, T>);
+  cudaError_t e = cudaFuncGetAttributes(&fa, k_batch<P, T, C67>);
   if (e == cudaSuccess) e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   if (e != cudaSuccess) return e;
   const size_t dyn = (size_t)optin - fa.sharedSizeBytes;
-  e = opt_in_smem((const void*)k_batch<P, T>, (int)dyn);
+  e = opt_in_smem((const void*)k_batch<P, T, C67>, (int)dyn);
   if (e != cudaSuccess) return e;
   max_dyn = dyn;
   if (smem > max_dyn) return cudaErrorInvalidValue;
   per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch<P, T>, T, smem);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch<P, T, C67>, T, smem);
   if (e == cudaSuccess && per_sm < 1) per_sm = 1;
   return e;
 }
 
-template <class P, int T>
+template <class P, int T, bool C67>
 cudaError_t batch_launch_t(const BatchPass* d_pass, int npass, int nitems, int* ctl, int buf_elems, int grid,
                            size_t smem, cudaStream_t st) {
-  k_batch<P, T><<<grid, T, smem, st>>>(d_pass, npass, nitems, ctl, buf_elems);
+  k_batch<P, T, C67><<<grid, T, smem, st>>>(d_pass, npass, nitems, ctl, buf_elems);
   return cudaGetLastError();
 }
 
-#define P3G_BATCH_INSTANTIATE(P, T)                                                                      \
-  template cudaError_t batch_config_t<P, T>(size_t, int&, size_t&);                                        \
-  template cudaError_t batch_launch_t<P, T>(const BatchPass*, int, int, int*, int, int, size_t, cudaStream_t);
+#define P3G_BATCH_INSTANTIATE(P, T, C67)                                                                  \
+  template cudaError_t batch_config_t<P, T, C67>(size_t, int&, size_t&);                                   \
+  template cudaError_t batch_launch_t<P, T, C67>(const BatchPass*, int, int, int*, int, int, size_t, cudaStream_t);
 
 }  // namespace p3g

@@ -31,6 +31,12 @@ constexpr int kElemsPerThread = 16;  // E
 constexpr int kFamilies[] = {32, 16, 8, 4, 2, 12, 10, 15, 9, 6, 3, 5, 7};
 constexpr int kNumFamilies = sizeof(kFamilies) / sizeof(kFamilies[0]);
 P3G_HD int family_count(unsigned long long fam, int i) { return (int)(fam >> (4 * i)) & 15; }
+// Plans with a 6- or 7-point stage.  The binary32 CTA-wide kernels are compiled
+// with and without these codelets: their registers and code cost every other
+// plan (24 transforms of powers of two in one launch 1.59 against 1.55 ms, 220^3
+// round trips, 20 x 11 points, 1.6 %), and generic 7-point stages are four times
+// slower than the codelet.
+P3G_HD bool has_c67(unsigned long long fam) { return family_count(fam, 9) + family_count(fam, 12) > 0; }
 
 // Most butterflies of radix r that a thread of E elements runs per stage: as
 // many as cover E elements or, where the launch can have the threads for it
@@ -462,11 +468,12 @@ __device__ __forceinline__ void run_family(const Tile<P, TH>& t, const float4* _
 // the live ranges of every codelet at once and spill.  FULL: a plan of
 // power-of-two radices whose stages all fill every thread; only those
 // families are compiled, without guards.
+// C67: the 6- and 7-point codelets are compiled in.
 // The first stage's twiddles start at tw[off].  E = elements each thread holds
 // per stage.  LAY: the tile layout when the caller knows it (kPointMajor, kLineMajor).  RAW: the
 // tile still holds the raw line pairs of an X r2c or c2r tile (kRawR2C,
 // kRawC2R; plans without generic stages only), read by the first stage.
-template <class P, int DIR, int E, int LAY, int RAW, int MAXR, bool FULL, class TH>
+template <class P, int DIR, int E, int LAY, int RAW, int MAXR, bool FULL, bool C67, class TH>
 __device__ __forceinline__ void run_families(const Tile<P, TH>& t, const float4* __restrict__ tw, int N,
                                              unsigned long long fam, int off) {
   int ns = 1;
@@ -482,21 +489,21 @@ __device__ __forceinline__ void run_families(const Tile<P, TH>& t, const float4*
       run_family<P, DIR, 15, E, LAY, false, RAW>(t, tw, N, family_count(fam, 7), ns, off);
       run_family<P, DIR, 9, E, LAY, false, RAW>(t, tw, N, family_count(fam, 8), ns, off);
     }
-    run_family<P, DIR, 6, E, LAY, false, RAW>(t, tw, N, family_count(fam, 9), ns, off);
+    if constexpr (C67) run_family<P, DIR, 6, E, LAY, false, RAW>(t, tw, N, family_count(fam, 9), ns, off);
     run_family<P, DIR, 3, E, LAY, false, RAW>(t, tw, N, family_count(fam, 10), ns, off);
     run_family<P, DIR, 5, E, LAY, false, RAW>(t, tw, N, family_count(fam, 11), ns, off);
-    run_family<P, DIR, 7, E, LAY, false, RAW>(t, tw, N, family_count(fam, 12), ns, off);
+    if constexpr (C67) run_family<P, DIR, 7, E, LAY, false, RAW>(t, tw, N, family_count(fam, 12), ns, off);
   }
 }
 
 // The CTA-wide form reads the plan from global memory and runs generic primes.
-template <class P, int DIR, int E = kElemsPerThread, int LAY = kAnyLayout, int RAW = kRawNone,
+template <class P, bool C67, int DIR, int E = kElemsPerThread, int LAY = kAnyLayout, int RAW = kRawNone,
           int MAXR = P::kF64 ? 8 : 16>
 __device__ __forceinline__ void cta_fft(const Tile<P>& t, const StagePlan* __restrict__ sp,
                                         const float4* __restrict__ tw) {
   const int N = __ldg(&sp->n);
   const unsigned long long fam = __ldg(&sp->fam);
-  run_families<P, DIR, E, LAY, RAW, MAXR, false>(t, tw, N, fam, __ldg(&sp->tw_off[0]));
+  run_families<P, DIR, E, LAY, RAW, MAXR, false, C67>(t, tw, N, fam, __ldg(&sp->tw_off[0]));
   if (__ldg(&sp->has_generic)) {
     int sg = 0;
     for (int i = 0; i < kNumFamilies; ++i) sg += family_count(fam, i);

@@ -173,14 +173,14 @@ cudaError_t opt_in_smem(const void* func, int bytes);
 
 // Launchers (one per path).  Return the cudaError_t of the launch.
 template <class P>
-cudaError_t launch_x_r2c(const XParams& p, const StagePlan* sp, const float4* tw, int threads, size_t smem,
-                         int nfields, cudaStream_t st);
+cudaError_t launch_x_r2c(const XParams& p, const StagePlan* sp, unsigned long long fam, const float4* tw, int threads,
+                         size_t smem, int nfields, cudaStream_t st);
 template <class P>
-cudaError_t launch_x_c2r(const XParams& p, const StagePlan* sp, const float4* tw, int threads, size_t smem,
-                         int nfields, cudaStream_t st);
+cudaError_t launch_x_c2r(const XParams& p, const StagePlan* sp, unsigned long long fam, const float4* tw, int threads,
+                         size_t smem, int nfields, cudaStream_t st);
 template <class P>
-cudaError_t launch_strided(const SParams& p, const StagePlan* sp, const float4* tw, bool forward_sign, int threads,
-                           size_t smem, int nfields, cudaStream_t st);
+cudaError_t launch_strided(const SParams& p, const StagePlan* sp, unsigned long long fam, const float4* tw,
+                           bool forward_sign, int threads, size_t smem, int nfields, cudaStream_t st);
 template <class P>
 cudaError_t launch_cheby(const ChebyParams& p, int nfields, cudaStream_t st);
 // long X lines: kind 0 pack, 1 split, 2 merge, 3 unpack (p3g_kernels_impl.cuh)

@@ -26,7 +26,7 @@ struct PathLimits<PathF32> {
 // Real lines 2p and 2p+1 form z = x1 + i x2; Z = FFT(z);
 // X1[k] = (Z[k] + conj Z[N-k]) / 2, X2[k] = -i (Z[k] - conj Z[N-k]) / 2.
 // One tile (M line pairs) of field `field`; sm = the tile's shared memory.
-template <class P, bool CG>
+template <class P, bool CG, bool C67>
 P3G_D void x_r2c_tile(const XParams& prm, const StagePlan* __restrict__ sp, const float4* __restrict__ tw,
                       typename P::W* sm, int tile, int field, uint32_t& amax) {
   const int kb = range_k(prm.range);
@@ -61,15 +61,15 @@ P3G_D void x_r2c_tile(const XParams& prm, const StagePlan* __restrict__ sp, cons
   }
   __syncthreads();
   Tile<P> t{sm, sm + M * LS, M, prm.log2m, LS, 1, ps};
-  cta_fft<P, -1, kElemsPerThread, kLineMajor>(t, sp, tw);
+  cta_fft<P, C67, -1, kElemsPerThread, kLineMajor>(t, sp, tw);
   xr2c_store<P>(prm, sm, p0, field, kb);
 }
 
-template <class P>
+template <class P, bool C67>
 __global__ void __launch_bounds__(PathLimits<P>::kMaxThreads, PathLimits<P>::kMinBlocks)
     k_x_r2c(const XParams prm, const StagePlan* __restrict__ sp, const float4* __restrict__ tw) {
   uint32_t amax = 0;
-  x_r2c_tile<P, false>(prm, sp, tw, reinterpret_cast<typename P::W*>(p3g_smem), blockIdx.x, blockIdx.y, amax);
+  x_r2c_tile<P, false, C67>(prm, sp, tw, reinterpret_cast<typename P::W*>(p3g_smem), blockIdx.x, blockIdx.y, amax);
   range_flush(prm.range, amax);
 }
 
@@ -77,7 +77,7 @@ __global__ void __launch_bounds__(PathLimits<P>::kMaxThreads, PathLimits<P>::kMi
 // Z[k] = X1[k] + i X2[k] (k <= N/2, imaginary parts of DC and Nyquist
 // dropped as FFTW's c2r does), Z[N-k] = conj X1[k] + i conj X2[k];
 // z = IFFT(Z) (unnormalised) gives x1 = Re z, x2 = Im z.
-template <class P, bool CG>
+template <class P, bool CG, bool C67>
 P3G_D void x_c2r_tile(const XParams& prm, const StagePlan* __restrict__ sp, const float4* __restrict__ tw,
                       typename P::W* sm, int tile, int field) {
   const int kb = range_k(prm.range);
@@ -108,7 +108,7 @@ P3G_D void x_c2r_tile(const XParams& prm, const StagePlan* __restrict__ sp, cons
   }
   __syncthreads();
   Tile<P> t{sm, sm + M * LS, M, prm.log2m, LS, 1, ps};
-  cta_fft<P, 1, kElemsPerThread, kLineMajor>(t, sp, tw);
+  cta_fft<P, C67, 1, kElemsPerThread, kLineMajor>(t, sp, tw);
   const float* smf = reinterpret_cast<const float*>(sm);
   constexpr int kW = sizeof(W) / sizeof(float);
   for (int e = threadIdx.x; e < 2 * M * N; e += blockDim.x) {
@@ -126,16 +126,16 @@ P3G_D void x_c2r_tile(const XParams& prm, const StagePlan* __restrict__ sp, cons
   }
 }
 
-template <class P>
+template <class P, bool C67>
 __global__ void __launch_bounds__(PathLimits<P>::kMaxThreads, PathLimits<P>::kMinBlocks)
     k_x_c2r(const XParams prm, const StagePlan* __restrict__ sp, const float4* __restrict__ tw) {
-  x_c2r_tile<P, false>(prm, sp, tw, reinterpret_cast<typename P::W*>(p3g_smem), blockIdx.x, blockIdx.y);
+  x_c2r_tile<P, false, C67>(prm, sp, tw, reinterpret_cast<typename P::W*>(p3g_smem), blockIdx.x, blockIdx.y);
 }
 
 // ------------------------------------------------------------- strided Y/Z
 
 // One tile (M columns x L rows); `bid` enumerates (x tile, o1, o2 = field).
-template <class P, int DIR, bool CG>
+template <class P, int DIR, bool CG, bool C67>
 P3G_D void strided_tile(const SParams& prm, const StagePlan* __restrict__ sp, const float4* __restrict__ tw,
                         typename P::W* sm, long long bid, uint32_t& amax) {
   const int kb = range_k(prm.range);
@@ -188,7 +188,7 @@ P3G_D void strided_tile(const SParams& prm, const StagePlan* __restrict__ sp, co
   }
   __syncthreads();
   Tile<P> t{sm, sm + M * N, M, prm.log2m, 1, M};
-  cta_fft<P, DIR, kElemsPerThread, kPointMajor>(t, sp, tw);
+  cta_fft<P, C67, DIR, kElemsPerThread, kPointMajor>(t, sp, tw);
   const bool out_rows_fast = prm.out_xs != 1;
   const FastDiv div_lo(prm.Lout);
   for (int e = threadIdx.x; e < M * prm.Lout; e += blockDim.x) {
@@ -214,11 +214,11 @@ P3G_D void strided_tile(const SParams& prm, const StagePlan* __restrict__ sp, co
   }
 }
 
-template <class P, int DIR>
+template <class P, int DIR, bool C67>
 __global__ void __launch_bounds__(PathLimits<P>::kMaxThreads, PathLimits<P>::kMinBlocks)
     k_strided(const SParams prm, const StagePlan* __restrict__ sp, const float4* __restrict__ tw) {
   uint32_t amax = 0;
-  strided_tile<P, DIR, false>(prm, sp, tw, reinterpret_cast<typename P::W*>(p3g_smem), blockIdx.x, amax);
+  strided_tile<P, DIR, false, C67>(prm, sp, tw, reinterpret_cast<typename P::W*>(p3g_smem), blockIdx.x, amax);
   range_flush(prm.range, amax);
 }
 
@@ -395,33 +395,43 @@ cudaError_t launch_x_long(int kind, const XLongParams& q, int sm_count, cudaStre
 }
 
 // ---------------------------------------------------------------- launchers
-template <class P>
-cudaError_t launch_x_r2c(const XParams& p, const StagePlan* sp, const float4* tw, int threads, size_t smem,
-                         int nfields, cudaStream_t st) {
-  cudaError_t ea = opt_in_smem((const void*)k_x_r2c<P>, 227 * 1024);
-  if (ea != cudaSuccess) return ea;
-  k_x_r2c<P><<<dim3(p.tiles, nfields), threads, smem, st>>>(p, sp, tw);
+// fam: the plan's stages (has_c67)
+template <class... Params, class... Args>
+cudaError_t launch_single(void (*kernel)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t st,
+                          const Args&... args) {
+  const cudaError_t e = opt_in_smem((const void*)kernel, 227 * 1024);
+  if (e != cudaSuccess) return e;
+  kernel<<<grid, threads, smem, st>>>(args...);
   return cudaGetLastError();
 }
 template <class P>
-cudaError_t launch_x_c2r(const XParams& p, const StagePlan* sp, const float4* tw, int threads, size_t smem,
-                         int nfields, cudaStream_t st) {
-  cudaError_t ea = opt_in_smem((const void*)k_x_c2r<P>, 227 * 1024);
-  if (ea != cudaSuccess) return ea;
-  k_x_c2r<P><<<dim3(p.tiles, nfields), threads, smem, st>>>(p, sp, tw);
-  return cudaGetLastError();
+cudaError_t launch_x_r2c(const XParams& p, const StagePlan* sp, unsigned long long fam, const float4* tw, int threads,
+                         size_t smem, int nfields, cudaStream_t st) {
+  auto kernel = k_x_r2c<P, true>;
+  if constexpr (!P::kF64) {
+    if (!has_c67(fam)) kernel = k_x_r2c<P, false>;
+  }
+  return launch_single(kernel, dim3(p.tiles, nfields), threads, smem, st, p, sp, tw);
 }
 template <class P>
-cudaError_t launch_strided(const SParams& p, const StagePlan* sp, const float4* tw, bool forward_sign, int threads,
-                           size_t smem, int nfields, cudaStream_t st) {
-  cudaError_t ea = opt_in_smem((const void*)k_strided<P, -1>, 227 * 1024);
-  if (ea == cudaSuccess) ea = opt_in_smem((const void*)k_strided<P, 1>, 227 * 1024);
-  if (ea != cudaSuccess) return ea;
+cudaError_t launch_x_c2r(const XParams& p, const StagePlan* sp, unsigned long long fam, const float4* tw, int threads,
+                         size_t smem, int nfields, cudaStream_t st) {
+  auto kernel = k_x_c2r<P, true>;
+  if constexpr (!P::kF64) {
+    if (!has_c67(fam)) kernel = k_x_c2r<P, false>;
+  }
+  return launch_single(kernel, dim3(p.tiles, nfields), threads, smem, st, p, sp, tw);
+}
+template <class P>
+cudaError_t launch_strided(const SParams& p, const StagePlan* sp, unsigned long long fam, const float4* tw,
+                           bool forward_sign, int threads, size_t smem, int nfields, cudaStream_t st) {
   const long long blocks = (long long)p.xtiles * p.O1 * nfields;
   if (blocks <= 0 || blocks > 0x7FFFFFFFLL) return cudaErrorInvalidConfiguration;
-  if (forward_sign) k_strided<P, -1><<<(unsigned)blocks, threads, smem, st>>>(p, sp, tw);
-  else k_strided<P, 1><<<(unsigned)blocks, threads, smem, st>>>(p, sp, tw);
-  return cudaGetLastError();
+  auto kernel = forward_sign ? k_strided<P, -1, true> : k_strided<P, 1, true>;
+  if constexpr (!P::kF64) {
+    if (!has_c67(fam)) kernel = forward_sign ? k_strided<P, -1, false> : k_strided<P, 1, false>;
+  }
+  return launch_single(kernel, dim3((unsigned)blocks), threads, smem, st, p, sp, tw);
 }
 template <class P>
 cudaError_t launch_cheby(const ChebyParams& p, int nfields, cudaStream_t st) {
@@ -431,12 +441,12 @@ cudaError_t launch_cheby(const ChebyParams& p, int nfields, cudaStream_t st) {
 }
 
 #define P3G_INSTANTIATE(P)                                                                                          \
-  template cudaError_t launch_x_r2c<P>(const XParams&, const StagePlan*, const float4*, int, size_t, int,          \
-                                       cudaStream_t);                                                              \
-  template cudaError_t launch_x_c2r<P>(const XParams&, const StagePlan*, const float4*, int, size_t, int,          \
-                                       cudaStream_t);                                                              \
-  template cudaError_t launch_strided<P>(const SParams&, const StagePlan*, const float4*, bool, int, size_t, int,  \
-                                         cudaStream_t);                                                            \
+  template cudaError_t launch_x_r2c<P>(const XParams&, const StagePlan*, unsigned long long, const float4*, int,   \
+                                       size_t, int, cudaStream_t);                                                 \
+  template cudaError_t launch_x_c2r<P>(const XParams&, const StagePlan*, unsigned long long, const float4*, int,   \
+                                       size_t, int, cudaStream_t);                                                 \
+  template cudaError_t launch_strided<P>(const SParams&, const StagePlan*, unsigned long long, const float4*, bool, \
+                                         int, size_t, int, cudaStream_t);                                          \
   template cudaError_t launch_cheby<P>(const ChebyParams&, int, cudaStream_t);                                     \
   template cudaError_t launch_x_long<P>(int, const XLongParams&, int, cudaStream_t);
 

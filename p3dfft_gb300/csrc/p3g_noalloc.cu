@@ -70,12 +70,12 @@ int forward_passes(p3g_plan p, const void* in, void* out, int zi, bool fsign, vo
   z.range = range_params(p, false, true);
   const int rc = launch_range_scan(p, in, rsize, rsize, 1, st);  // P3G_RANGE_AUTO only
   if (rc) return rc;
-  cudaError_t e = launch_x_r2c<P>(x, p->d_sp + p->ax_x.sp_index, p->d_tw, p->ax_x.threads, p->ax_x.smem, 1, st);
+  cudaError_t e = launch_x_r2c<P>(x, p->d_sp + p->ax_x.sp_index, p->ax_x.sp.fam, p->d_tw, p->ax_x.threads, p->ax_x.smem, 1, st);
   if (e != cudaSuccess) return fail(P3G_E_CUDA, std::string("X r2c launch: ") + cudaGetErrorString(e));
-  e = launch_strided<P>(y, p->d_sp + p->ax_y.sp_index, p->d_tw, true, p->ax_y.threads, p->ax_y.smem, 1, st);
+  e = launch_strided<P>(y, p->d_sp + p->ax_y.sp_index, p->ax_y.sp.fam, p->d_tw, true, p->ax_y.threads, p->ax_y.smem, 1, st);
   if (e != cudaSuccess) return fail(P3G_E_CUDA, std::string("Y pass launch: ") + cudaGetErrorString(e));
   const AxisPlan& az = p->ax_z[zi];
-  e = launch_strided<P>(z, p->d_sp + az.sp_index, p->d_tw, fsign, az.threads, az.smem, 1, st);
+  e = launch_strided<P>(z, p->d_sp + az.sp_index, az.sp.fam, p->d_tw, fsign, az.threads, az.smem, 1, st);
   if (e != cudaSuccess) return fail(P3G_E_CUDA, std::string("Z pass launch: ") + cudaGetErrorString(e));
   p->launches += 3;
   return P3G_OK;

@@ -451,7 +451,7 @@ __global__ void __launch_bounds__(tile_max_threads(MODE, P::kF64, false), 1)
       Tile<P, GroupThreads> t{sm.buf0 + b * pp.c.buf_elems, nullptr, pp.s.M, pp.s.log2m, 1, pp.s.M, 0, 0, nullptr, th};
       constexpr int E = MODE == kTileSmall ? TileElems<P>::value / 2 : TileElems<P>::value;
       constexpr bool kFull = MODE == kTileFull || MODE == kTileFullWide;
-      run_families<P, DIR, E, kPointMajor, kRawNone, E, kFull>(t, sm.tw, pp.s.N, pp.c.fam, 0);
+      run_families<P, DIR, E, kPointMajor, kRawNone, E, kFull, true>(t, sm.tw, pp.s.N, pp.c.fam, 0);
     }
     {
       int xt, o1, o2;
@@ -853,7 +853,7 @@ __global__ void __launch_bounds__(tile_max_threads(MODE, P::kF64, true), 1)
       uint32_t amax = 0;
       Tile<P, GroupThreads> t{tb, nullptr, pp.x.M, pp.x.log2m, pp.x.LS, 1, pp.x.ps, R2C ? sm.cta[1] : 0,
                               R2C ? &amax : nullptr, th, R2C ? reinterpret_cast<unsigned*>(&sm.cta[2]) : nullptr};
-      run_families<P, R2C ? -1 : 1, E, kLineMajor, R2C ? kRawR2C : kRawC2R, E, kFull>(t, sm.tw, pp.x.nx, pp.c.fam, 0);
+      run_families<P, R2C ? -1 : 1, E, kLineMajor, R2C ? kRawR2C : kRawC2R, E, kFull, true>(t, sm.tw, pp.x.nx, pp.c.fam, 0);
     }
     asm volatile("" : "+r"(tile));  // the tile's place again, rather than held across the stages
     place(field, p0);

@@ -858,7 +858,7 @@ int run_strided(p3g_plan p, SParams& s, AxisPlan& ap, bool fwd_sign, int nv, cud
     p->launches++;
     return P3G_OK;
   }
-  cudaError_t e = launch_strided<P>(s, p->d_sp + ap.sp_index, p->d_tw, fwd_sign, ap.threads, ap.smem, nv, st);
+  cudaError_t e = launch_strided<P>(s, p->d_sp + ap.sp_index, ap.sp.fam, p->d_tw, fwd_sign, ap.threads, ap.smem, nv, st);
   if (e != cudaSuccess) return fail(P3G_E_CUDA, std::string("strided pass launch: ") + cudaGetErrorString(e));
   p->launches++;
   return P3G_OK;
@@ -902,7 +902,7 @@ int run_x_r2c(p3g_plan p, XParams& x, int nv, cudaStream_t st, int max_sms = 0) 
     p->launches++;
     return P3G_OK;
   }
-  cudaError_t e = launch_x_r2c<P>(x, p->d_sp + ap.sp_index, p->d_tw, ap.threads, ap.smem, nv, st);
+  cudaError_t e = launch_x_r2c<P>(x, p->d_sp + ap.sp_index, ap.sp.fam, p->d_tw, ap.threads, ap.smem, nv, st);
   if (e != cudaSuccess) return fail(P3G_E_CUDA, std::string("X r2c launch: ") + cudaGetErrorString(e));
   p->launches++;
   return P3G_OK;
@@ -948,7 +948,7 @@ int run_x_c2r(p3g_plan p, XParams& x, int nv, cudaStream_t st, int max_sms = 0) 
     p->launches++;
     return P3G_OK;
   }
-  cudaError_t e = launch_x_c2r<P>(x, p->d_sp + ap.sp_index, p->d_tw, ap.threads, ap.smem, nv, st);
+  cudaError_t e = launch_x_c2r<P>(x, p->d_sp + ap.sp_index, ap.sp.fam, p->d_tw, ap.threads, ap.smem, nv, st);
   if (e != cudaSuccess) return fail(P3G_E_CUDA, std::string("X c2r launch: ") + cudaGetErrorString(e));
   p->launches++;
   return P3G_OK;
