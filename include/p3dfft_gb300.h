@@ -66,7 +66,10 @@ int p3g_get_dims(p3g_plan plan, int conf, int start[3], int end[3], int size[3])
  * build/ftran.F90:489-780 and :104-317).  op is 3 letters; op[2] selects the
  * Z transform: 't'/'f' FFT, 'c' DCT-I (REDFT00), 's' DST-I (RODFT00), 'n'/'0'
  * none.  dim_in/dim_out are the element spacings between fields (reals /
- * complexes); <= 0 selects the dense size.  in and out may alias. */
+ * complexes); <= 0 selects the dense size.  in and out may alias.
+ * Fields are independent of one another, but the FFT stages are chosen for all
+ * nv together: a field's result may differ in rounding (within the transform's
+ * error) from that of a call with another nv. */
 int p3g_ftran_r2c(p3g_plan plan, const void* in, void* out, const char* op, int nv, long long dim_in,
                   long long dim_out, void* stream);
 
