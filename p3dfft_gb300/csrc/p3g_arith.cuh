@@ -334,15 +334,6 @@ P3G_D df dadd(df a, df b) {
   r.lo = fadd_rn(fadd_rn(a.lo, b.lo), e);
   return r;
 }
-P3G_D df dsub(df a, df b) {
-  float s, e;
-  two_sum(a.hi, -b.hi, s, e);
-  df r;
-  r.hi = s;
-  r.lo = fadd_rn(fsub_rn(a.lo, b.lo), e);
-  return r;
-}
-P3G_D df dneg(df a) { return df{-a.hi, -a.lo}; }
 // a * c for a double-float constant c (the lo*lo term is below 2^-48)
 P3G_D df dmulc(df a, float chi, float clo) {
   df r;

@@ -49,11 +49,9 @@ template <class P, bool R2C>
 cudaError_t launch_x_pipe(const XPipeParams& p, const float4* tw, TileMode mode, int threads,
                           size_t smem, int grid, cudaStream_t st) {
   auto kernel = k_x_pipe<P, R2C, kTileGeneral>;
-  if (mode == kTileFull) kernel = k_x_pipe<P, R2C, kTileFull>;
   if (mode == kTileSmall) kernel = k_x_pipe<P, R2C, kTileSmall>;
-  if constexpr (!P::kF64) {
-    if (mode == kTileFullWide) kernel = k_x_pipe<P, R2C, kTileFullWide>;
-  }
+  constexpr TileMode kFull = P::kF64 ? kTileFull : kTileFullWide;  // the unguarded form that size_x gives
+  if (mode == kFull) kernel = k_x_pipe<P, R2C, kFull>;
   const cudaError_t e = opt_in_smem((const void*)kernel, 227 * 1024);
   if (e != cudaSuccess) return e;
   return launch_pass(kernel, p.c, grid, threads, smem, st, p, tw);

@@ -126,9 +126,10 @@ static void best_split(std::array<int, 4> e, int rmax, int odd_max, int E, size_
 // plans: of at most 8 besides the powers of two).
 //
 // kSplitFixed: radices 3 and 5 after the powers of two and other primes as
-// generic stages.  The binary32 STRIDE1 plans keep it: their output goes into
-// the shell spectrum, whose binary64 sums callers compare far below binary32's
-// rounding, and another split rounds otherwise.
+// generic stages.  The binary32 STRIDE1 plans keep it, so that their results and
+// the binary64 shell sums formed from them keep the bits they have always had
+// (another split moves the sums by up to 1e-7, binary32's own rounding).  It
+// costs them the wide plans of mixed lengths and the 7-point codelet.
 enum SplitKind { kSplitNarrow = 0, kSplitWide = 1, kSplitFixed = 2 };
 static bool factor(int n, int max_pow2, SplitKind kind, std::vector<int>& radices) {
   if (kind != kSplitFixed && n > 1 && (n & (n - 1)) != 0 && max_pow2 >= 8) {
@@ -450,9 +451,8 @@ static TileShape size_strided(const AxisPlan& ap, long long nv) {
   // groups, 1.81 ms with one; 256 points of 1024 x 256 x 2048: 0.73 ms with four
   // groups, 0.95 with two)
   const bool wide_regs = !f64 && ((far_rows && n > 512) || (tstore && !in_l2 && n >= 256));
-  const int wide_index = ap.spw_index;
   double best = 1e300;
-  for (int narrow = wide_index >= 0 ? 0 : 1; narrow < (ap.fixed_plan && wide_index >= 0 ? 1 : 2); ++narrow) {
+  for (int narrow = ap.has_spw ? 0 : 1; narrow < (ap.fixed_plan && ap.has_spw ? 1 : 2); ++narrow) {
     const StagePlan& sp = narrow ? ap.sp : ap.spw;
     bool pow2 = true;
     int rmax = 0;
@@ -490,7 +490,6 @@ static TileShape size_strided(const AxisPlan& ap, long long nv) {
           best = t;
           TileShape& o = best_shape;
           o.ok = true;
-          o.wide = !narrow;
           o.m = M;
           o.log2m = ilog2(M);
           o.mode = mode;
@@ -540,9 +539,8 @@ static TileShape size_x(const AxisPlan& ap, long long nv) {
   const int n = ap.n;
   const size_t room = 227 * 1024;
   const bool small_ok = !f64 && 2.0 * esize * n * pairs * nv <= kXSmallBytes;  // real lines and modes
-  const int wide_index = ap.spw_index;
   double best = 1e300;
-  for (int narrow = wide_index >= 0 ? 0 : 1; narrow < (ap.fixed_plan && wide_index >= 0 ? 1 : 2); ++narrow) {
+  for (int narrow = ap.has_spw ? 0 : 1; narrow < (ap.fixed_plan && ap.has_spw ? 1 : 2); ++narrow) {
     const StagePlan& sp = narrow ? ap.sp : ap.spw;
     bool pow2 = true;
     int rmax = 0;
@@ -576,7 +574,6 @@ static TileShape size_x(const AxisPlan& ap, long long nv) {
           best = t;
           TileShape& o = best_shape;
           o.ok = true;
-          o.wide = !narrow;
           o.m = M;
           o.log2m = ilog2(M);
           o.mode = mode;
@@ -817,7 +814,6 @@ int run_strided(p3g_plan p, SParams& s, AxisPlan& ap, bool fwd_sign, int nv, cud
     pp.c.groups = ts.g;
     pp.c.gthreads = ts.threads / ts.g;
     pp.c.err = p->d_err;
-    pp.chunk = esize;
     CUtensorMap map, omap;
     std::memset(&map, 0, sizeof(map));
     std::memset(&omap, 0, sizeof(omap));
@@ -920,7 +916,6 @@ int run_x_c2r(p3g_plan p, XParams& x, int nv, cudaStream_t st, int max_sms = 0) 
     x.tiles = ((x.nlines + 1) / 2 + x.M - 1) / x.M;
     XPipeParams xp{};
     xp.x = x;
-    xp.chunk = (int)sizeof(typename P::W);
     xp.c.tiles_per_field = x.tiles;
     xp.c.ntiles = x.tiles * nv;
     xp.c.tw_base = ts.tw_lo;
@@ -1739,7 +1734,7 @@ int p3g_plan_create_tuned(p3g_plan* out, int nx, int ny, int nz, int nxc, int ny
   // caps the radix, a wide one for the grouped kernels: up to 16 on F64, 32
   // for powers of two on F32.
   const bool fixed_split = !f64 && layout == P3G_LAYOUT_STRIDE1;
-  auto wide_ok = [&](const AxisPlan&, int n) {
+  auto wide_ok = [&](int n) {
     if (fixed_split && (n & (n - 1)) != 0) return false;
     if (f64) return max_radix == 0 || max_radix >= 16;
     return max_radix == 0 || max_radix >= ((n & (n - 1)) == 0 ? 32 : 16);
@@ -1755,16 +1750,14 @@ int p3g_plan_create_tuned(p3g_plan* out, int nx, int ny, int nz, int nxc, int ny
     // the wide plan (1024 = 16 x 16 x 4 against 8 x 8 x 4 x 4 on F64, 32 x 32
     // against 16 x 16 x 4 on F32; 540 = 12 x 9 x 5 against 6 x 6 x 5 x 3),
     // where it is another
-    if (wide_ok(ap, n)) {
+    if (wide_ok(n)) {
       StagePlan w;
-
       if (build_stages(n, f64 ? 16 : 32, kSplitWide, tw, w) && w.fam != ap.sp.fam &&
           (f64 || (n & (n - 1)) != 0 || family_count(w.fam, 0) > 0)) {
         ap.spw = w;
         ap.tw_lo_w = tw.mark;
         ap.tw_cnt_w = tw.count;
-        ap.spw_index = (int)sps.size();
-        sps.push_back(w);
+        ap.has_spw = true;
       }
     }
     return true;
@@ -1799,7 +1792,7 @@ int p3g_plan_create_tuned(p3g_plan* out, int nx, int ny, int nz, int nxc, int ny
       if (ls < nh2) ls = nh2;
     };
     pad_of(ax.sp, ax.ps, ax.ls);
-    if (ax.spw_index >= 0) pad_of(ax.spw, ax.ps_w, ax.ls_w);
+    if (ax.has_spw) pad_of(ax.spw, ax.ps_w, ax.ls_w);
     if (!x_fits) ax.ls = 0;
     ax.smem = (size_t)ax.M * ax.ls * (f64 ? 16 : 8) * (ax.sp.has_generic ? 2 : 1);
     if (ax.smem > 227 * 1024) {

@@ -16,9 +16,9 @@ namespace p3g {
 int fail(int code, const std::string& msg);
 
 // A pipelined kernel's tiles and launch: tiles of m lines (columns), g groups
-// over `threads` threads, a ring of nbuf buffers; wide: the stage plan spw.
+// over `threads` threads, a ring of nbuf buffers.
 struct TileShape {
-  bool ok = false, wide = false;
+  bool ok = false;
   int m = 1, log2m = 0, g = 1, threads = 32, nbuf = 2, buf_elems = 0;
   TileMode mode = kTileGeneral;
   size_t smem = 0;
@@ -53,7 +53,7 @@ struct AxisPlan {
   // the grouped pass kernels: a second stage plan with the large codelets and
   // its twiddle slice; the other kernels, and grids of few tiles, run sp
   StagePlan spw{};
-  int spw_index = -1;  // -1: none, the pipelined kernels run sp
+  bool has_spw = false;  // else the pipelined kernels run sp
   bool fixed_plan = false;  // kSplitFixed: no choice between spw and sp
   int tw_lo_w = 0, tw_cnt_w = 0;
   int ls_w = 0, ps_w = 0;  // X axis: line-pair stride and padding of the wide tiles
