@@ -404,10 +404,10 @@ constexpr StridedModel kStridedF64 = {{0.25, 0.25, 0.45, 0.97, 1.0, 1.0}, 12, 0.
 // 0.83 ms with 32 points, 0.72 with 16).  Where a line's points lie 1.5 MB apart,
 // every row of a tile is in a memory page of its own and rows of 32 bytes are
 // ruinous too (800^3 Z, 2.6 MB: M = 8 1.83 ms, M = 4 3.1; 1 MB apart: equal).
-constexpr StridedModel kStridedF32 = {{0.08, 0.44, 0.92, 0.97, 1.0, 1.0}, 14, 0.85, 0.9, 1.3, 50};
-constexpr StridedModel kStridedF32User = {{0.08, 0.41, 0.85, 0.95, 1.0, 1.0}, 14, 0.85, 0.9, 1.3, 50};
+constexpr StridedModel kStridedF32 = {{0.08, 0.44, 0.92, 0.97, 1.0, 1.0}, 14, 0.85, 0.9, 1.45, 50};
+constexpr StridedModel kStridedF32User = {{0.08, 0.41, 0.85, 0.95, 1.0, 1.0}, 14, 0.85, 0.9, 1.45, 50};
 constexpr StridedModel kStridedF32Stride1 = {{0.08, 0.44, 0.92, 0.97, 1.0, 1.0}, 14, 0.85, 0.9, 0.95, 50};
-constexpr StridedModel kStridedF32Apart = {{0.08, 0.25, 0.45, 0.9, 1.0, 1.0}, 14, 0.85, 0.9, 1.3, 50};
+constexpr StridedModel kStridedF32Apart = {{0.08, 0.25, 0.45, 0.9, 1.0, 1.0}, 14, 0.85, 0.9, 1.45, 50};
 constexpr StridedModel kStridedF32L2 = {{0.08, 0.55, 0.95, 0.97, 1.0, 1.0}, 14, 0.85, 0.9, 1.05, 50};
 static const StridedModel& strided_model(const TileExtents& e, bool in_l2) {
   if (e.f64) return kStridedF64;
@@ -417,16 +417,20 @@ static const StridedModel& strided_model(const TileExtents& e, bool in_l2) {
   return e.tstore ? kStridedF32User : kStridedF32;
 }
 // Half the points per thread (16 of 32) in passes of more tiles than groups: for
-// mixed radices whose largest fills 12 to 16 of a thread's 16 points.  The
-// unguarded powers of two are faster with 32 (256-point Y of 512 x 256 x 512:
-// 0.104 against 0.124 ms), and a 10 leaves 6 of 16 idle and a 9 takes 18 (900-
-// point Y of 256 x 900 x 128: 0.100 against 0.140 ms).
-static bool small_form(bool f64, const StagePlan& sp, bool pow2, int rmax) {
+// mixed radices whose largest is 8, 12, 15 or 16 and fills most of a thread's 16
+// points.  The unguarded powers of two are faster with 32 (256-point Y of 512 x
+// 256 x 512: 0.104 against 0.124 ms), a 10 leaves 6 of 16 idle and a 9 takes 18
+// (900-point Y of 256 x 900 x 128: 0.100 against 0.140 ms), and radices 5 and 7
+// alone lose too (625-point Y of 256 x 625 x 128: 0.115 against 0.124 ms), as
+// does a narrow plan of more stages (1000-point X, 8 x 5 x 5 x 5 against 10 x 10
+// x 10: 102 against 81 us).
+static bool small_form(const AxisPlan& ap, const StagePlan& sp, bool pow2, int rmax) {
   bool nine = false;
   for (int i = 0; i < sp.nstages; ++i) nine = nine || sp.radix[i] == 9;
-  return !f64 && !pow2 && !nine && 16 / rmax * rmax >= 12;
+  return !ap.ext.f64 && !pow2 && !nine && rmax >= 8 && rmax != 10 &&
+         (!ap.has_spw || sp.nstages <= ap.spw.nstages);
 }
-constexpr double kL2Bytes = 128 << 20;
+constexpr double kL2Bytes = 144 << 20;  // a little over the L2 cache's 129 MB: 256^3 counts as inside
 
 static TileShape size_strided(const AxisPlan& ap, long long nv) {
   TileShape best_shape;
@@ -440,17 +444,18 @@ static TileShape size_strided(const AxisPlan& ap, long long nv) {
   const size_t room = 227 * 1024;
   const bool in_l2 = 2.0 * esize * n * X * O1 <= kL2Bytes;  // the pass's input and output
   const StridedModel& md = strided_model(ap.ext, in_l2);
-  // binary32 FULL passes of 256 points or more that store user rows by threads
-  // run half the groups with twice the registers where the data comes from
-  // DRAM: at 128 the spilled words and the stores share what is left of the L1
-  // (1024-point Z forward 5.4 ms against 2.5 ms; 512-point of 256 x 1024 x 512
-  // 0.31 against 0.29 ms, but 78 against 67 us of 64 x 256 x 512, in the L2
-  // cache).  So do those with far rows of more than 512 points, where every row
-  // of a tile is in a memory page of its own and groups that drift apart spread
-  // over more pages at a time (Y of 1024^3, 4.2 MB apart: 1.95 ms with two
-  // groups, 1.81 ms with one; 256 points of 1024 x 256 x 2048: 0.73 ms with four
-  // groups, 0.95 with two)
-  const bool wide_regs = !f64 && ((far_rows && n > 512) || (tstore && !in_l2 && n >= 256));
+  // binary32 FULL passes of 512 points or more (256 with rows pages apart: Z of
+  // 1024 x 2048 x 256 1.82 against 2.0 ms; of 512 x 512 x 256 0.264 against 0.252)
+  // that store user rows by threads run half the groups with twice the
+  // registers where the data comes from DRAM: at 128 the spilled words and the
+  // stores share what is left of the L1 (1024-point Z forward 5.4 ms against 2.5
+  // ms; 512-point of 256 x 1024 x 512 0.31 against 0.29 ms, but 78 against 67 us
+  // of 64 x 256 x 512, in the L2 cache).  So do those with far rows of more than
+  // 512 points: groups that drift apart spread over more memory pages at a time
+  // (Y of 1024^3, 4.2 MB apart: 1.95 ms with two groups, 1.81 ms with one; 256
+  // points of 1024 x 256 x 2048: 0.73 ms with four groups, 0.95 with two)
+  const bool apart = ap.ext.row_bytes >= 3 << 19;
+  const bool wide_regs = !f64 && ((far_rows && n > 512) || (tstore && !in_l2 && (n >= 512 || (n >= 256 && apart))));
   double best = 1e300;
   for (int narrow = ap.has_spw ? 0 : 1; narrow < (ap.fixed_plan && ap.has_spw ? 1 : 2); ++narrow) {
     const StagePlan& sp = narrow ? ap.sp : ap.spw;
@@ -478,13 +483,16 @@ static TileShape size_strided(const AxisPlan& ap, long long nv) {
         const int g = (int)std::max(
             1.0, std::min({(double)(max_threads / tg), (double)kMaxGroups, (double)(fit - 1), per_sm}));
         // half the points per thread: where every tile has a group of its own, or small_form
-        if (E < Emax && per_sm > g && !small_form(f64, sp, pow2, rmax)) continue;
+        if (E < Emax && per_sm > g && !small_form(ap, sp, pow2, rmax)) continue;
+        // a single round of tiles is latency; binary64's constants were found on those too
+        const StridedModel& m = per_sm <= g ? kStridedF64 : md;
         const size_t row = M * esize;
-        const double rows = md.rows[row >= 256 ? 5 : ilog2((int)row) - 3];
+        const double rows = m.rows[row >= 256 ? 5 : ilog2((int)row) - 3];
         const double warps = (mode == kTileFullWide ? 1.5 : 1.0) * g * tg / 32;
-        const double overlap = std::min(1.0, warps / md.warps) * (g >= 2 || mode == kTileFullWide ? 1.0 : md.one_group);
-        const double clocks = (f64 ? 1.0 : 0.35) * sp.nstages *
-                              (mode == kTileSmall ? md.small : (mode == kTileGeneral ? 1.0 : md.full));
+        const double alone = mode != kTileFullWide ? m.one_group : (in_l2 || per_sm <= g ? 1.0 : 0.93);
+        const double overlap = std::min(1.0, warps / m.warps) * (g >= 2 ? 1.0 : alone);
+        const double clocks =
+            (f64 ? 1.0 : 0.35) * sp.nstages * (mode == kTileSmall ? m.small : (mode == kTileGeneral ? 1.0 : m.full));
         const double t = per_sm * tg * E * clocks / (rows * overlap) + md.latency * E * sp.nstages;
         if (t < best * 0.999) {
           best = t;
@@ -498,12 +506,12 @@ static TileShape size_strided(const AxisPlan& ap, long long nv) {
           // buffers beyond the groups (loads in flight): two, one where the
           // tiles leave by threads (binary32 512^3 Y: 0.19 ms with two, 0.26
           // with one; 540-point binary32 Z: 1.42 with two, 1.34 with one) or
-          // one or two groups hold a guarded binary32 plan (640-point Y of
+          // two groups hold a guarded binary32 plan (640-point Y of
           // 256 x 640 x 1024: 0.45 ms with two, 0.38 with one), and twice as
           // many for the small tiles of short binary32 lines (256^3 Y:
           // 0.046 -> 0.040 ms with four, Z 0.051 -> 0.049 with two)
           const bool small_tile = !f64 && buf <= (tstore ? 24 : 16) * 1024;
-          const bool one = tstore || (!f64 && mode == kTileGeneral && g <= 2);
+          const bool one = tstore || (!f64 && mode == kTileGeneral && g == 2);
           o.nbuf = std::min(fit, g + (one ? 1 : 2) * (small_tile ? 2 : 1));
           o.buf_elems = (int)(buf / esize);
           o.smem = fixed + o.nbuf * buf;
@@ -565,9 +573,10 @@ static TileShape size_x(const AxisPlan& ap, long long nv) {
         const double per_sm = std::ceil((double)((pairs + M - 1) / M) * nv / sm_count);
         const int g = (int)std::max(
             1.0, std::min({(double)(max_threads / tg), (double)kMaxGroups, (double)(fit - 1), per_sm}));
-        if (E < Emax && per_sm > g && !(small_ok && per_sm >= 4 * g && small_form(f64, sp, pow2, rmax))) continue;
+        if (E < Emax && per_sm > g && !(small_ok && per_sm >= 4 * g && small_form(ap, sp, pow2, rmax))) continue;
         const double warps = (mode == kTileFullWide ? 1.3 : 1.0) * g * tg / 32;
-        const double overlap = std::min(1.0, warps / 12) * (g >= 2 ? 1.0 : 0.8) * (tg >= 64 ? 1.0 : 0.9);
+        const double few = g >= 2 ? (E < Emax && per_sm > g && g < 3 ? 0.9 : 1.0) : 0.8;
+        const double overlap = std::min(1.0, warps / 12) * few * (tg >= 64 ? 1.0 : 0.9);
         const double clocks = (f64 ? 1.0 : 0.35) * sp.nstages * (E < Emax && per_sm > g ? 0.85 : 1.0);
         const double t = per_sm * tg * E * clocks / overlap + 100.0 * E * sp.nstages / (f64 ? 1 : 2);
         if (t < best * 0.999) {
@@ -930,9 +939,10 @@ int run_x_c2r(p3g_plan p, XParams& x, int nv, cudaStream_t st, int max_sms = 0) 
       // the modes of a line arrive by one bulk copy, rounded up to 16 bytes,
       // which the line pitch and the raw stride hold; short lines by cp.async:
       // one thread issues a tile's copies, and 64 of 264 bytes cost it more than
-      // the group's own (64-point binary32 X c2r of 16 x 64^3: 33 against 27 us)
+      // the group's own (64-point binary32 X c2r of 16 x 64^3: 33 against 27 us;
+      // two copies cost less: 45 x 36 x 50 backward 23.6 against 24.3 us)
       const long long es = (long long)sizeof(typename P::W);
-      xp.bulk = x.nkeep * es >= 512 && (x.in_line * es) % 16 == 0 && (x.in_field * es) % 16 == 0 &&
+      xp.bulk = (x.nkeep * es >= 512 || ts.m <= 2) && (x.in_line * es) % 16 == 0 && (x.in_field * es) % 16 == 0 &&
                 (long long)x.in_line * es >= ((x.nkeep * es + 15) / 16) * 16 && aligned_to(x.in, 16) &&
                 device_memory(x.in);
     }
